@@ -26,54 +26,85 @@ __device__ __forceinline__ T warp_sum(T v) {
 }
 
 // VK 0: FP64 values, FP64 vectors.  VK 1: FP32 values, FP32 vectors (FP32 sums).
-// VK 2: FP32 value + FP32 remainder, FP64 vectors.  VK 3: FP32 values, FP64 vectors.
+// VK 2: FP32 value + FP32 remainder, FP64 vectors.
+//
+// One warp per row, consecutive warps on consecutive rows.  What bounds it is the latency
+// of the column stream (HBM) followed by the gather of x (L1 / L2), so the loop is
+// software pipelined: the next 256 elements' columns and values (of this row, or the
+// first ones of the warp's next row) are in flight while this chunk's x are gathered.
+// Measured, CUDA events: 200,003 rows, 2.0e8 elements, FP32: 420 us with four loads per
+// lane and no pipelining, 365 us here (4.4 TB/s of stream); 131,611 rows, 1.2e8
+// elements, FP64: 264 -> 253 us (5.6 TB/s); 6,943 rows: 13.9 -> 11.5 us.  Larger blocks,
+// and contiguous runs of rows per block, were slower (1.1x and 1.3-2x).
+constexpr int SPMV_U = 8;  // elements per lane in one chunk
+
 template <int VK, typename X>
-__global__ void __launch_bounds__(256) k_spmv(int64_t N, const int64_t* __restrict__ row_start,
-                                              const int32_t* __restrict__ row_len, const int32_t* __restrict__ cols,
-                                              const double* __restrict__ v64, const float* __restrict__ v32,
-                                              const float* __restrict__ vlo, const double* __restrict__ diag,
-                                              const X* __restrict__ x, X* __restrict__ y) {
+__global__ void __launch_bounds__(256, 4) k_spmv(int64_t N, const int64_t* __restrict__ row_start,
+                                                 const int32_t* __restrict__ row_len, const int32_t* __restrict__ cols,
+                                                 const double* __restrict__ v64, const float* __restrict__ v32,
+                                                 const float* __restrict__ vlo, const double* __restrict__ diag,
+                                                 const X* __restrict__ x, X* __restrict__ y) {
     using A = typename std::conditional<VK == 1, float, double>::type;
     const int lane = threadIdx.x & 31;
-    const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    for (int64_t p = warp; p < N; p += nwarps) {
-        const int64_t s = row_start[p];
-        const int len = row_len[p];
-        A acc = 0;
-        int k = lane;
-        // four independent loads in flight per lane
-        for (; k + 96 < len; k += 128) {
-            int c0 = __ldcs(cols + s + k), c1 = __ldcs(cols + s + k + 32);
-            int c2 = __ldcs(cols + s + k + 64), c3 = __ldcs(cols + s + k + 96);
-            A a0, a1, a2, a3;
-            if constexpr (VK == 0) {
-                a0 = __ldcs(v64 + s + k); a1 = __ldcs(v64 + s + k + 32);
-                a2 = __ldcs(v64 + s + k + 64); a3 = __ldcs(v64 + s + k + 96);
-            } else if constexpr (VK == 2) {
-                a0 = (double)__ldcs(v32 + s + k) + (double)__ldcs(vlo + s + k);
-                a1 = (double)__ldcs(v32 + s + k + 32) + (double)__ldcs(vlo + s + k + 32);
-                a2 = (double)__ldcs(v32 + s + k + 64) + (double)__ldcs(vlo + s + k + 64);
-                a3 = (double)__ldcs(v32 + s + k + 96) + (double)__ldcs(vlo + s + k + 96);
-            } else {
-                a0 = (A)__ldcs(v32 + s + k); a1 = (A)__ldcs(v32 + s + k + 32);
-                a2 = (A)__ldcs(v32 + s + k + 64); a3 = (A)__ldcs(v32 + s + k + 96);
+    int64_t p = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
+    if (p >= N) return;
+    // a chunk's columns (-1: past the row's end) and values
+    auto load = [&](int64_t s, int k0, int len, int (&c)[SPMV_U], A (&a)[SPMV_U]) {
+#pragma unroll
+        for (int j = 0; j < SPMV_U; j++) {
+            const int k = k0 + lane + 32 * j;
+            c[j] = -1;
+            a[j] = 0;
+            if (k < len) {
+                c[j] = __ldcs(cols + s + k);
+                if constexpr (VK == 0) a[j] = __ldcs(v64 + s + k);
+                else if constexpr (VK == 2) a[j] = (double)__ldcs(v32 + s + k) + (double)__ldcs(vlo + s + k);
+                else a[j] = __ldcs(v32 + s + k);
             }
-            acc += a0 * (A)__ldg(x + c0);
-            acc += a1 * (A)__ldg(x + c1);
-            acc += a2 * (A)__ldg(x + c2);
-            acc += a3 * (A)__ldg(x + c3);
         }
-        for (; k < len; k += 32) {
-            int c = __ldcs(cols + s + k);
-            A a;
-            if constexpr (VK == 0) a = __ldcs(v64 + s + k);
-            else if constexpr (VK == 2) a = (double)__ldcs(v32 + s + k) + (double)__ldcs(vlo + s + k);
-            else a = (A)__ldcs(v32 + s + k);
-            acc += a * (A)__ldg(x + c);
+    };
+    int64_t s = row_start[p], s_next = 0;
+    int len = row_len[p], len_next = 0;
+    if (p + nwarps < N) {
+        s_next = row_start[p + nwarps];
+        len_next = row_len[p + nwarps];
+    }
+    int c[SPMV_U], cn[SPMV_U];
+    A a[SPMV_U], an[SPMV_U];
+    load(s, 0, len, c, a);
+    int k0 = 0;
+    A acc = 0;
+    for (;;) {
+        const bool more = k0 + 32 * SPMV_U < len;
+        const int kn = more ? k0 + 32 * SPMV_U : 0;
+        load(more ? s : s_next, kn, more ? len : len_next, cn, an);
+        A xv[SPMV_U];
+#pragma unroll
+        for (int j = 0; j < SPMV_U; j++) xv[j] = c[j] >= 0 ? (A)__ldg(x + c[j]) : (A)0;
+#pragma unroll
+        for (int j = 0; j < SPMV_U; j++)
+            if (c[j] >= 0) acc += a[j] * xv[j];
+        if (!more) {
+            acc = warp_sum(acc);
+            if (lane == 0) y[p] = (X)(diag[p] * (double)x[p] + (double)acc);
+            acc = 0;
+            p += nwarps;
+            if (p >= N) break;
+            s = s_next;
+            len = len_next;
+            len_next = 0;
+            if (p + nwarps < N) {
+                s_next = row_start[p + nwarps];
+                len_next = row_len[p + nwarps];
+            }
         }
-        acc = warp_sum(acc);
-        if (lane == 0) y[p] = (X)(diag[p] * (double)x[p] + (double)acc);
+        k0 = kn;
+#pragma unroll
+        for (int j = 0; j < SPMV_U; j++) {
+            c[j] = cn[j];
+            a[j] = an[j];
+        }
     }
 }
 
@@ -194,21 +225,9 @@ __global__ void __launch_bounds__(256) k_self_energy(int64_t N, const int64_t* _
 
 }  // namespace
 
-int spmv_grid(risqgpu* h) {
-    static int cached_dev = -1, cached = 0;
-    if (cached_dev != h->device) {
-        int occ = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_spmv<0, double>, 256, 0);
-        cached = num_sms(h) * std::max(occ, 1);
-        cached_dev = h->device;
-    }
-    return cached;
-}
-
 int sigma_device(risqgpu* h, const void* x, void* y, int kind) {
     if (!h->built) { h->err = "sigma before build"; return RISQGPU_ERR_INVALID; }
     const int64_t n = (int64_t)h->N;
-    const int grid = spmv_grid(h);
     if (h->upper) return sigma_tiles(h, x, y, kind);
     if (h->precision == RISQGPU_MATRIX_FREE) {
         if (kind != 0) {
@@ -217,6 +236,8 @@ int sigma_device(risqgpu* h, const void* x, void* y, int kind) {
         }
         return sigma_matrix_free(h, (const double*)x, (double*)y);
     }
+    // every warp of the chip resident, no more of them than rows
+    const int grid = (int)std::min<int64_t>((n + 7) / 8, (int64_t)num_sms(h) * 4);
     if (kind == 0) {
         const double* xd = (const double*)x;
         double* yd = (double*)y;
@@ -291,7 +312,7 @@ int self_energy_impl(risqgpu* h, double energy, double gmin, double* out) {
         RQ_CUDA(h, cudaMemcpyAsync(out, sc, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream));
         return sync(h, "self energy");
     }
-    const int grid = spmv_grid(h);
+    const int grid = num_sms(h) * 8;
     const int up = h->upper ? 1 : 0;
     if (h->precision == RISQGPU_FP64)
         k_self_energy<0><<<grid, 256, 0, h->stream>>>(n, h->d_row_start, h->d_row_len, h->d_cols, h->d_val64, nullptr,
