@@ -147,12 +147,14 @@ int set_mlp_impl(risqgpu* h, int n_in, int hidden, const float* w1, const float*
         std::vector<uint16_t> t(n);
         for (size_t i = 0; i < n; i++) t[i] = f_to_bf16(src[i]);
         RQ_TRY(dalloc(h, dst, n));
-        RQ_CUDA(h, cudaMemcpy(dst, t.data(), n * sizeof(uint16_t), cudaMemcpyHostToDevice));
+        RQ_CUDA(h, cudaMemcpyAsync(dst, t.data(), n * sizeof(uint16_t), cudaMemcpyHostToDevice, h->stream));
+        RQ_TRY(sync(h, "MLP weights"));
         return RISQGPU_OK;
     };
     auto up32 = [&](const float* src, size_t n, float*& dst) -> int {
         RQ_TRY(dalloc(h, dst, n));
-        RQ_CUDA(h, cudaMemcpy(dst, src, n * sizeof(float), cudaMemcpyHostToDevice));
+        RQ_CUDA(h, cudaMemcpyAsync(dst, src, n * sizeof(float), cudaMemcpyHostToDevice, h->stream));
+        RQ_TRY(sync(h, "MLP weights"));
         return RISQGPU_OK;
     };
     RQ_TRY(up16(w1, (size_t)hidden * n_in, h->mlp.w1));
