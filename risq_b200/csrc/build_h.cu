@@ -305,14 +305,21 @@ struct SigmaIO {
 // in shared memory (singles, which sum over the occupied orbitals, and doubles,
 // which read one or two integrals), and each queue is evaluated whenever it holds
 // 32 entries, with every lane busy.  Stored elements are written in queue order.
-template <int W, int MODE>
-__global__ void __launch_bounds__(256) k_build_rows(SetView<W> v, Ints I, double thr_single, int upper,
+//
+// OUT_UPPER: only q > p.  OUT_BINS (q > p too): MODE 0 counts the candidates of every (row
+// block, window) bin, MODEs 2 and 3 append the elements to their bins; the hits of a warp
+// that fall in one bin share one atomic.
+enum BuildOut : int { OUT_ROWS = 0, OUT_UPPER = 1, OUT_BINS = 2 };
+
+template <int W, int MODE, int OUT>
+__global__ void __launch_bounds__(256) k_build_rows(SetView<W> v, Ints I, double thr_single, TileOut T,
                                                     int* __restrict__ row_counter,
                                                     int64_t* __restrict__ cnt, const int64_t* __restrict__ row_start,
                                                     int32_t* __restrict__ row_len, int32_t* __restrict__ cols,
                                                     double* __restrict__ v64, float* __restrict__ v32,
                                                     float* __restrict__ vlo, int64_t row_lo, int64_t row_hi,
                                                     int64_t base_off, SigmaIO io) {
+    constexpr bool upper = OUT != OUT_ROWS, TILED = OUT == OUT_BINS;
     constexpr int WARPS = 256 / 32;
     constexpr int QCAP = 64;  // < 32 pending + 32 new
     __shared__ int s_q[WARPS][2][QCAP];
@@ -331,7 +338,14 @@ __global__ void __launch_bounds__(256) k_build_rows(SetView<W> v, Ints I, double
         if (p >= row_hi) break;
         const Bits<W> a = v.up_at(p), b = v.dn_at(p);
         const bool p_new = v.nsh == 0 || v.orig[p] >= v.nsh;
-        int64_t base = (MODE >= 1 && MODE <= 4) ? row_start[p] - base_off : 0;
+        int64_t base = (!TILED && MODE >= 1 && MODE <= 4) ? row_start[p] - base_off : 0;
+        int64_t bin0 = 0;  // OUT_BINS: bin of window 0 (may lie before the block's first bin)
+        uint32_t code0 = 0;
+        if constexpr (TILED) {
+            const int64_t b = p >> T.kb;
+            bin0 = T.bin_off[b] - ((b << T.kb) >> T.cb);
+            code0 = (uint32_t)(p & ((1 << T.rb) - 1)) << T.cb;
+        }
         int count = 0;
         double acc = 0.0;  // MODE 5
         int ns = 0, nd = 0;  // queue fill, warp-uniform
@@ -363,6 +377,30 @@ __global__ void __launch_bounds__(256) k_build_rows(SetView<W> v, Ints I, double
             }
             if constexpr (MODE == 5) {
                 if (ok) acc += val * __ldg(io.x + q);
+            } else if constexpr (TILED) {
+                const unsigned grp = __match_any_sync(FULL, ok ? (unsigned)(q >> T.cb) : 0x80000000u | lane);
+                const int leader = __ffs(grp) - 1;
+                const int64_t bin = bin0 + (q >> T.cb);
+                unsigned long long pos = 0;
+                if (ok && lane == leader) pos = atomicAdd(T.cur + bin, (unsigned long long)__popc(grp));
+                if (ok && lane == leader && (pos & LEFT_BIN))
+                    pos = LEFT_BIN | atomicAdd(T.left_cur + (p >> T.rb), (unsigned long long)__popc(grp));
+                pos = __shfl_sync(FULL, pos, leader) + __popc(grp & lt);
+                if (ok) {
+                    const float hi = (float)val;
+                    if (pos & LEFT_BIN) {
+                        const int64_t at = (int64_t)(pos & ~LEFT_BIN);
+                        T.lcol[at] = (uint32_t)q;
+                        T.lrow[at] = (uint16_t)(code0 >> T.cb);
+                        T.l32[at] = hi;
+                        if (MODE == 3) T.llo[at] = (float)(val - (double)hi);
+                    } else {
+                        const int64_t at = (int64_t)pos - T.el0;
+                        T.code[at] = code0 | ((uint32_t)q & ((1u << T.cb) - 1u));
+                        v32[at] = hi;
+                        if (MODE == 3) vlo[at] = (float)(val - (double)hi);
+                    }
+                }
             } else {
                 const unsigned m = __ballot_sync(FULL, ok);
                 if (ok) store(base + count + __popc(m & lt), q, val);
@@ -377,8 +415,28 @@ __global__ void __launch_bounds__(256) k_build_rows(SetView<W> v, Ints I, double
             __syncwarp();
             nq = rem;
         };
+        // OUT_BINS search: the first `take` queued candidates into the bins' counts
+        auto tally = [&](int take) {
+            const int q = lane < take ? qd[lane] : 0;
+            const unsigned grp = __match_any_sync(FULL, lane < take ? (unsigned)(q >> T.cb) : 0x80000000u | lane);
+            if (lane < take && lane == __ffs(grp) - 1) atomicAdd(T.hist + bin0 + (q >> T.cb), (uint32_t)__popc(grp));
+            const int rem = nd - take;
+            const int tq = lane < rem ? qd[take + lane] : 0;
+            __syncwarp();
+            if (lane < rem) qd[lane] = tq;
+            __syncwarp();
+            nd = rem;
+        };
         auto push = [&](bool hit, bool single, int q, int kind) {
             hit = hit && (!upper || q > p);
+            if constexpr (MODE == 0 && TILED) {
+                const unsigned m = __ballot_sync(FULL, hit);
+                if (hit) qd[nd + __popc(m & lt)] = q;
+                nd += __popc(m);
+                __syncwarp();
+                if (nd >= 32) tally(32);
+                return;
+            }
             if (MODE == 0) {
                 count += __popc(__ballot_sync(FULL, hit));
                 return;
@@ -395,7 +453,7 @@ __global__ void __launch_bounds__(256) k_build_rows(SetView<W> v, Ints I, double
         };
 
         // (0) elements kept from the previous build (pairs of old determinants)
-        if (MODE != 5 && !p_new && v.prev_inv_of_caller) {
+        if (OUT == OUT_ROWS && MODE != 5 && !p_new && v.prev_inv_of_caller) {
             int op = v.prev_inv_of_caller[v.orig[p]];
             int64_t ps = v.prev_row_start[op];
             int pl = v.prev_row_len[op];
@@ -547,6 +605,8 @@ __global__ void __launch_bounds__(256) k_build_rows(SetView<W> v, Ints I, double
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
             if (lane == 0) io.y[p] = io.diag[p] * io.x[p] + acc;
+        } else if constexpr (TILED) {
+            if (MODE == 0 && nd > 0) tally(nd);
         } else if (lane == 0) {
             // row capacities are rounded up to 4 elements so that every row starts on a
             // 16-byte (columns) / 32-byte (FP64 values) boundary for vector loads
@@ -843,89 +903,64 @@ __global__ void k_invert(const int32_t* __restrict__ orig, int64_t n, int32_t* _
         inv[orig[p]] = (int32_t)p;
 }
 
-template <int W>
-int launch_fill(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int upper, int precision, int* counter,
-                int blocks, int threads, int32_t* cols, double* v64, float* v32, float* vlo, int64_t row_lo,
-                int64_t row_hi, int64_t base) {
-    if (precision == RISQGPU_FP64)
-        k_build_rows<W, 1><<<blocks, threads, 0, h->stream>>>(v, I, thr, upper, counter, nullptr, h->d_row_start,
-                                                              h->d_row_len, cols, v64, nullptr, nullptr, row_lo,
-                                                              row_hi, base, SigmaIO{});
-    else if (precision == RISQGPU_FP32)
-        k_build_rows<W, 2><<<blocks, threads, 0, h->stream>>>(v, I, thr, upper, counter, nullptr, h->d_row_start,
-                                                              h->d_row_len, cols, nullptr, v32, nullptr, row_lo,
-                                                              row_hi, base, SigmaIO{});
-    else if (precision == RISQGPU_MIXED)
-        k_build_rows<W, 3><<<blocks, threads, 0, h->stream>>>(v, I, thr, upper, counter, nullptr, h->d_row_start,
-                                                              h->d_row_len, cols, nullptr, v32, vlo, row_lo, row_hi,
-                                                              base, SigmaIO{});
-    else
-        k_build_rows<W, 4><<<blocks, threads, 0, h->stream>>>(v, I, thr, upper, counter, nullptr, h->d_row_start,
-                                                              h->d_row_len, cols, nullptr, nullptr, nullptr, row_lo,
-                                                              row_hi, base, SigmaIO{});
+template <int W, int OUT>
+int launch_fill(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, const TileOut& T, int precision,
+                int* counter, int blocks, int threads, int32_t* cols, double* v64, float* v32, float* vlo,
+                int64_t row_lo, int64_t row_hi, int64_t base) {
+#define RQ_FILL(MODE)                                                                                            \
+    k_build_rows<W, MODE, OUT><<<blocks, threads, 0, h->stream>>>(v, I, thr, T, counter, nullptr, h->d_row_start, \
+                                                                  h->d_row_len, cols, v64, v32, vlo, row_lo,      \
+                                                                  row_hi, base, SigmaIO{})
+    if constexpr (OUT != OUT_BINS)
+        if (precision == RISQGPU_FP64) RQ_FILL(1);
+    if constexpr (OUT != OUT_UPPER) {
+        if (precision == RISQGPU_FP32) RQ_FILL(2);
+        if (precision == RISQGPU_MIXED) RQ_FILL(3);
+    }
+    if constexpr (OUT == OUT_ROWS)
+        if (precision == RISQGPU_COLS) RQ_FILL(4);
+#undef RQ_FILL
     return check_launch(h, "fill rows");
 }
 
-__global__ void k_panel_starts(const int64_t* __restrict__ row_start, int64_t n, int rb, int64_t np,
-                               int64_t* __restrict__ out) {
-    for (int64_t P = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; P <= np; P += (int64_t)gridDim.x * blockDim.x)
-        out[P] = row_start[min(n, P << rb)];
+// stored elements of the filled rows
+int count_rows(risqgpu* h, int64_t& nnz) {
+    const int64_t n = (int64_t)h->N;
+    int64_t* sum = nullptr;
+    char* tmp = nullptr;
+    ScopedFree<2> release(sum, tmp);
+    RQ_TRY(dalloc(h, sum, 1));
+    size_t tb = 0;
+    cub::DeviceReduce::Sum(nullptr, tb, h->d_row_len, sum, (int)n, h->stream);
+    RQ_TRY(dalloc(h, tmp, tb));
+    cub::DeviceReduce::Sum(tmp, tb, h->d_row_len, sum, (int)n, h->stream);
+    RQ_CUDA(h, cudaMemcpyAsync(&nnz, sum, sizeof(int64_t), cudaMemcpyDeviceToHost, h->stream));
+    return sync(h, "fill rows");
 }
 
-// Upper-triangle fill through the tiled layout: the rows are filled chunk by chunk of
-// whole panels into a CSR buffer that holds one chunk, and every chunk is regrouped
-// into tiles before the next is filled, so that the device holds the tiled arrays
-// plus one chunk rather than two copies of the matrix.
-template <int W>
-int fill_tiled(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int precision, int* counter, int64_t cap,
-               int blocks, int threads) {
-    const int64_t n = (int64_t)h->N;
-    int rb = 0, cb = 0;
-    if (tile_shape(n, rb, cb) != RISQGPU_OK) {
-        h->err = "determinant set too large for the tiled upper-triangle layout";
-        return RISQGPU_ERR_INVALID;
-    }
-    h->tile_rb = rb;
-    h->tile_cb = cb;
-    const int64_t np = (n + ((int64_t)1 << rb) - 1) >> rb;
-    std::vector<int64_t> ps((size_t)np + 1);
-    {
-        int64_t* dps = nullptr;
-        ScopedFree<1> release(dps);
-        RQ_TRY(dalloc(h, dps, (size_t)np + 1));
-        k_panel_starts<<<grid_for(h, np + 1), 256, 0, h->stream>>>(h->d_row_start, n, rb, np, dps);
-        RQ_CUDA(h, cudaMemcpyAsync(ps.data(), dps, sizeof(int64_t) * (np + 1), cudaMemcpyDeviceToHost, h->stream));
-        RQ_TRY(sync(h, "panel starts"));
-    }
-    // this handle's panels: all of them, or with a row-block partition the rank's share,
-    // contiguous panels cut where the counted pairs reach rank / nranks of the total
-    int64_t own_lo = 0, own_hi = np;
-    if (h->part_n > 1) {
-        auto cut = [&](int r) -> int64_t {
-            const int64_t goal = (int64_t)((double)ps[np] * r / h->part_n);
-            return (int64_t)(std::lower_bound(ps.begin(), ps.end() - 1, goal) - ps.begin());
-        };
-        own_lo = h->part_rank == 0 ? 0 : cut(h->part_rank);
-        own_hi = h->part_rank == h->part_n - 1 ? np : cut(h->part_rank + 1);
-        own_hi = std::max(own_hi, own_lo);
-        // rows of other ranks' panels hold no stored pairs here
-        RQ_CUDA(h, cudaMemsetAsync(h->d_row_len, 0, sizeof(int32_t) * n, h->stream));
-    }
-    h->part_p_lo = own_lo;
-    h->part_p_hi = own_hi;
-    const int64_t own_cap = ps[own_hi] - ps[own_lo];
-    const size_t vb = precision == RISQGPU_FP64 ? 8 : (precision == RISQGPU_MIXED ? 8 : 4);
-    const size_t per_el = 4 + vb;
-    // bytes held besides the element arrays: per-row tile data and accumulators, plus a
-    // margin for the conversion's work buffers that grows with the set (at most 256 MiB)
-    const size_t base_need = (size_t)own_cap * per_el + (size_t)n * 32;
-    const size_t fixed = base_need + std::max((size_t)8 << 20, std::min((size_t)256 << 20, base_need / 32));
+// The share of panels [lo, hi) of a handle with a row-block partition: contiguous panels
+// cut where the counted pairs (ps: before each panel) reach rank / nranks of the total.
+void own_panels(const risqgpu* h, const std::vector<int64_t>& ps, int64_t& lo, int64_t& hi) {
+    const int64_t np = (int64_t)ps.size() - 1;
+    lo = 0;
+    hi = np;
+    if (h->part_n <= 1) return;
+    auto cut = [&](int r) -> int64_t {
+        const int64_t goal = (int64_t)((double)ps[np] * r / h->part_n);
+        return (int64_t)(std::lower_bound(ps.begin(), ps.end() - 1, goal) - ps.begin());
+    };
+    if (h->part_rank > 0) lo = cut(h->part_rank);
+    if (h->part_rank < h->part_n - 1) hi = cut(h->part_rank + 1);
+    hi = std::max(hi, lo);
+}
+
+// Chunks of the panels [own_lo, own_hi): the fewest whose largest one, at per_el bytes an
+// element, fits beside `fixed` bytes; chunk k ends at the panel boundary nearest to k/K of
+// the pairs, so the chunks hold about equal shares.
+int chunk_cuts(risqgpu* h, const std::vector<int64_t>& ps, int64_t own_lo, int64_t own_hi, size_t fixed, size_t per_el,
+               std::vector<int64_t>& cuts, int64_t& max_chunk) {
     const size_t avail = mem_available(h);
-    // chunks: the fewest whose largest chunk fits beside the tiled arrays; chunk k ends at
-    // the panel boundary nearest to k/K of the pairs, so the chunks hold about equal shares
-    std::vector<int64_t> cuts;
-    int64_t max_chunk = 0;
-    const int64_t own_np = own_hi - own_lo;
+    const int64_t own_cap = ps[own_hi] - ps[own_lo], own_np = own_hi - own_lo;
     for (int64_t K = 1;; K = K < 8 ? K + 1 : K * 2) {
         cuts.assign(1, own_lo);
         for (int64_t k = 1; k < K; k++) {
@@ -944,87 +979,194 @@ int fill_tiled(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int p
             return RISQGPU_ERR_OOM;
         }
     }
-    int32_t* ccols = nullptr;
-    double* c64 = nullptr;
-    float *c32 = nullptr, *clo = nullptr;
-    ScopedFree<4> release(ccols, c64, c32, clo);
-    RQ_TRY(dalloc(h, h->d_el_idx, (size_t)own_cap));
-    if (precision == RISQGPU_FP64) RQ_TRY(dalloc(h, h->d_val64, (size_t)own_cap));
-    else RQ_TRY(dalloc(h, h->d_val32, (size_t)own_cap));
-    if (precision == RISQGPU_MIXED) RQ_TRY(dalloc(h, h->d_val_lo, (size_t)own_cap));
-    RQ_TRY(dalloc(h, ccols, (size_t)max_chunk));
-    if (precision == RISQGPU_FP64) RQ_TRY(dalloc(h, c64, (size_t)max_chunk));
-    else RQ_TRY(dalloc(h, c32, (size_t)max_chunk));
-    if (precision == RISQGPU_MIXED) RQ_TRY(dalloc(h, clo, (size_t)max_chunk));
-    TileBuilder tb;
-    RQ_TRY(tb.begin(h, np, own_cap));
-    const bool verbose = std::getenv("RISQGPU_VERBOSE") != nullptr;
-    if (verbose)
+    if (std::getenv("RISQGPU_VERBOSE"))
         std::fprintf(stderr, "[risqgpu] tiled build: %zu chunks, largest %lld pairs, %zu MiB available\n",
                      cuts.size() - 1, (long long)max_chunk, avail >> 20);
-    for (size_t c = 0; c + 1 < cuts.size(); c++) {
-        const auto tc0 = std::chrono::steady_clock::now();
-        const int64_t p_lo = cuts[c], p_hi = cuts[c + 1];
-        const int64_t r_lo = p_lo << rb, r_hi = std::min(n, p_hi << rb);
-        const int64_t base = ps[p_lo];
-        RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
-        RQ_TRY(launch_fill<W>(h, v, I, thr, 1, precision, counter, blocks, threads, ccols, c64, c32, clo, r_lo, r_hi,
-                              base));
-        if (verbose) RQ_TRY(sync(h, "fill"));
-        const auto tc1 = std::chrono::steady_clock::now();
-        if (precision == RISQGPU_FP64)
-            RQ_TRY(tb.chunk<double>(p_lo, p_hi, h->d_row_start, base, h->d_row_len, ccols, c64, nullptr, h->d_val64,
-                                    nullptr));
-        else
-            RQ_TRY(tb.chunk<float>(p_lo, p_hi, h->d_row_start, base, h->d_row_len, ccols, c32, clo, h->d_val32,
-                                   h->d_val_lo));
-        if (verbose)
-            std::fprintf(stderr, "[risqgpu]   chunk %zu: panels %lld..%lld fill %.1f ms, regroup %.1f ms\n", c,
-                         (long long)p_lo, (long long)p_hi,
-                         std::chrono::duration<double, std::milli>(tc1 - tc0).count(),
-                         std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - tc1).count());
-    }
-    RQ_TRY(tb.finish());
-    // every stored element went into the tiles exactly once
-    int64_t* sum = nullptr;
-    char* tmp = nullptr;
-    ScopedFree<2> release_sum(sum, tmp);
-    RQ_TRY(dalloc(h, sum, 1));
-    size_t tbytes = 0;
-    cub::DeviceReduce::Sum(nullptr, tbytes, h->d_row_len, sum, (int)n, h->stream);
-    RQ_TRY(dalloc(h, tmp, tbytes));
-    cub::DeviceReduce::Sum(tmp, tbytes, h->d_row_len, sum, (int)n, h->stream);
-    int64_t stored = 0;
-    RQ_CUDA(h, cudaMemcpyAsync(&stored, sum, sizeof(int64_t), cudaMemcpyDeviceToHost, h->stream));
-    RQ_TRY(sync(h, "tiled count check"));
-    if (stored != tb.el_next) {
-        h->err = "tiled layout holds " + std::to_string(tb.el_next) + " elements for " + std::to_string(stored) +
-                 " stored";
-        return RISQGPU_ERR_INVALID;
-    }
     return RISQGPU_OK;
 }
 
-// stored count, statistics and handle state after a fill
-int finish_build(risqgpu* h, int precision, int upper, int64_t cap, std::chrono::steady_clock::time_point t0,
-                 std::chrono::steady_clock::time_point t1, std::chrono::steady_clock::time_point t2, cudaEvent_t* ev,
-                 risqgpu_hstats* st) {
-    using clk = std::chrono::steady_clock;
+__global__ void k_panel_starts(const int64_t* __restrict__ row_start, int64_t n, int rb, int64_t np,
+                               int64_t* __restrict__ out) {
+    for (int64_t P = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; P <= np; P += (int64_t)gridDim.x * blockDim.x)
+        out[P] = row_start[min(n, P << rb)];
+}
+
+// FP64 upper triangle: rows filled chunk by chunk of whole panels into a CSR buffer that
+// holds one chunk, each chunk regrouped into tiles before the next is filled.
+template <int W>
+int fill_upper64(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int* counter, int blocks, int threads,
+                 int64_t& nnz) {
     const int64_t n = (int64_t)h->N;
-    int64_t* sum = nullptr;
-    char* tmp = nullptr;
-    ScopedFree<2> release(sum, tmp);
-    RQ_TRY(dalloc(h, sum, 1));
-    size_t tb = 0;
-    cub::DeviceReduce::Sum(nullptr, tb, h->d_row_len, sum, (int)n, h->stream);
-    RQ_TRY(dalloc(h, tmp, tb));
-    cub::DeviceReduce::Sum(tmp, tb, h->d_row_len, sum, (int)n, h->stream);
-    RQ_TRY(sync(h, "fill rows"));
+    if (tile_shape64(n, h->tile_rb, h->tile_cb) != RISQGPU_OK) {
+        h->err = "determinant set too large for the tiled upper-triangle layout";
+        return RISQGPU_ERR_INVALID;
+    }
+    const int rb = h->tile_rb;
+    h->tile_kb = rb;
+    const int64_t np = (n + ((int64_t)1 << rb) - 1) >> rb;
+    h->n_panels = np;
+    std::vector<int64_t> ps((size_t)np + 1);
+    {
+        int64_t* dps = nullptr;
+        ScopedFree<1> release(dps);
+        RQ_TRY(dalloc(h, dps, (size_t)np + 1));
+        k_panel_starts<<<grid_for(h, np + 1), 256, 0, h->stream>>>(h->d_row_start, n, rb, np, dps);
+        RQ_CUDA(h, cudaMemcpyAsync(ps.data(), dps, sizeof(int64_t) * (np + 1), cudaMemcpyDeviceToHost, h->stream));
+        RQ_TRY(sync(h, "panel starts"));
+    }
+    own_panels(h, ps, h->part_p_lo, h->part_p_hi);
+    const int64_t own_lo = h->part_p_lo, own_hi = h->part_p_hi;
+    // rows of other ranks' panels hold no stored pairs here
+    RQ_CUDA(h, cudaMemsetAsync(h->d_row_len, 0, sizeof(int32_t) * n, h->stream));
+    // bytes of the tiled arrays (10 an element, an eighth more for padding and headers),
+    // per row tile data and accumulators, plus a margin that grows with the set
+    const size_t base_need = (size_t)(ps[own_hi] - ps[own_lo]) * 10 / 8 * 9 + (size_t)n * 40;
+    const size_t fixed = base_need + std::max((size_t)8 << 20, std::min((size_t)256 << 20, base_need / 32));
+    std::vector<int64_t> cuts;
+    int64_t max_chunk = 0;
+    RQ_TRY(chunk_cuts(h, ps, own_lo, own_hi, fixed, 24, cuts, max_chunk));
+    int32_t* ccols = nullptr;
+    uint32_t* code = nullptr;
+    double *c64 = nullptr, *t64 = nullptr;
+    ScopedFree<4> release(ccols, c64, code, t64);
+    RQ_TRY(dalloc(h, ccols, (size_t)max_chunk));
+    RQ_TRY(dalloc(h, c64, (size_t)max_chunk));
+    RQ_TRY(dalloc(h, code, (size_t)max_chunk));
+    RQ_TRY(dalloc(h, t64, (size_t)max_chunk));
+    Tiles64Builder tb;
+    RQ_TRY(tb.begin(h));
+    for (size_t c = 0; c + 1 < cuts.size(); c++) {
+        const int64_t p_lo = cuts[c], p_hi = cuts[c + 1];
+        RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
+        RQ_TRY((launch_fill<W, OUT_UPPER>(h, v, I, thr, TileOut{}, RISQGPU_FP64, counter, blocks, threads, ccols, c64,
+                                          nullptr, nullptr, p_lo << rb, std::min(n, p_hi << rb), ps[p_lo])));
+        RQ_TRY(tb.chunk(p_lo, p_hi, h->d_row_start, ps[p_lo], h->d_row_len, ccols, c64, code, t64, max_chunk));
+    }
+    RQ_TRY(tb.finish());
+    RQ_TRY(count_rows(h, nnz));
+    // every stored element went into the tiles or the leftovers exactly once
+    if (nnz != tb.stored) {
+        h->err = "tiled layout holds " + std::to_string(tb.stored) + " elements for " + std::to_string(nnz) + " stored";
+        return RISQGPU_ERR_INVALID;
+    }
+    dfree(h->d_row_start);
+    dfree(h->d_row_len);
+    return RISQGPU_OK;
+}
+
+// First bin of every block of rows: block b holds the windows from its own column on.
+__global__ void k_bin_off(int64_t n_blocks, int64_t n_windows, int cb, int kb, int64_t* __restrict__ off) {
+    for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b <= n_blocks; b += (int64_t)gridDim.x * blockDim.x) {
+        // sum over b' < b of n_windows - floor(b' 2^kb / 2^cb)
+        const int64_t per = (int64_t)1 << (cb - kb), q = b / per, r = b - q * per;
+        off[b] = b * n_windows - (per * (q * (q - 1) / 2) + r * q);
+    }
+}
+
+// FP32 upper triangle (with or without remainders).  The search pass counts the candidates of
+// every (row block, window) bin; the fill pass then appends every stored pair to its bin
+// in temporary arrays that hold one chunk of whole panels, and each chunk is arranged into
+// tiles before the next is filled, so that the device holds the tiled arrays plus one
+// chunk rather than two copies of the matrix.
+template <int W>
+int build_tiled(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int precision, int* counter, int blocks,
+                int threads, cudaEvent_t* ev, std::chrono::steady_clock::time_point& t1, int64_t& cap, int64_t& nnz) {
+    const int64_t n = (int64_t)h->N;
+    int rb = 0, cb = 0, kb = 0;
+    if (tile_shape(n, rb, cb, kb) != RISQGPU_OK) {
+        h->err = "determinant set too large for the tiled upper-triangle layout";
+        return RISQGPU_ERR_INVALID;
+    }
+    h->tile_rb = rb;
+    h->tile_cb = cb;
+    h->tile_kb = kb;
+    const int64_t np = (n + ((int64_t)1 << rb) - 1) >> rb;
+    const int64_t nblk = (n + ((int64_t)1 << kb) - 1) >> kb, nw = ((n - 1) >> cb) + 1;
+    h->n_panels = np;
+    int64_t* bin_off = nullptr;
+    uint32_t* hist = nullptr;
+    unsigned long long* cur = nullptr;
+    ScopedFree<3> release_bins(bin_off, hist, cur);
+    RQ_TRY(dalloc(h, bin_off, (size_t)nblk + 1));
+    k_bin_off<<<grid_for(h, nblk + 1), 256, 0, h->stream>>>(nblk, nw, cb, kb, bin_off);
+    int64_t n_bins = 0;
+    RQ_CUDA(h, cudaMemcpyAsync(&n_bins, bin_off + nblk, sizeof(int64_t), cudaMemcpyDeviceToHost, h->stream));
+    RQ_TRY(sync(h, "bins"));
+    RQ_TRY(dalloc(h, hist, (size_t)n_bins));
+    RQ_CUDA(h, cudaMemsetAsync(hist, 0, sizeof(uint32_t) * n_bins, h->stream));
+    TileOut T;
+    T.rb = rb;
+    T.cb = cb;
+    T.kb = kb;
+    T.bin_off = bin_off;
+    T.hist = hist;
+    RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
+    RQ_CUDA(h, cudaEventRecord(ev[0], h->stream));
+    k_build_rows<W, 0, OUT_BINS><<<blocks, threads, 0, h->stream>>>(v, I, thr, T, counter, nullptr, nullptr, nullptr,
+                                                                nullptr, nullptr, nullptr, nullptr, 0, n, 0, SigmaIO{});
+    RQ_CUDA(h, cudaEventRecord(ev[1], h->stream));
+    RQ_TRY(check_launch(h, "count bins"));
+    TileBuilder tb;
+    RQ_TRY(tb.plan(h, hist, bin_off, nblk));
+    t1 = std::chrono::steady_clock::now();
+    RQ_CUDA(h, cudaEventRecord(ev[2], h->stream));
+    std::vector<int64_t> ps((size_t)np + 1, 0);  // candidates before each panel
+    for (int64_t P = 0; P < np; P++)
+        ps[(size_t)P + 1] = ps[(size_t)P] + tb.counts[(size_t)P].dense + tb.counts[(size_t)P].left;
+    cap = ps[(size_t)np];
+    own_panels(h, ps, h->part_p_lo, h->part_p_hi);
+    const int64_t own_lo = h->part_p_lo, own_hi = h->part_p_hi;
+    const size_t vb = precision == RISQGPU_MIXED ? 8 : 4;
+    // bytes of the tiled arrays (an eighth more for their padding), plus a margin that grows with the set (at most 256 MiB)
+    // for what the allocator rounds up
+    size_t need = sizeof(unsigned long long) * (size_t)n_bins + (size_t)n * 8 + (size_t)np * 64;
+    for (int64_t P = own_lo; P < own_hi; P++) {
+        const PanelCount& c = tb.counts[(size_t)P];
+        need += (size_t)c.vecs * 2 * (2 + vb) / 8 * 9 + (size_t)c.groups * 136 + (size_t)c.left * (6 + vb) +
+                (size_t)c.tiles * 24 + (size_t)c.blocks * (sizeof(TileBlock) + ((size_t)2 << kb));
+    }
+    const size_t fixed = need + std::max((size_t)8 << 20, std::min((size_t)256 << 20, need / 32));
+    std::vector<int64_t> cuts;
+    int64_t max_chunk = 0;
+    RQ_TRY(chunk_cuts(h, ps, own_lo, own_hi, fixed, 4 + vb, cuts, max_chunk));
+    RQ_TRY(dalloc(h, cur, (size_t)n_bins));
+    RQ_TRY(tb.begin(own_lo, own_hi, precision, hist, bin_off, cur));
+    dfree(hist);
+    uint32_t* code = nullptr;
+    float *c32 = nullptr, *clo = nullptr;
+    ScopedFree<3> release(code, c32, clo);
+    RQ_TRY(dalloc(h, code, (size_t)max_chunk));
+    RQ_TRY(dalloc(h, c32, (size_t)max_chunk));
+    if (precision == RISQGPU_MIXED) RQ_TRY(dalloc(h, clo, (size_t)max_chunk));
+    T.cur = cur;
+    T.left_cur = tb.left_cur;
+    T.code = code;
+    T.lcol = h->d_left_col;
+    T.lrow = h->d_left_row;
+    T.l32 = h->d_left32;
+    T.llo = h->d_left_lo;
+    for (size_t c = 0; c + 1 < cuts.size(); c++) {
+        const int64_t p_lo = cuts[c], p_hi = cuts[c + 1];
+        T.el0 = tb.base[(size_t)p_lo].el;
+        RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
+        RQ_TRY((launch_fill<W, OUT_BINS>(h, v, I, thr, T, precision, counter, blocks, threads, nullptr, nullptr, c32, clo,
+                                         p_lo << rb, std::min(n, p_hi << rb), 0)));
+        RQ_TRY(tb.chunk(p_lo, p_hi, T.el0, cur, code, c32, clo));
+    }
+    RQ_TRY(tb.finish());
+    nnz = tb.stored;
+    RQ_CUDA(h, cudaEventRecord(ev[3], h->stream));
+    return RISQGPU_OK;
+}
+
+// statistics and handle state after a fill of nnz elements
+int finish_build(risqgpu* h, int precision, int upper, int64_t cap, int64_t nnz,
+                 std::chrono::steady_clock::time_point t0, std::chrono::steady_clock::time_point t1,
+                 std::chrono::steady_clock::time_point t2, cudaEvent_t* ev, risqgpu_hstats* st) {
+    using clk = std::chrono::steady_clock;
+    RQ_TRY(sync(h, "build"));
     auto t3 = clk::now();
-    int64_t nnz = 0;
-    RQ_CUDA(h, cudaMemcpyAsync(&nnz, sum, sizeof(int64_t), cudaMemcpyDeviceToHost, h->stream));
-    RQ_TRY(sync(h, "nnz"));
-    h->cap = (size_t)cap;
+    h->cap = (size_t)(upper ? nnz : cap);
     h->nnz_full = upper ? 2 * (uint64_t)nnz : (uint64_t)nnz;
     h->nnz_upper = upper ? (uint64_t)nnz : (uint64_t)nnz / 2;
     h->precision = precision;
@@ -1039,7 +1181,7 @@ int finish_build(risqgpu* h, int precision, int upper, int64_t cap, std::chrono:
         st->ms_count = std::chrono::duration<double, std::milli>(t1 - t0).count();
         st->ms_fill = std::chrono::duration<double, std::milli>(t3 - t2).count();
         size_t vb = precision == RISQGPU_FP64 ? 8 : (precision == RISQGPU_FP32 ? 4 : (precision == RISQGPU_COLS ? 0 : 8));
-        st->bytes_csr = (uint64_t)nnz * (4 + vb);
+        st->bytes_csr = (uint64_t)nnz * ((upper ? 2 : 4) + vb);
         st->n_tiles = (uint64_t)h->n_tiles;
         st->nnz_dense = h->n_dense_el;
     }
@@ -1071,12 +1213,11 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
     SetView<W> v = make_view<W>(h, incremental, prev_inv);
     Ints I{h->d_h1, h->d_h2, h->nuc};
     RQ_TRY(dalloc(h, counter, 1));
-    RQ_TRY(dalloc(h, cnt, n + 1));
-    RQ_TRY(dalloc(h, h->d_row_start, n + 1));
-    RQ_TRY(dalloc(h, h->d_row_len, n));
     const int threads = 256;
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_build_rows<W, 1>, threads, 0);
+    if (upper && precision != RISQGPU_FP64)
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_build_rows<W, 3, OUT_BINS>, threads, 0);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_build_rows<W, 1, OUT_ROWS>, threads, 0);
     const int blocks = num_sms(h) * std::max(occ, 1);
 
     RQ_TRY(sync(h, "pre-count"));
@@ -1084,10 +1225,25 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
     cudaEvent_t* ev = be.ev;
     for (int k = 0; k < 4; k++) RQ_CUDA(h, cudaEventCreate(&ev[k]));
     auto t0 = clk::now();
+    if (upper && precision != RISQGPU_FP64) {
+        auto t1 = t0;
+        int64_t cap = 0, nnz = 0;
+        RQ_TRY(build_tiled<W>(h, v, I, thr, precision, counter, blocks, threads, ev, t1, cap, nnz));
+        return finish_build(h, precision, upper, cap, nnz, t0, t1, t1, ev, st);
+    }
+    RQ_TRY(dalloc(h, cnt, n + 1));
+    RQ_TRY(dalloc(h, h->d_row_start, n + 1));
+    RQ_TRY(dalloc(h, h->d_row_len, n));
     RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
     RQ_CUDA(h, cudaEventRecord(ev[0], h->stream));
-    k_build_rows<W, 0><<<blocks, threads, 0, h->stream>>>(v, I, thr, upper, counter, cnt, nullptr, nullptr, nullptr,
-                                                          nullptr, nullptr, nullptr, 0, n, 0, SigmaIO{});
+    if (upper)
+        k_build_rows<W, 0, OUT_UPPER><<<blocks, threads, 0, h->stream>>>(v, I, thr, TileOut{}, counter, cnt, nullptr, nullptr,
+                                                                         nullptr, nullptr, nullptr, nullptr, 0, n, 0,
+                                                                         SigmaIO{});
+    else
+        k_build_rows<W, 0, OUT_ROWS><<<blocks, threads, 0, h->stream>>>(v, I, thr, TileOut{}, counter, cnt, nullptr, nullptr,
+                                                                        nullptr, nullptr, nullptr, nullptr, 0, n, 0,
+                                                                        SigmaIO{});
     RQ_CUDA(h, cudaEventRecord(ev[1], h->stream));
     RQ_TRY(check_launch(h, "count rows"));
     {
@@ -1098,7 +1254,6 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
         RQ_TRY(dalloc(h, tmp, tb));
         RQ_CUDA(h, cudaMemsetAsync(cnt + n, 0, sizeof(int64_t), h->stream));
         cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, h->d_row_start, (int)(n + 1), h->stream);
-        RQ_TRY(sync(h, "row scan"));
     }
     int64_t cap = 0;
     RQ_CUDA(h, cudaMemcpyAsync(&cap, h->d_row_start + n, sizeof(int64_t), cudaMemcpyDeviceToHost, h->stream));
@@ -1106,12 +1261,11 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
     dfree(cnt);
     auto t1 = clk::now();
     if (upper) {
-        // upper-triangle storage: filled chunk by chunk and regrouped into tiles
-        auto t2 = clk::now();
+        int64_t nnz = 0;
         RQ_CUDA(h, cudaEventRecord(ev[2], h->stream));
-        RQ_TRY(fill_tiled<W>(h, v, I, thr, precision, counter, cap, blocks, threads));
+        RQ_TRY(fill_upper64<W>(h, v, I, thr, counter, blocks, threads, nnz));
         RQ_CUDA(h, cudaEventRecord(ev[3], h->stream));
-        return finish_build(h, precision, upper, cap, t0, t1, t2, ev, st);
+        return finish_build(h, precision, upper, cap, nnz, t0, t1, t1, ev, st);
     }
     {
         // refuse up front when the rows cannot be stored, leaving the handle unchanged
@@ -1133,10 +1287,12 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
     auto t2 = clk::now();
     RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
     RQ_CUDA(h, cudaEventRecord(ev[2], h->stream));
-    RQ_TRY(launch_fill<W>(h, v, I, thr, upper, precision, counter, blocks, threads, h->d_cols, h->d_val64, h->d_val32,
-                          h->d_val_lo, 0, n, 0));
+    RQ_TRY((launch_fill<W, OUT_ROWS>(h, v, I, thr, TileOut{}, precision, counter, blocks, threads, h->d_cols, h->d_val64,
+                                     h->d_val32, h->d_val_lo, 0, n, 0)));
     RQ_CUDA(h, cudaEventRecord(ev[3], h->stream));
-    return finish_build(h, precision, upper, cap, t0, t1, t2, ev, st);
+    int64_t nnz = 0;
+    RQ_TRY(count_rows(h, nnz));
+    return finish_build(h, precision, upper, cap, nnz, t0, t1, t2, ev, st);
 }
 
 // Matrix-free FP64 sigma: the build's connection search and Slater-Condon evaluation
@@ -1152,15 +1308,14 @@ int sigma_mf(risqgpu* h, const double* x, double* y) {
     static int cached_dev[2] = {-1, -1}, cached_blocks[2] = {0, 0};
     if (cached_dev[W - 1] != h->device) {
         int occ = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_build_rows<W, 5>, 256, 0);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_build_rows<W, 5, OUT_ROWS>, 256, 0);
         cached_blocks[W - 1] = num_sms(h) * std::max(occ, 1);
         cached_dev[W - 1] = h->device;
     }
     RQ_CUDA(h, cudaMemsetAsync(h->d_mf_counter, 0, sizeof(int), h->stream));
-    k_build_rows<W, 5><<<cached_blocks[W - 1], 256, 0, h->stream>>>(v, I, h->mf_thr, 0, h->d_mf_counter, nullptr,
-                                                                    nullptr, nullptr, nullptr, nullptr, nullptr,
-                                                                    nullptr, 0, (int64_t)h->N, 0,
-                                                                    SigmaIO{x, y, h->d_diag});
+    k_build_rows<W, 5, OUT_ROWS><<<cached_blocks[W - 1], 256, 0, h->stream>>>(
+        v, I, h->mf_thr, TileOut{}, h->d_mf_counter, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0,
+        (int64_t)h->N, 0, SigmaIO{x, y, h->d_diag});
     return check_launch(h, "matrix-free sigma");
 }
 

@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/risqgpu.h"
+#include "tiles.cuh"
 
 namespace risq {
 
@@ -109,34 +110,38 @@ struct risqgpu {
     int* d_mf_counter = nullptr;
     double mf_thr = 0.0;
 
-    // Tiled upper-triangle storage (upper builds).  Rows are cut into panels of
-    // 2^tile_rb consecutive rows and columns into windows of 2^tile_cb.  Each panel
-    // holds its dense (panel, window) tiles, elements coded (row in panel << tile_cb |
-    // column in window), followed by its leftover elements (pairs in tiles too sparse
-    // to stage), coded by their column, in row order.  Values share d_val64 / d_val32
-    // / d_val_lo with the element index.
+    // Tiled upper-triangle storage (upper builds), see tiles.cu.  Rows are cut into panels
+    // of 2^tile_rb consecutive rows and columns into windows of 2^tile_cb; panels into
+    // blocks of 2^tile_kb rows.  A dense (panel, window) tile holds its blocks' rows in
+    // groups of 32; the pairs of sparse tiles are the panel's leftovers.
     bool tiled = false;
-    int tile_rb = 0, tile_cb = 0;
+    int tile_rb = 0, tile_cb = 0, tile_kb = 0;
     int64_t n_panels = 0;
     int64_t n_tiles = 0;
     uint64_t n_dense_el = 0;          // stored pairs in dense tiles
     int64_t* d_panel_tile = nullptr;  // n_panels + 1: first tile of each panel
-    // sigma work units: runs of one panel's tiles of about equal pair counts, largest
-    // first; 3 int64 each: first tile, end tile, panel * 2 + (1 if the unit also takes
-    // the panel's leftover pairs)
-    int64_t n_units = 0;
-    int64_t* d_units = nullptr;
+    int64_t n_units = 0;              // sigma work units, large ones first
+    risq::SigmaUnit* d_units = nullptr;
     int32_t* d_tile_win = nullptr;    // window of each tile
-    float* d_tile_bound = nullptr;    // FP32 values: largest row or column sum of |H| in each tile
-    int32_t* d_tile_len = nullptr;    // elements of each tile
-    int64_t* d_tile_off = nullptr;    // first element of each tile
-    int64_t* d_left_off = nullptr;    // N: first leftover element of each row
-    int32_t* d_left_len = nullptr;    // N: leftover elements of each row
-    uint32_t* d_el_idx = nullptr;     // element index (coded as above)
-    double h_row_abs_max = 0.0;       // max over rows of sum_q |H_pq| (both triangles), for the fixed-point scale
-    // sigma work space, allocated with the matrix: int64 fixed-point accumulators
-    // (N) and two scalars (max |x|, scale)
+    int32_t* d_tile_blk = nullptr;    // n_tiles + 1: first block record of each tile
+    float2* d_tile_bound = nullptr;   // largest row sum of |H| in each tile, bound on its column sums
+    risq::TileBlock* d_tile_blocks = nullptr;
+    std::vector<risq::TileChunk> chunks;  // the element arrays, chunk of panels by chunk
+    risq::TileChunk* d_chunk_tab = nullptr;
+    int64_t* d_left_off = nullptr;    // per panel: first leftover, their number; then their
+    int32_t* d_left_len = nullptr;    // columns, rows in the panel and values
+    uint32_t* d_left_col = nullptr;
+    uint16_t* d_left_row = nullptr;
+    float* d_left32 = nullptr;
+    float* d_left_lo = nullptr;
+    int64_t* d_row_left = nullptr;    // FP64 values: N, first leftover of each row (columns in
+    int32_t* d_row_nleft = nullptr;   // d_left_col), and their number
+    double* d_left64 = nullptr;
+    double h_row_abs_max = 0.0;       // bound on sum_q |H_pq| (both triangles) of any row, for the fixed-point scale
+    // sigma work space, allocated with the matrix: the accumulator (N int64), max |x| per
+    // run of entries, and the scalars of k_sigma_prep
     long long* d_acc = nullptr;
+    double* d_wmax = nullptr;
     double* d_sig_scalars = nullptr;
 
     // Row-block partition for several GPUs (risqgpu_set_partition): this handle builds
@@ -283,7 +288,8 @@ int permute_in(risqgpu* h, const double* x, double* xi);
 int permute_out(risqgpu* h, const double* yi, double* y);
 
 // tiled upper-triangle storage (tiles.cu)
-int tile_shape(int64_t N, int& rb, int& cb);
+int tile_shape(int64_t N, int& rb, int& cb, int& kb);
+int tile_shape64(int64_t N, int& rb, int& cb);
 int sigma_tiles(risqgpu* h, const void* x, void* y, int kind);
 // FP64 sigma of a matrix-free build (build_h.cu), internal order
 int sigma_matrix_free(risqgpu* h, const double* x, double* y);
@@ -297,23 +303,50 @@ int tiles_rows(risqgpu* h, const uint32_t* mark, int64_t* out_r, int64_t* out_c,
 int export_rows_impl(risqgpu* h, const int64_t* rows, size_t k, int64_t* out_r, int64_t* out_c, double* out_v,
                      size_t cap, size_t* count);
 void free_tiles(risqgpu* h);
-// Converts the CSR rows of a build, chunk by chunk of whole panels, into the tiled
-// arrays (d_el_idx and the value arrays must already hold room for every element).
+// Turns the bins that a build's search pass counted and its fill pass filled, chunk by
+// chunk of whole panels, into the tiled arrays.
 struct TileBuilder {
     risqgpu* h = nullptr;
-    unsigned long long* row_abs = nullptr;  // N: sum_q |H_pq| over both triangles, units of 2^-32
-    unsigned long long* absmax = nullptr;
-    size_t tile_cap = 0;
-    int64_t el_cap = 0;
-    int64_t el_next = 0, tile_next = 0;
-    std::vector<int64_t> panel_el;  // host: first element of each panel, and the end
-    int begin(risqgpu* h, int64_t n_panels, int64_t element_capacity);
-    template <typename VIN>
-    int chunk(int64_t p_lo, int64_t p_hi, const int64_t* row_start, int64_t base, const int32_t* row_len,
-              const int32_t* cols, const VIN* vin, const float* vlo_in, VIN* vout, float* vlo_out);
+    int64_t n_blocks = 0;
+    std::vector<PanelCount> counts;                 // per panel, by candidates
+    std::vector<PanelBase> base;                    // per panel, and the end
+    unsigned long long* left_cur = nullptr;         // per panel: next leftover
+    unsigned long long* sums = nullptr;             // row bounds per panel, column bounds per window
+    unsigned long long* counters = nullptr;
+    std::vector<int32_t> panel_chunk;
+    int64_t stored = 0;                             // pairs, after finish
+    int plan(risqgpu* h, const uint32_t* hist, const int64_t* bin_off, int64_t n_blocks);
+    int begin(int64_t p_lo, int64_t p_hi, int precision, const uint32_t* hist, const int64_t* bin_off,
+              unsigned long long* cur);
+    int chunk(int64_t p_lo, int64_t p_hi, int64_t chunk_el0, const unsigned long long* cur, const uint32_t* code,
+              const float* vin, const float* lin);
     int finish();
     int make_units();
     ~TileBuilder();
+};
+
+// The FP64 upper triangle's conversion, from CSR rows, chunk by chunk of whole panels.
+struct Tiles64Builder {
+    risqgpu* h = nullptr;
+    unsigned long long* row_abs = nullptr;          // N: sum_q |H_pq| over both triangles, units of 2^-32
+    unsigned long long* absmax = nullptr;
+    unsigned long long* counters = nullptr;
+    struct Chunk {                                  // what a chunk of panels adds to the arrays
+        int64_t p_lo, p_hi, tiles, left;
+        TileBlock* blocks;
+        int32_t* win;
+        float2* bound;
+        uint32_t* lcol;
+        double* lval;
+    };
+    std::vector<Chunk> parts;
+    std::vector<int64_t> panel_tile;
+    int64_t tiles = 0, left = 0, stored = 0;
+    int begin(risqgpu* h);
+    int chunk(int64_t p_lo, int64_t p_hi, const int64_t* row_start, int64_t base, const int32_t* row_len,
+              const int32_t* cols, const double* vin, uint32_t* code, double* val, int64_t cap);
+    int finish();
+    ~Tiles64Builder();
 };
 
 // davidson (davidson.cu)

@@ -188,22 +188,20 @@ __global__ void k_permute_out(const double* __restrict__ yi, const int32_t* __re
 
 // Second-order self-energy of every determinant over the stored matrix:
 // S_i = -sum_{j != i} H_ij^2 / max(H_jj - E, gmin).  VK as in k_spmv (0 FP64 values,
-// 1 FP32, 2 FP32 + remainder).  Full rows: one warp per row, private sum.  Upper
-// triangle: each stored pair adds to both rows (atomics; `out` zeroed first).
+// 1 FP32, 2 FP32 + remainder).  One warp per row, private sum.
 template <int VK>
 __global__ void __launch_bounds__(256) k_self_energy(int64_t N, const int64_t* __restrict__ row_start,
                                                      const int32_t* __restrict__ row_len,
                                                      const int32_t* __restrict__ cols, const double* __restrict__ v64,
                                                      const float* __restrict__ v32, const float* __restrict__ vlo,
                                                      const double* __restrict__ diag, double energy, double gmin,
-                                                     int upper, double* __restrict__ out) {
+                                                     double* __restrict__ out) {
     const int lane = threadIdx.x & 31;
     const int64_t warp = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     for (int64_t p = warp; p < N; p += nwarps) {
         const int64_t s = row_start[p];
         const int len = row_len[p];
-        const double gp = fmax(diag[p] - energy, gmin);
         double acc = 0.0;
         for (int k = lane; k < len; k += 32) {
             const int c = cols[s + k];
@@ -211,15 +209,10 @@ __global__ void __launch_bounds__(256) k_self_energy(int64_t N, const int64_t* _
             if constexpr (VK == 0) v = v64[s + k];
             else if constexpr (VK == 2) v = (double)v32[s + k] + (double)vlo[s + k];
             else v = (double)v32[s + k];
-            const double v2 = v * v;
-            acc += v2 / fmax(diag[c] - energy, gmin);
-            if (upper) atomicAdd(out + c, -v2 / gp);
+            acc += v * v / fmax(diag[c] - energy, gmin);
         }
         acc = warp_sum(acc);
-        if (lane == 0) {
-            if (upper) atomicAdd(out + p, -acc);
-            else out[p] = -acc;
-        }
+        if (lane == 0) out[p] = -acc;
     }
 }
 
@@ -313,16 +306,15 @@ int self_energy_impl(risqgpu* h, double energy, double gmin, double* out) {
         return sync(h, "self energy");
     }
     const int grid = num_sms(h) * 8;
-    const int up = h->upper ? 1 : 0;
     if (h->precision == RISQGPU_FP64)
         k_self_energy<0><<<grid, 256, 0, h->stream>>>(n, h->d_row_start, h->d_row_len, h->d_cols, h->d_val64, nullptr,
-                                                      nullptr, h->d_diag, energy, gmin, up, si);
+                                                      nullptr, h->d_diag, energy, gmin, si);
     else if (h->precision == RISQGPU_MIXED)
         k_self_energy<2><<<grid, 256, 0, h->stream>>>(n, h->d_row_start, h->d_row_len, h->d_cols, nullptr, h->d_val32,
-                                                      h->d_val_lo, h->d_diag, energy, gmin, up, si);
+                                                      h->d_val_lo, h->d_diag, energy, gmin, si);
     else
         k_self_energy<1><<<grid, 256, 0, h->stream>>>(n, h->d_row_start, h->d_row_len, h->d_cols, nullptr, h->d_val32,
-                                                      nullptr, h->d_diag, energy, gmin, up, si);
+                                                      nullptr, h->d_diag, energy, gmin, si);
     RQ_TRY(check_launch(h, "self energy"));
     RQ_TRY(permute_out(h, si, sc));
     RQ_CUDA(h, cudaMemcpyAsync(out, sc, sizeof(double) * n, cudaMemcpyDeviceToHost, h->stream));
