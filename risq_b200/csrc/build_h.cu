@@ -290,6 +290,7 @@ struct SigmaIO {
     const double* __restrict__ x;
     double* __restrict__ y;
     const double* __restrict__ diag;
+    const int* __restrict__ stop;  // null, or set: do nothing
 };
 
 // MODE 0: count structural candidates per row.  MODE 1/2/3: evaluate and store
@@ -320,6 +321,7 @@ __global__ void __launch_bounds__(256) k_build_rows(SetView<W> v, Ints I, double
                                                     float* __restrict__ vlo, int64_t row_lo, int64_t row_hi,
                                                     int64_t base_off, SigmaIO io) {
     constexpr bool upper = OUT != OUT_ROWS, TILED = OUT == OUT_BINS;
+    if (MODE == 5 && io.stop && *io.stop) return;
     constexpr int WARPS = 256 / 32;
     constexpr int QCAP = 64;  // < 32 pending + 32 new
     __shared__ int s_q[WARPS][2][QCAP];
@@ -1315,7 +1317,7 @@ int sigma_mf(risqgpu* h, const double* x, double* y) {
     RQ_CUDA(h, cudaMemsetAsync(h->d_mf_counter, 0, sizeof(int), h->stream));
     k_build_rows<W, 5, OUT_ROWS><<<cached_blocks[W - 1], 256, 0, h->stream>>>(
         v, I, h->mf_thr, TileOut{}, h->d_mf_counter, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0,
-        (int64_t)h->N, 0, SigmaIO{x, y, h->d_diag});
+        (int64_t)h->N, 0, SigmaIO{x, y, h->d_diag, h->stop_flag});
     return check_launch(h, "matrix-free sigma");
 }
 

@@ -267,6 +267,7 @@ void risqgpu_destroy(risqgpu_t* h) {
     free_mlp(h);
     dfree(h->d_h1);
     dfree(h->d_h2);
+    if (h->pinned) cudaFreeHost(h->pinned);
     if (h->own_stream) {
         cudaStreamSynchronize(h->own_stream);
         cudaStreamDestroy(h->own_stream);

@@ -18,11 +18,12 @@
 // per column); one sigma; one pass for the new projected column.  All
 // reductions are two-stage with a fixed grid, so results are reproducible.
 // The restart takes H*ritz as the combination of the stored H*V columns rather
-// than a fresh sigma (same vector, one sigma fewer).  The host waits twice per
-// iteration: for the residual norms (convergence test) and for the new projected
-// column, which arrives together with the squared norm of the new vector; the
-// reference's dependent-vector exit is therefore taken after that vector's sigma,
-// whose result is dropped.
+// than a fresh sigma (same vector, one sigma fewer).  With one root the host waits
+// once per iteration, after the new projected column (the device decides whether the
+// solve has converged and then skips the rest of the iteration); with several it
+// waits twice, for the residual norms and for the new projected columns.  The squared
+// norm of the new vector arrives with its column; the reference's dependent-vector
+// exit is therefore taken after that vector's sigma, whose result is dropped.
 //
 // MIXED mode keeps V and H*V in FP32 and runs the FP32 sigma; dots, Gram-Schmidt
 // coefficients, the projected matrix and the Ritz vectors stay FP64.  After it
@@ -32,6 +33,7 @@
 #include <chrono>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <utility>
 #include <vector>
 
@@ -44,29 +46,31 @@ int mlp_scale_impl(risqgpu* h, double energy, float* out);
 
 namespace {
 
-// sigma bracketed by CUDA events on the handle's stream; the events are read once the
-// solve has finished (no synchronisation per sigma)
+// sigma bracketed by CUDA events on the handle's stream.  A solve uses a few pairs again
+// and again: they are read after the wait that every iteration has anyway.
 struct SigmaTimer {
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev;
+    size_t used = 0;
     int run(risqgpu* h, const void* x, void* y, int kind) {
-        cudaEvent_t a, b;
-        cudaEventCreate(&a);
-        cudaEventCreate(&b);
-        cudaEventRecord(a, h->stream);
+        if (used == ev.size()) {
+            cudaEvent_t a, b;
+            cudaEventCreate(&a);
+            cudaEventCreate(&b);
+            ev.emplace_back(a, b);
+        }
+        cudaEventRecord(ev[used].first, h->stream);
         int rc = sigma_device(h, x, y, kind);
-        cudaEventRecord(b, h->stream);
-        ev.emplace_back(a, b);
+        cudaEventRecord(ev[used].second, h->stream);
+        used++;
         return rc;
     }
     // after the stream has been synchronised
     void collect(risqgpu* h) {
-        for (auto& e : ev) {
+        for (size_t k = 0; k < used; k++) {
             float ms = 0.f;
-            if (cudaEventElapsedTime(&ms, e.first, e.second) == cudaSuccess) h->sigma_ms_acc += ms;
-            cudaEventDestroy(e.first);
-            cudaEventDestroy(e.second);
+            if (cudaEventElapsedTime(&ms, ev[k].first, ev[k].second) == cudaSuccess) h->sigma_ms_acc += ms;
         }
-        ev.clear();
+        used = 0;
     }
     ~SigmaTimer() {
         for (auto& e : ev) {
@@ -193,7 +197,9 @@ __global__ void __launch_bounds__(DBLK) k_combine(const T* __restrict__ V, const
 }
 
 template <typename T>
-__global__ void k_scale(T* __restrict__ t, int64_t N, const double* __restrict__ nrm2) {
+__global__ void k_scale(T* __restrict__ t, int64_t N, const double* __restrict__ nrm2,
+                        const int* __restrict__ stop = nullptr) {
+    if (stop && *stop) return;
     double s = 1.0 / sqrt(*nrm2);
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x)
         t[i] = (T)((double)t[i] * s);
@@ -248,6 +254,177 @@ __global__ void __launch_bounds__(DBLK) k_ritz(const T* __restrict__ V, const T*
 #pragma unroll
     for (int c = 0; c <= RMAX; c++) out[c] = c < nr ? acc[c] : (c == nr ? acc[RMAX] : 0.0);
     block_reduce_store<RMAX + 1>(out, nr + 1, partial, KMAX + 1);
+}
+
+// ---- one root: an iteration in five launches and one wait --------------------------------
+//
+// At the sizes of early HCI iterations an iteration is bound by launches and waits (6,943
+// determinants: 20 launches, 5 copies and 2 waits, 100 us of which sigma is 7).  For one
+// root the iteration is k_ritz1 (Ritz vector, residual, correction and its first
+// projections), two k_cgs1 (Gram-Schmidt update and the next projections or the norm),
+// k_scale, sigma, and k_dots1 (the projected column), each reduced by the last of its
+// blocks to finish, which puts what the host needs into page-locked memory.  The first
+// kernel also decides whether the solve ends there; the ones after it then do nothing.
+// Every sum is formed in the order of the kernels above (same grid, same tree).
+// Measured: 6,943 determinants 100 -> 38 us an iteration besides sigma.
+
+// Slots of the results, in device and in page-locked memory.
+enum Slot : int { S_RES2 = 0, S_T2 = 1, S_NORM2 = 2, S_STOP = 3, S_COL = 4 };
+
+struct RitzPar {  // Ritz pair of the projected problem
+    double y[KMAX];
+    double lam;
+};
+
+// The sums of `m` columns of partial[nblk][KMAX + 2], formed as k_reduce does, by one warp
+// each; out(j, sum) is called by lane 0.
+template <typename F>
+__device__ __forceinline__ void reduce_slots(const double* __restrict__ partial, int nblk, int m, F out) {
+    const int lane = threadIdx.x & 31;
+    for (int j = threadIdx.x >> 5; j < m; j += DBLK / 32) {
+        double s[DBLK / 32];
+#pragma unroll
+        for (int k = 0; k < DBLK / 32; k++) {
+            s[k] = 0.0;
+            for (int b = lane + 32 * k; b < nblk; b += DBLK) s[k] += __ldcg(partial + b * (KMAX + 2) + j);
+        }
+#pragma unroll
+        for (int o = DBLK / 64; o > 0; o >>= 1)
+#pragma unroll
+            for (int k = 0; k < o; k++) s[k] += s[k + o];
+        double v = s[0];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0) out(j, v);
+    }
+}
+
+// Whether this block is the last of its grid to arrive; the others' writes are then visible.
+__device__ __forceinline__ bool last_block(int* __restrict__ done) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        last = atomicAdd(done, 1) == (int)gridDim.x - 1;
+        if (last) *done = 0;
+    }
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
+// Ritz vector, H ritz, residual, preconditioned correction t (into Vnew, when `room`) and
+// the projections <V_j, t>.  dev: |t|^2, then <V_j, t> from slot S_COL on.
+template <typename T, int CM>
+__global__ void __launch_bounds__(DBLK) k_ritz1(const T* __restrict__ V, const T* __restrict__ HV, int dim, int64_t N,
+                                               RitzPar par, const double* __restrict__ diag,
+                                               const float* __restrict__ fscale, int room, int energy_settled, double tol,
+                                               double* __restrict__ ritz, double* __restrict__ hr, T* __restrict__ Vnew,
+                                               double* __restrict__ partial, int* __restrict__ done,
+                                               double* __restrict__ dev, int* __restrict__ stop,
+                                               double* __restrict__ host) {
+    __shared__ double y[KMAX];
+    if (threadIdx.x < KMAX) y[threadIdx.x] = par.y[threadIdx.x];
+    __syncthreads();
+    const double lam = par.lam;
+    double acc[CM + 2];
+#pragma unroll
+    for (int j = 0; j < CM + 2; j++) acc[j] = 0.0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
+        double rz = 0.0, hz = 0.0;
+#pragma unroll 8
+        for (int j = 0; j < dim; j++) {
+            const double v = (double)V[j * N + i], hv = (double)HV[j * N + i];
+            rz += v * y[j];
+            hz += hv * y[j];
+        }
+        const double d = diag[i];
+        const double f = fscale ? (double)fscale[i] : 1.0;
+        const double r = hz - rz * lam;
+        ritz[i] = rz;
+        hr[i] = hz;
+        acc[0] += r * r;
+        if (room) {
+            const double tc = r / (lam - d) * f;
+            const T tt = (T)tc;
+            Vnew[i] = tt;
+            acc[1] += (double)tt * (double)tt;
+            const double bi = (double)tt;
+#pragma unroll
+            for (int j = 0; j < CM; j++)
+                if (j < dim) acc[2 + j] += (double)V[(int64_t)j * N + i] * bi;
+        }
+    }
+    block_reduce_store<CM + 2>(acc, room ? dim + 2 : 1, partial, KMAX + 2);
+    if (!last_block(done)) return;
+    __shared__ double res[2];
+    reduce_slots(partial, gridDim.x, room ? dim + 2 : 1, [&](int j, double v) {
+        if (j < 2) res[j] = host[j == 0 ? S_RES2 : S_T2] = v;
+        else dev[S_COL + j - 2] = v;
+    });
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const bool end = (sqrt(res[0]) < tol && energy_settled) || (room && sqrt(res[1]) < 1e-9);
+        if (end) *stop = 1;
+        __threadfence_system();
+    }
+}
+
+// t -= sum_{j < m} coef[j] A_j, rounded to the basis type, then the projections <A_j, t>
+// (into out[j]), or with `norm` only |t|^2 (into out[0] and the page-locked result).
+template <typename T, int CM>
+__global__ void __launch_bounds__(DBLK) k_cgs1(const T* __restrict__ A, int m, T* __restrict__ t, int64_t N,
+                                              const double* __restrict__ coef, int norm, double* __restrict__ partial,
+                                              int* __restrict__ done, double* __restrict__ out,
+                                              const int* __restrict__ stop, double* __restrict__ host) {
+    if (*stop) return;
+    __shared__ double c[KMAX];
+    if (threadIdx.x < KMAX) c[threadIdx.x] = threadIdx.x < m ? coef[threadIdx.x] : 0.0;
+    __syncthreads();
+    double acc[CM];
+#pragma unroll
+    for (int j = 0; j < CM; j++) acc[j] = 0.0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
+        double ti = (double)t[i];
+#pragma unroll 8
+        for (int j = 0; j < m; j++) ti -= c[j] * (double)A[(int64_t)j * N + i];
+        const T tt = (T)ti;
+        t[i] = tt;
+        const double bi = (double)tt;
+        if (norm) {
+            acc[0] += bi * bi;
+        } else {
+#pragma unroll
+            for (int j = 0; j < CM; j++)
+                if (j < m) acc[j] += (double)A[(int64_t)j * N + i] * bi;
+        }
+    }
+    block_reduce_store<CM>(acc, norm ? 1 : m, partial, KMAX + 2);
+    if (!last_block(done)) return;
+    reduce_slots(partial, gridDim.x, norm ? 1 : m, [&](int j, double v) {
+        out[j] = v;
+        if (norm) host[S_NORM2] = v;
+    });
+}
+
+// Projected column: <A_j, b> for the columns j < m, into the page-locked result.
+template <typename T, int CM>
+__global__ void __launch_bounds__(DBLK) k_dots1(const T* __restrict__ A, int m, const T* __restrict__ b, int64_t N,
+                                               double* __restrict__ partial, int* __restrict__ done,
+                                               const int* __restrict__ stop, double* __restrict__ host) {
+    if (*stop) return;
+    double acc[CM];
+#pragma unroll
+    for (int j = 0; j < CM; j++) acc[j] = 0.0;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
+        const double bi = (double)b[i];
+#pragma unroll
+        for (int j = 0; j < CM; j++)
+            if (j < m) acc[j] += (double)A[(int64_t)j * N + i] * bi;
+    }
+    block_reduce_store<CM>(acc, m, partial, KMAX + 2);
+    if (!last_block(done)) return;
+    reduce_slots(partial, gridDim.x, m, [&](int j, double v) { host[S_COL + j] = v; });
 }
 
 template <typename T>
@@ -341,7 +518,39 @@ struct Work {
     double* small = nullptr;    // Y + lambda
     double* coef = nullptr;     // KMAX+1
     double* cols = nullptr;     // (RMAX + KMAX) x (KMAX+1): reduced projected columns, then saved norms
+    int* flags = nullptr;       // one-root iterations: blocks done, and whether the solve has ended
+    double* host = nullptr;     // page-locked results (Slot)
     SigmaTimer timer;
+    // One-root iteration up to the new vector: see k_ritz1.
+    template <typename T>
+    int ritz1(const T* V, const T* HV, int dim, const RitzPar& par, const float* fs, bool room, bool settled, double tol,
+              double* ritz, double* hr, T* Vnew) {
+        auto go = [&](auto cm) {
+            constexpr int CM = decltype(cm)::value;
+            k_ritz1<T, CM><<<grid, DBLK, 0, h->stream>>>(V, HV, dim, N, par, h->d_diag, fs, room ? 1 : 0, settled ? 1 : 0,
+                                                         tol, ritz, hr, Vnew, partial, flags, red, flags + 1, host);
+            if (!room) return;
+            k_cgs1<T, CM><<<grid, DBLK, 0, h->stream>>>(V, dim, Vnew, N, red + S_COL, 0, partial, flags, coef, flags + 1,
+                                                        host);
+            k_cgs1<T, CM><<<grid, DBLK, 0, h->stream>>>(V, dim, Vnew, N, coef, 1, partial, flags, red, flags + 1, host);
+            k_scale<T><<<grid, DBLK, 0, h->stream>>>(Vnew, N, red, flags + 1);
+        };
+        if (dim <= 16) go(std::integral_constant<int, 16>{});
+        else if (dim <= 32) go(std::integral_constant<int, 32>{});
+        else go(std::integral_constant<int, KMAX>{});
+        return check_launch(h, "davidson iteration");
+    }
+    template <typename T>
+    int dots1(const T* V, int m, const T* b) {
+        auto go = [&](auto cm) {
+            constexpr int CM = decltype(cm)::value;
+            k_dots1<T, CM><<<grid, DBLK, 0, h->stream>>>(V, m, b, N, partial, flags, flags + 1, host);
+        };
+        if (m <= 16) go(std::integral_constant<int, 16>{});
+        else if (m <= 32) go(std::integral_constant<int, 32>{});
+        else go(std::integral_constant<int, KMAX>{});
+        return check_launch(h, "projected column");
+    }
     // partial dots of the columns j < m of A with b (and <b, b> as column m when self)
     template <typename T>
     int dots(const T* A, int m, const T* b, bool self) {
@@ -431,7 +640,7 @@ int davidson_loop(Work& wk, int nr, const double* init_int, int ninit, bool norm
     if (init_int && (dim > 1 || normalize_init)) {
         for (int c = 0; c < dim; c++) {
             RQ_TRY(orthogonalise(c));
-            k_scale<T><<<g, DBLK, 0, h->stream>>>(V + (size_t)c * N, N, wk.red + c);
+            k_scale<T><<<g, DBLK, 0, h->stream>>>(V + (size_t)c * N, N, wk.red + c, nullptr);
         }
     }
     for (int c = 0; c < dim; c++) RQ_TRY(wk.timer.run(h, V + (size_t)c * N, HV + (size_t)c * N, sigma_kind));
@@ -461,6 +670,13 @@ int davidson_loop(Work& wk, int nr, const double* init_int, int ninit, bool norm
         return RISQGPU_OK;
     };
     RQ_TRY(proj_cols(0, dim, dim, -1));
+    wk.timer.collect(h);
+    // one root: the kernels after the end of the solve look at this flag and do nothing
+    struct StopFlag {
+        risqgpu* h;
+        ~StopFlag() { h->stop_flag = nullptr; }
+    } stop_flag{h};
+    RQ_CUDA(h, cudaMemsetAsync(wk.flags, 0, sizeof(int) * 2, h->stream));
     std::vector<double> last(nr, 0.0);
     if (last_init) for (int c = 0; c < nr; c++) last[c] = last_init[c];
     std::vector<double> w(KMAX), Y(KMAX * KMAX), Pd(KMAX * KMAX), hostsmall(KMAX * RMAX + RMAX), ykeep(KMAX * KMAX);
@@ -474,11 +690,13 @@ int davidson_loop(Work& wk, int nr, const double* init_int, int ninit, bool norm
             for (int j = 0; j < dim; j++) Pd[i * dim + j] = P[i * KMAX + j];
         jacobi_sorted(dim, Pd.data(), w.data(), Y.data());
         const bool room = dim + nr <= mss;
-        for (int j = 0; j < dim; j++)
-            for (int c = 0; c < nr; c++) hostsmall[j * nr + c] = Y[j * dim + c];
-        for (int c = 0; c < nr; c++) hostsmall[dim * nr + c] = w[c];
-        RQ_CUDA(h, cudaMemcpyAsync(wk.small, hostsmall.data(), sizeof(double) * (dim * nr + nr), cudaMemcpyHostToDevice,
-                                   h->stream));
+        if (nr > 1) {
+            for (int j = 0; j < dim; j++)
+                for (int c = 0; c < nr; c++) hostsmall[j * nr + c] = Y[j * dim + c];
+            for (int c = 0; c < nr; c++) hostsmall[dim * nr + c] = w[c];
+            RQ_CUDA(h, cudaMemcpyAsync(wk.small, hostsmall.data(), sizeof(double) * (dim * nr + nr),
+                                       cudaMemcpyHostToDevice, h->stream));
+        }
         // learned scaling: refresh the per-determinant factors when the energy used in
         // their features moved by more than 0.1 Ha (the network is trained on features
         // at the Ritz values of whole trajectories, so coarse refreshes suffice); fall
@@ -501,10 +719,30 @@ int davidson_loop(Work& wk, int nr, const double* init_int, int ninit, bool norm
             if (stalled) out.fallbacks++;
             else fs = fscale;
         }
-        k_ritz<T><<<g, DBLK, 0, h->stream>>>(V, HV, dim, nr, N, wk.small, h->d_diag, fs, room ? 1 : 0, ritz, hr,
-                                             V + (size_t)dim * N, wk.partial);
-        RQ_TRY(check_launch(h, "ritz"));
-        RQ_TRY(wk.reduce(nr + 1, red.data()));
+        if (nr == 1) {
+            RitzPar par;
+            for (int j = 0; j < KMAX; j++) par.y[j] = j < dim ? Y[j * dim] : 0.0;
+            par.lam = w[0];
+            T* t = V + (size_t)dim * N;
+            T* ht = HV + (size_t)dim * N;
+            RQ_TRY(wk.ritz1(V, HV, dim, par, fs, room, std::fabs(w[0] - last[0]) < etol, tol, ritz, hr, t));
+            if (room) {
+                h->stop_flag = wk.flags + 1;
+                const int rc = wk.timer.run(h, t, ht, sigma_kind);
+                h->stop_flag = nullptr;
+                RQ_TRY(rc);
+                RQ_TRY(wk.dots1(V, dim + 1, ht));
+            }
+            RQ_TRY(sync(h, "davidson iteration"));
+            wk.timer.collect(h);
+            red[0] = wk.host[S_RES2];
+            red[1] = wk.host[S_T2];
+        } else {
+            k_ritz<T><<<g, DBLK, 0, h->stream>>>(V, HV, dim, nr, N, wk.small, h->d_diag, fs, room ? 1 : 0, ritz, hr,
+                                                 V + (size_t)dim * N, wk.partial);
+            RQ_TRY(check_launch(h, "ritz"));
+            RQ_TRY(wk.reduce(nr + 1, red.data()));
+        }
         bool all_small = true, all_e = true;
         res_hist.push_back(std::sqrt(red[0]));
         for (int c = 0; c < nr; c++) {
@@ -521,6 +759,17 @@ int davidson_loop(Work& wk, int nr, const double* init_int, int ninit, bool norm
         for (int c = 0; c < nr; c++) last[c] = w[c];
         if (room) {
             if (std::sqrt(red[nr]) < 1e-9) { out.converged = true; out.reason = 1; break; }
+            if (nr == 1) {
+                // the new vector, its sigma and its projected column are already there
+                if (std::sqrt(wk.host[S_NORM2]) < 1e-9) { out.converged = true; out.reason = 2; break; }
+                for (int i = 0; i <= dim; i++) {
+                    P[i * KMAX + dim] = wk.host[S_COL + i];
+                    P[dim * KMAX + i] = wk.host[S_COL + i];
+                }
+                out.n_sigma++;
+                dim++;
+                continue;
+            }
             // slot of the last new vector's squared norm: after the nr projected columns
             const int norm_slot = nr * (KMAX + 1);
             for (int c = 0; c < nr; c++) {
@@ -529,7 +778,7 @@ int davidson_loop(Work& wk, int nr, const double* init_int, int ninit, bool norm
                 if (c == nr - 1)
                     RQ_CUDA(h, cudaMemcpyAsync(wk.cols + norm_slot, wk.red + col, sizeof(double),
                                                cudaMemcpyDeviceToDevice, h->stream));
-                k_scale<T><<<g, DBLK, 0, h->stream>>>(V + (size_t)col * N, N, wk.red + col);
+                k_scale<T><<<g, DBLK, 0, h->stream>>>(V + (size_t)col * N, N, wk.red + col, nullptr);
             }
             for (int c = 0; c < nr; c++)
                 RQ_TRY(wk.timer.run(h, V + (size_t)(dim + c) * N, HV + (size_t)(dim + c) * N, sigma_kind));
@@ -616,13 +865,17 @@ int davidson_impl(risqgpu* h, int nroots, const double* init, int ninit, double 
     wk.N = N;
     double *ritz = nullptr, *hr = nullptr, *init_int = nullptr, *tmp = nullptr, *seed = nullptr, *outv = nullptr;
     float* fscale = nullptr;
-    ScopedFree<5> release_work(wk.partial, wk.red, wk.small, wk.coef, wk.cols);
+    ScopedFree<6> release_work(wk.partial, wk.red, wk.small, wk.coef, wk.cols, wk.flags);
     ScopedFree<7> release_vecs(ritz, hr, init_int, tmp, seed, outv, fscale);
     wk.grid = std::max(1, std::min<int>((int)((N + DBLK - 1) / DBLK), num_sms(h) * 4));
-    RQ_TRY(dalloc(h, wk.partial, (size_t)wk.grid * (KMAX + 1)));
-    RQ_TRY(dalloc(h, wk.red, KMAX + 1));
+    RQ_TRY(dalloc(h, wk.partial, (size_t)wk.grid * (KMAX + 2)));
+    RQ_TRY(dalloc(h, wk.red, S_COL + KMAX + 1));
     RQ_TRY(dalloc(h, wk.small, KMAX * RMAX + RMAX));
     RQ_TRY(dalloc(h, wk.coef, KMAX + 1));
+    RQ_TRY(dalloc(h, wk.flags, 2));
+    if (!h->pinned)
+        RQ_CUDA(h, cudaHostAlloc((void**)&h->pinned, sizeof(double) * (S_COL + KMAX + 1), cudaHostAllocDefault));
+    wk.host = h->pinned;
     RQ_TRY(dalloc(h, wk.cols, (size_t)(KMAX + 2) * (KMAX + 1)));
     RQ_TRY(dalloc(h, ritz, (size_t)nroots * N));
     RQ_TRY(dalloc(h, hr, (size_t)nroots * N));

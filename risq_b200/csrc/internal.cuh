@@ -172,6 +172,11 @@ struct risqgpu {
     int dav_space = 0;
     int dav_keep = 0;
 
+    // page-locked results of a Davidson iteration, and the device flag that a sigma looks at
+    // before it starts (null, or set by a solve that has ended)
+    double* pinned = nullptr;
+    const int* stop_flag = nullptr;
+
     // variational wavefunction of the last risqgpu_variational run (caller order)
     std::vector<uint64_t> wf_dets;
     std::vector<double> wf_coeffs, wf_diag;

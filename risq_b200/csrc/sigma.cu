@@ -43,7 +43,9 @@ __global__ void __launch_bounds__(256, 4) k_spmv(int64_t N, const int64_t* __res
                                                  const int32_t* __restrict__ row_len, const int32_t* __restrict__ cols,
                                                  const double* __restrict__ v64, const float* __restrict__ v32,
                                                  const float* __restrict__ vlo, const double* __restrict__ diag,
-                                                 const X* __restrict__ x, X* __restrict__ y) {
+                                                 const X* __restrict__ x, X* __restrict__ y,
+                                                 const int* __restrict__ stop) {
+    if (stop && *stop) return;
     using A = typename std::conditional<VK == 1, float, double>::type;
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -120,7 +122,8 @@ __global__ void __launch_bounds__(1024, 1) k_spmv_otf(int64_t N, const uint64_t*
                                                       const int32_t* __restrict__ cols,
                                                       const double* __restrict__ diag, Ints Ig, uint32_t n1,
                                                       uint32_t n2, const double* __restrict__ x,
-                                                      double* __restrict__ y) {
+                                                      double* __restrict__ y, const int* __restrict__ stop) {
+    if (stop && *stop) return;
     extern __shared__ double sm[];
     if constexpr (SMEM) {
         for (uint32_t k = threadIdx.x; k < n1; k += blockDim.x) sm[k] = Ig.h1[k];
@@ -164,13 +167,13 @@ int launch_otf(risqgpu* h, const double* x, double* y) {
         RQ_CUDA(h, cudaFuncSetAttribute(k_spmv_otf<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
         k_spmv_otf<W, true><<<num_sms(h), 1024, smem, h->stream>>>(n, h->d_up, h->d_dn, h->d_row_start, h->d_row_len,
                                                                    h->d_cols, h->d_diag, I, (uint32_t)h->n1,
-                                                                   (uint32_t)h->n2, x, y);
+                                                                   (uint32_t)h->n2, x, y, h->stop_flag);
     } else {
         int occ = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_spmv_otf<W, false>, 1024, 0);
         k_spmv_otf<W, false><<<num_sms(h) * std::max(occ, 1), 1024, 0, h->stream>>>(
             n, h->d_up, h->d_dn, h->d_row_start, h->d_row_len, h->d_cols, h->d_diag, I, (uint32_t)h->n1,
-            (uint32_t)h->n2, x, y);
+            (uint32_t)h->n2, x, y, h->stop_flag);
     }
     return check_launch(h, "sigma otf");
 }
@@ -236,10 +239,10 @@ int sigma_device(risqgpu* h, const void* x, void* y, int kind) {
         double* yd = (double*)y;
         if (h->precision == RISQGPU_FP64)
             k_spmv<0, double><<<grid, 256, 0, h->stream>>>(n, h->d_row_start, h->d_row_len, h->d_cols, h->d_val64,
-                                                           nullptr, nullptr, h->d_diag, xd, yd);
+                                                           nullptr, nullptr, h->d_diag, xd, yd, h->stop_flag);
         else if (h->precision == RISQGPU_MIXED)
             k_spmv<2, double><<<grid, 256, 0, h->stream>>>(n, h->d_row_start, h->d_row_len, h->d_cols, nullptr,
-                                                           h->d_val32, h->d_val_lo, h->d_diag, xd, yd);
+                                                           h->d_val32, h->d_val_lo, h->d_diag, xd, yd, h->stop_flag);
         else  // FP32 or columns-only storage: exact FP64 elements recomputed on the fly
             return h->W == 1 ? launch_otf<1>(h, xd, yd) : launch_otf<2>(h, xd, yd);
     } else {
@@ -248,7 +251,7 @@ int sigma_device(risqgpu* h, const void* x, void* y, int kind) {
             return RISQGPU_ERR_INVALID;
         }
         k_spmv<1, float><<<grid, 256, 0, h->stream>>>(n, h->d_row_start, h->d_row_len, h->d_cols, nullptr, h->d_val32,
-                                                      nullptr, h->d_diag, (const float*)x, (float*)y);
+                                                      nullptr, h->d_diag, (const float*)x, (float*)y, h->stop_flag);
     }
     return check_launch(h, "sigma");
 }

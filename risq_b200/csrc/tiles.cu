@@ -702,7 +702,8 @@ __global__ void k_tile_finish64(int64_t nt, int32_t chunk, TileBlock* __restrict
 template <typename X, typename Y>
 __global__ void __launch_bounds__(256) k_sigma_prep(const X* __restrict__ x, int64_t N, int wb, Y* __restrict__ acc,
                                                     double* __restrict__ wmax, double row_abs_max, int smax, int top,
-                                                    double* __restrict__ scalars) {
+                                                    double* __restrict__ scalars, const int* __restrict__ stop) {
+    if (stop && *stop) return;
     __shared__ double s_m[8];
     __shared__ bool s_last;
     auto block_max = [&](double v) {
@@ -838,7 +839,9 @@ __device__ __forceinline__ int fixed_shift(double b, int most) {
 template <typename X, typename V, bool VLO, bool EXACT>
 __global__ void __launch_bounds__(ST, sizeof(X) == 4 ? 6 : 3)
     k_sigma_fx(int64_t N, int64_t n_units, const SigmaUnit* __restrict__ units, TileView<V> T, const X* __restrict__ x,
-               const double* __restrict__ wmax, void* __restrict__ acc_out, double* __restrict__ scalars) {
+               const double* __restrict__ wmax, void* __restrict__ acc_out, double* __restrict__ scalars,
+               const int* __restrict__ stop) {
+    if (stop && *stop) return;
     constexpr bool DBL = std::is_same<X, double>::value;
     constexpr bool V64 = std::is_same<V, double>::value;
     using RS = typename std::conditional<DBL, long long, typename std::conditional<EXACT, int, float>::type>::type;
@@ -1219,8 +1222,8 @@ int launch_fx(risqgpu* h, const X* x, X* y, const TileView<V>& T) {
         (int)std::max<int64_t>(1, std::min<int64_t>(h->n_units, (int64_t)num_sms(h) * std::max(occ, 1)));
     k_sigma_prep<X, Y><<<(int)(((N - 1) >> T.wb) + 1), 256, 0, h->stream>>>(
         x, N, T.wb, reinterpret_cast<Y*>(h->d_acc), h->d_wmax, h->h_row_abs_max,
-        std::is_same<X, float>::value ? 100 : 1000, 61, h->d_sig_scalars);
-    kern<<<grid, ST, smem, h->stream>>>(N, h->n_units, h->d_units, T, x, h->d_wmax, h->d_acc, h->d_sig_scalars);
+        std::is_same<X, float>::value ? 100 : 1000, 61, h->d_sig_scalars, h->stop_flag);
+    kern<<<grid, ST, smem, h->stream>>>(N, h->n_units, h->d_units, T, x, h->d_wmax, h->d_acc, h->d_sig_scalars, h->stop_flag);
     RQ_TRY(check_launch(h, "sigma (tiles)"));
     // with a row-block partition every rank summed its own panels: the exact integer
     // sums are added across the ranks
