@@ -961,8 +961,8 @@ void own_panels(const risqgpu* h, const std::vector<int64_t>& ps, int64_t& lo, i
 // the pairs, so the chunks hold about equal shares.
 int chunk_cuts(risqgpu* h, const std::vector<int64_t>& ps, int64_t own_lo, int64_t own_hi, size_t fixed, size_t per_el,
                std::vector<int64_t>& cuts, int64_t& max_chunk) {
-    const size_t avail = mem_available(h);
     const int64_t own_cap = ps[own_hi] - ps[own_lo], own_np = own_hi - own_lo;
+    const size_t avail = mem_available(h, fixed + (size_t)own_cap * per_el);
     for (int64_t K = 1;; K = K < 8 ? K + 1 : K * 2) {
         cuts.assign(1, own_lo);
         for (int64_t k = 1; k < K; k++) {
@@ -1274,7 +1274,7 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
         size_t vb = precision == RISQGPU_FP64 ? 8 : (precision == RISQGPU_FP32 ? 4 : (precision == RISQGPU_COLS ? 0 : 8));
         const size_t arrays = (size_t)cap * (4 + vb);
         size_t need = arrays + std::max((size_t)8 << 20, std::min((size_t)64 << 20, arrays / 16));
-        const size_t fr = mem_available(h);
+        const size_t fr = mem_available(h, need);
         if (need > fr) {
             h->err = "sparse H needs " + std::to_string(need >> 20) + " MiB, " + std::to_string(fr >> 20) +
                      " MiB available";

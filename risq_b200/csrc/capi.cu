@@ -5,6 +5,7 @@
 #include <mutex>
 #include <new>
 #include <unordered_map>
+#include <vector>
 
 #include "internal.cuh"
 
@@ -12,64 +13,97 @@ namespace risq {
 
 namespace {
 
+// Where a buffer came from.  Buffers below POOL_LARGE: the device's stream-ordered pool.
+// From there to POOL_HUGE: whole blocks kept for reuse, sizes rounded up to a quarter of
+// their power of two, so that one set's matrix fits the blocks another one left; a pool
+// that cuts small buffers, or the first of two large ones, from a freed matrix's hole has
+// to map new memory for the rest (131,611 determinants, three handles in turn: 13 ms a
+// build, against 8 here).  Larger ones, and those of handles with a memory bound: the
+// device.
+enum Source { FROM_DEVICE, FROM_POOL, FROM_BLOCKS };
+constexpr size_t POOL_LARGE = (size_t)64 << 20, POOL_HUGE = (size_t)6 << 30;
+
 struct Buffer {
     risqgpu* h;
-    size_t bytes;
-    int pool;  // -1: allocated from the device directly
+    size_t bytes;   // counted against the handle
+    Source source;
+    size_t held;    // of its block
 };
 std::mutex g_ledger_mu;
 std::unordered_map<void*, Buffer> g_ledger;
 
-// Two pools per device: were the small buffers of set_dets cut from the hole that a freed
-// matrix leaves, the next matrix of that size would not fit it again and would be mapped
-// anew (131,611 determinants, three handles in turn: 13 ms a build, against 8 here).
-constexpr size_t POOL_LARGE = (size_t)64 << 20;  // buffers from this size use the second
-struct Pools {
-    cudaMemPool_t pool[2] = {nullptr, nullptr};
-    size_t keep[2] = {0, 0};   // idle bytes each may hold
-    size_t freed[2] = {0, 0};  // bytes returned to each since its idle bytes were looked at
+struct Block {  // an idle block: free once `done` has passed on the stream it was used on
+    void* p;
+    size_t bytes;
+    cudaStream_t stream;
+    cudaEvent_t done;
+};
+struct Pool {
+    cudaMemPool_t small = nullptr;
+    std::vector<Block> blocks;  // oldest first
+    size_t idle = 0;            // bytes of blocks
+    size_t keep = 0;            // most of them
+    size_t freed = 0;           // bytes returned to the small pool since it was looked at
     int users = 0;
 };
 std::mutex g_pool_mu;
-std::unordered_map<int, Pools> g_pools;
+std::unordered_map<int, Pool> g_pools;
 
-Pools pools_of(int device) {
-    std::lock_guard<std::mutex> lk(g_pool_mu);
-    auto it = g_pools.find(device);
-    return it == g_pools.end() ? Pools{} : it->second;
+size_t block_size(size_t bytes) {
+    size_t unit = POOL_LARGE;
+    while (unit * 2 <= bytes) unit *= 2;
+    unit /= 4;
+    return (bytes + unit - 1) / unit * unit;
+}
+
+void drop_oldest(Pool& P) {  // cudaFree waits for the work that uses the block
+    const Block b = P.blocks.front();
+    P.blocks.erase(P.blocks.begin());
+    P.idle -= b.bytes;
+    cudaFree(b.p);
+    cudaEventDestroy(b.done);
+}
+
+bool pool_bytes(cudaMemPool_t pool, uint64_t& reserved, uint64_t& used) {
+    if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
+        return true;
+    cudaGetLastError();
+    return false;
 }
 
 }  // namespace
 
 int pool_acquire(int device) {
     std::lock_guard<std::mutex> lk(g_pool_mu);
-    Pools& P = g_pools[device];
-    for (int k = 0; k < 2; k++) {
-        cudaMemPool_t& pool = P.pool[k];
-        if (pool) continue;
+    Pool& P = g_pools[device];
+    if (!P.small) {
         cudaMemPoolProps props = {};
         props.allocType = cudaMemAllocationTypePinned;
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = device;
-        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+        if (cudaMemPoolCreate(&P.small, &props) != cudaSuccess) {
             cudaGetLastError();
-            pool = nullptr;
+            P.small = nullptr;
             return RISQGPU_ERR_CUDA;
         }
+        // the pool's own threshold counts the bytes in use too; mem_free bounds the idle ones
+        uint64_t all = UINT64_MAX;
+        cudaMemPoolSetAttribute(P.small, cudaMemPoolAttrReleaseThreshold, &all);
         size_t fr = 0, tot = 0;
         cudaMemGetInfo(&fr, &tot);
-        P.keep[k] = std::min(POOL_KEEP, tot / 8) / (k == 0 ? 8 : 1);
-        // the pool's own threshold counts the bytes in use too; bound_idle bounds the idle ones
-        uint64_t all = UINT64_MAX;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &all);
+        P.keep = std::min(POOL_KEEP, tot / 8);
     }
     P.users++;
     return RISQGPU_OK;
 }
 
 void pool_trim(int device) {
-    for (cudaMemPool_t pool : pools_of(device).pool)
-        if (pool) cudaMemPoolTrimTo(pool, 0);
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    auto it = g_pools.find(device);
+    if (it == g_pools.end()) return;
+    while (!it->second.blocks.empty()) drop_oldest(it->second);
+    if (it->second.small) cudaMemPoolTrimTo(it->second.small, 0);
 }
 
 void pool_release(int device) {
@@ -82,42 +116,13 @@ void pool_release(int device) {
     if (last) pool_trim(device);
 }
 
-namespace {
-
-bool pool_bytes(cudaMemPool_t pool, uint64_t& reserved, uint64_t& used) {
-    if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) == cudaSuccess &&
-        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) == cudaSuccess)
-        return true;
-    cudaGetLastError();
-    return false;
-}
-
-// After `bytes` went back to pool k: every quarter of its idle allowance, give the
-// device what it holds beyond three quarters of it.
-void bound_idle(int device, int k, size_t bytes) {
-    cudaMemPool_t pool = nullptr;
-    size_t keep = 0;
-    {
-        std::lock_guard<std::mutex> lk(g_pool_mu);
-        Pools& P = g_pools[device];
-        P.freed[k] += bytes;
-        if (P.freed[k] < P.keep[k] / 4) return;
-        P.freed[k] = 0;
-        pool = P.pool[k];
-        keep = P.keep[k] / 4 * 3;
-    }
-    uint64_t reserved = 0, used = 0;
-    if (pool_bytes(pool, reserved, used) && reserved > used + keep) cudaMemPoolTrimTo(pool, used + keep);
-}
-
-}  // namespace
-
 size_t pool_idle(int device) {
-    size_t idle = 0;
-    for (cudaMemPool_t pool : pools_of(device).pool) {
-        uint64_t reserved = 0, used = 0;
-        if (pool_bytes(pool, reserved, used) && reserved > used) idle += (size_t)(reserved - used);
-    }
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    auto it = g_pools.find(device);
+    if (it == g_pools.end()) return 0;
+    uint64_t reserved = 0, used = 0;
+    size_t idle = it->second.idle;
+    if (pool_bytes(it->second.small, reserved, used) && reserved > used) idle += (size_t)(reserved - used);
     return idle;
 }
 
@@ -128,27 +133,47 @@ int mem_alloc(risqgpu* h, void** p, size_t bytes) {
                  std::to_string(h->mem_used) + " of " + std::to_string(h->mem_limit) + " bytes in use)";
         return RISQGPU_ERR_OOM;
     }
-    const int which = bytes >= POOL_LARGE;
-    cudaMemPool_t pool = h->mem_limit ? nullptr : pools_of(h->device).pool[which];
-    auto take = [&]() {
-        return pool ? cudaMallocFromPoolAsync(p, bytes, pool, h->stream) : cudaMalloc(p, bytes);
-    };
-    cudaError_t e = take();
-    if (e == cudaErrorMemoryAllocation) {
-        // idle pool memory of the wrong shape may be all that is missing
-        cudaGetLastError();
-        cudaStreamSynchronize(h->stream);
-        pool_trim(h->device);
-        e = take();
+    Buffer b{h, bytes, FROM_DEVICE, bytes};
+    cudaMemPool_t small = nullptr;
+    if (!h->mem_limit && bytes < POOL_HUGE) {
+        b.source = bytes < POOL_LARGE ? FROM_POOL : FROM_BLOCKS;
+        if (b.source == FROM_BLOCKS) b.held = block_size(bytes);
+        std::lock_guard<std::mutex> lk(g_pool_mu);
+        Pool& P = g_pools[h->device];
+        small = P.small;
+        auto best = P.blocks.end();
+        if (b.source == FROM_BLOCKS)
+            best = std::find_if(P.blocks.begin(), P.blocks.end(), [&](const Block& k) { return k.bytes == b.held; });
+        if (best != P.blocks.end()) {
+            if (best->stream != h->stream) cudaStreamWaitEvent(h->stream, best->done, 0);
+            cudaEventDestroy(best->done);
+            *p = best->p;
+            P.idle -= best->bytes;
+            P.blocks.erase(best);
+        }
     }
-    if (e != cudaSuccess) {
-        *p = nullptr;
-        cudaGetLastError();
-        h->err = "device allocation of " + std::to_string(bytes) + " bytes: " + cudaGetErrorString(e);
-        return e == cudaErrorMemoryAllocation ? RISQGPU_ERR_OOM : RISQGPU_ERR_CUDA;
+    if (!*p) {
+        auto take = [&]() {
+            return b.source == FROM_POOL ? cudaMallocFromPoolAsync(p, b.held, small, h->stream) : cudaMalloc(p, b.held);
+        };
+        cudaError_t e = take();
+        if (e == cudaErrorMemoryAllocation) {
+            // idle memory may be all that is missing
+            cudaGetLastError();
+            cudaStreamSynchronize(h->stream);
+            pool_trim(h->device);
+            b.held = bytes;
+            e = take();
+        }
+        if (e != cudaSuccess) {
+            *p = nullptr;
+            cudaGetLastError();
+            h->err = "device allocation of " + std::to_string(bytes) + " bytes: " + cudaGetErrorString(e);
+            return e == cudaErrorMemoryAllocation ? RISQGPU_ERR_OOM : RISQGPU_ERR_CUDA;
+        }
     }
     std::lock_guard<std::mutex> lk(g_ledger_mu);
-    g_ledger[*p] = {h, bytes, pool ? which : -1};
+    g_ledger[*p] = b;
     h->mem_used += bytes;
     return RISQGPU_OK;
 }
@@ -163,12 +188,33 @@ void mem_free(void* p) {
         b.h->mem_used -= b.bytes;
         g_ledger.erase(it);
     }
-    if (b.pool < 0) {
+    if (b.source == FROM_DEVICE) {
         cudaFree(p);
         return;
     }
-    cudaFreeAsync(p, b.h->stream);
-    bound_idle(b.h->device, b.pool, b.bytes);
+    if (b.source == FROM_POOL) cudaFreeAsync(p, b.h->stream);
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    Pool& P = g_pools[b.h->device];
+    if (b.source == FROM_POOL) {
+        // every eighth of the allowance: give the device what is idle beyond it
+        P.freed += b.held;
+        if (P.freed < P.keep / 8) return;
+        P.freed = 0;
+        uint64_t reserved = 0, used = 0;
+        if (pool_bytes(P.small, reserved, used) && reserved > used + P.keep / 8) cudaMemPoolTrimTo(P.small, used + P.keep / 8);
+        return;
+    }
+    Block k{p, b.held, b.h->stream, nullptr};
+    if (cudaEventCreateWithFlags(&k.done, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventRecord(k.done, k.stream) != cudaSuccess) {
+        cudaGetLastError();
+        if (k.done) cudaEventDestroy(k.done);
+        cudaFree(p);
+        return;
+    }
+    P.blocks.push_back(k);
+    P.idle += k.bytes;
+    while (P.idle > P.keep) drop_oldest(P);
 }
 
 }  // namespace risq

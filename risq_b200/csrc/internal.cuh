@@ -191,21 +191,20 @@ namespace risq {
 
 // Device memory of the handles.  Every buffer comes from dalloc and goes back through
 // dfree; a ledger records each one's handle and size (mem_used).  A handle without a
-// memory bound takes its buffers from stream-ordered pools of its device, shared by the
-// process's handles: a build or a solve makes and drops 50 to 90 buffers, and with
-// cudaMalloc / cudaFree those cost more than its kernels (131,611 determinants: 11.4 ms
-// of a 20 ms build; 551,147: 49 of 113 ms).  The pools keep about POOL_KEEP idle bytes at
-// most (and an eighth of the device) for reuse, give everything back when the last handle
-// on the device goes, and are emptied before any allocation is reported as failed.  A
-// handle with a memory bound allocates from the device directly, so that what it holds is
-// what its bound counts.
+// memory bound takes its buffers from memory that the process keeps per device (capi.cu):
+// a build or a solve makes and drops 50 to 90 buffers, and with cudaMalloc / cudaFree those
+// cost more than its kernels (131,611 determinants: 11.4 ms of a 20 ms build; 551,147: 49
+// of 113 ms).  At most POOL_KEEP idle bytes and an eighth more (and an eighth of the device
+// and an eighth more) are kept; all are given back when the last handle on the device goes,
+// and before any allocation is reported as failed.  A handle with a memory bound allocates
+// from the device directly, so that what it holds is what its bound counts.
 constexpr size_t POOL_KEEP = (size_t)12 << 30;
 int mem_alloc(risqgpu* h, void** p, size_t bytes);  // RISQGPU status; sets h->err
 void mem_free(void* p);
 int pool_acquire(int device);  // one call per handle made on the device
 void pool_release(int device);  // one call per handle destroyed, after its buffers
 void pool_trim(int device);
-size_t pool_idle(int device);  // bytes the pools hold that no buffer uses
+size_t pool_idle(int device);  // idle bytes kept
 
 // Free a device pointer (ignores null) and reset it.  Stream-ordered: work already issued
 // on the handle's stream may still use the buffer.
@@ -222,9 +221,13 @@ inline int dalloc(risqgpu* h, T*& p, size_t count) {
     return mem_alloc(h, (void**)&p, count * sizeof(T));
 }
 
-// Device bytes a new allocation may take: free device memory and what the pools could give
-// back, bounded by the handle's limit.
-inline size_t mem_available(risqgpu* h) {
+// Device bytes that new allocations may take: free device memory and what is kept idle,
+// bounded by the handle's limit.  The device is asked only when the idle memory does not
+// cover `need`: on a host whose GPUs are shared cudaMemGetInfo was seen to take from 0.1 to
+// 75 ms (a build of 551,147 determinants: 47 ms).
+inline size_t mem_available(risqgpu* h, size_t need) {
+    const size_t idle = h->mem_limit ? 0 : pool_idle(h->device);
+    if (idle >= need) return idle;
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
         cudaGetLastError();
