@@ -30,6 +30,7 @@
 #include <cstring>
 
 #include "bits.cuh"
+#include "det_table.cuh"
 #include "internal.cuh"
 
 namespace risq {
@@ -176,15 +177,6 @@ __global__ void k_pa_start(const int64_t* __restrict__ off_e, int64_t G, int nup
         pa_start[g] = (int32_t)(g < G ? off_e[g * nup] : total);
 }
 
-// Hash of (alpha group, beta string) for the determinant table (splitmix64 finaliser).
-__device__ __forceinline__ uint64_t det_hash(uint32_t g, uint64_t beta) {
-    uint64_t h = beta * 0x9E3779B97F4A7C15ull ^ ((uint64_t)(g + 1) * 0xC2B2AE3D27D4EB4Full);
-    h ^= h >> 31;
-    h *= 0xBF58476D1CE4E5B9ull;
-    h ^= h >> 29;
-    return h;
-}
-
 // Insert every determinant (one-word strings) into the open-addressing table.  A slot
 // is {beta low, beta high, alpha group, internal index} (16 bytes, one vector load per
 // probe); index -1 marks an empty slot.
@@ -257,19 +249,7 @@ struct SetView {
         for (int k = 0; k < W; k++) b.w[k] = __ldg(up_b + k * N + t);
         return b;
     }
-    // internal index of the determinant (alpha group g, beta string beta), or -1
-    __device__ __forceinline__ int find(int g, uint64_t beta) const {
-        const uint32_t mask = (1u << ht_bits) - 1u;
-        uint32_t slot = (uint32_t)(det_hash((uint32_t)g, beta) >> (64 - ht_bits));
-        const int lo = (int)(uint32_t)beta, hi = (int)(uint32_t)(beta >> 32);
-        for (uint32_t t = 0; t <= mask; t++) {
-            const int4 e = __ldg(ht + slot);
-            if (e.w < 0) return -1;
-            if (e.x == lo && e.y == hi && e.z == g) return e.w;
-            slot = (slot + 1) & mask;
-        }
-        return -1;
-    }
+    __device__ __forceinline__ int find(int g, uint64_t beta) const { return DetTable{ht, ht_bits}.find(g, beta); }
 };
 
 // n-th (0-based) set bit of x; 64 if there is none

@@ -112,45 +112,27 @@ int build_select_tables(risqgpu* h, int ncore, int n_up, int n_dn, SelectTables&
     t.valence[0] = t.valence[1] = 0;
     for (int v : t.valence_orbs) t.valence[v >> 6] |= 1ull << (v & 63);
     const std::vector<int>& vo = t.valence_orbs;
+    const int nv = (int)vo.size();
     t.opp_off.assign((size_t)n * n + 1, 0);
     t.same_off.assign((size_t)n * n + 1, 0);
     t.sing_off.assign((size_t)n + 1, 0);
-    t.r.clear(); t.s.clear(); t.habs.clear();
     t.max_opp = t.max_same = t.max_sing = 0.0;
-    std::vector<std::vector<Entry>> opp((size_t)n * n), same((size_t)n * n), sing(n);
+    // list lengths: (p, q) -> (r, s) with r != p, s != q; p < q -> r < s, neither p nor q
+    std::vector<char> is_v(n, 0);
+    for (int p : vo) is_v[p] = 1;
+    int32_t at = 0;
+    for (int k = 0; k < n * n; k++) {
+        t.opp_off[k] = at;
+        if (is_v[k / n] && is_v[k % n]) at += (nv - 1) * (nv - 1);
+    }
+    t.opp_off[(size_t)n * n] = at;
+    for (int k = 0; k < n * n; k++) {
+        t.same_off[k] = at;
+        if (k / n < k % n && is_v[k / n] && is_v[k % n]) at += (nv - 2) * (nv - 3) / 2;
+    }
+    t.same_off[(size_t)n * n] = at;
+    std::vector<std::vector<Entry>> sing(n);
     std::vector<Entry> v;
-    for (int p : vo)
-        for (int q : vo) {
-            v.clear();
-            for (int r : vo) {
-                if (p == r) continue;
-                for (int s : vo) {
-                    if (q == s) continue;
-                    double hv = std::fabs(I.direct(p, q, r, s));
-                    if (hv > t.max_opp) t.max_opp = hv;
-                    v.push_back({r, s, hv});
-                }
-            }
-            stable_desc(v);
-            opp[(size_t)p * n + q] = v;
-        }
-    for (int p : vo)
-        for (int q : vo) {
-            if (p >= q) continue;
-            v.clear();
-            for (int r : vo) {
-                if (p == r || q == r) continue;
-                for (int s : vo) {
-                    if (r >= s) continue;
-                    if (p == s || q == s) continue;
-                    double hv = std::fabs(I.dpe(p, q, r, s));
-                    if (hv > t.max_same) t.max_same = hv;
-                    v.push_back({r, s, hv});
-                }
-            }
-            stable_desc(v);
-            same[(size_t)p * n + q] = v;
-        }
     std::vector<double> vs, vp;
     for (int p : vo) {
         v.clear();
@@ -183,20 +165,37 @@ int build_select_tables(risqgpu* h, int ncore, int n_up, int n_dn, SelectTables&
         double x = sing[p].empty() ? 0.0 : sing[p][0].h;
         t.max_sing = std::fmax(t.max_sing, x);
     }
-    auto flatten = [&](std::vector<std::vector<Entry>>& lists, std::vector<int32_t>& off) {
-        for (size_t k = 0; k < lists.size(); k++) {
-            off[k] = (int32_t)t.habs.size();
-            for (const Entry& e : lists[k]) {
-                t.r.push_back((uint8_t)e.r);
-                t.s.push_back((uint8_t)e.s);
-                t.habs.push_back(e.h);
-            }
+    std::vector<uint8_t> sr;
+    std::vector<double> sh;
+    for (int p = 0; p < n; p++) {
+        t.sing_off[p] = at + (int32_t)sr.size();
+        for (const Entry& e : sing[p]) {
+            sr.push_back((uint8_t)e.r);
+            sh.push_back(e.h);
         }
-        off[lists.size()] = (int32_t)t.habs.size();
-    };
-    flatten(opp, t.opp_off);
-    flatten(same, t.same_off);
-    flatten(sing, t.sing_off);
+    }
+    t.sing_off[n] = at + (int32_t)sr.size();
+    t.entries = (size_t)at + sr.size();
+    RQ_TRY(sort_double_lists(h, t));
+    if (!sr.empty()) {
+        RQ_CUDA(h, cudaMemcpyAsync(t.d_r + at, sr.data(), sr.size(), cudaMemcpyHostToDevice, h->stream));
+        RQ_CUDA(h, cudaMemsetAsync(t.d_s + at, 0, sr.size(), h->stream));
+        RQ_CUDA(h, cudaMemcpyAsync(t.d_habs + at, sh.data(), sizeof(double) * sh.size(), cudaMemcpyHostToDevice, h->stream));
+    }
+    return sync(h, "excitation tables");
+}
+
+int tables_to_host(risqgpu* h, SelectTables& t) {
+    t.r.resize(t.entries);
+    t.s.resize(t.entries);
+    t.habs.resize(t.entries);
+    RQ_CUDA(h, cudaMemcpyAsync(t.r.data(), t.d_r, t.entries, cudaMemcpyDeviceToHost, h->stream));
+    RQ_CUDA(h, cudaMemcpyAsync(t.s.data(), t.d_s, t.entries, cudaMemcpyDeviceToHost, h->stream));
+    RQ_CUDA(h, cudaMemcpyAsync(t.habs.data(), t.d_habs, sizeof(double) * t.entries, cudaMemcpyDeviceToHost, h->stream));
+    RQ_TRY(sync(h, "excitation tables"));
+    dfree(t.d_r);
+    dfree(t.d_s);
+    dfree(t.d_habs);
     return RISQGPU_OK;
 }
 
@@ -207,6 +206,7 @@ int variational_impl(risqgpu* h, int nup, int ndn, int ncore, double eps_var, in
     if (!(eps_var > 0)) { h->err = "eps_var must be positive"; return RISQGPU_ERR_INVALID; }
     SelectTables tab;
     RQ_TRY(build_select_tables(h, ncore, nup, ndn, tab));
+    RQ_TRY(tables_to_host(h, tab));  // the stage's solves and builds come between its selections
     // HF determinant: lowest nup / ndn orbitals (src/wf/mod.rs:1697-1698)
     uint64_t hf[4] = {0, 0, 0, 0};
     for (int i = 0; i < nup; i++) hf[i >> 6] |= 1ull << (i & 63);

@@ -11,8 +11,7 @@
 // its position in the reference's sequence.  "First occurrence wins" then
 // becomes a stable sort by configuration keeping the first of each run, and the
 // spin-flip pushes become a second stable unique over [flip(d), d] pairs.
-// Membership in the current space is a binary search over the (up, dn)-sorted
-// determinant set the handle already holds.
+// Membership in the current space goes through the handle's determinant table.
 #include <cub/cub.cuh>
 
 #include <algorithm>
@@ -21,6 +20,7 @@
 #include <vector>
 
 #include "bits.cuh"
+#include "det_table.cuh"
 #include "internal.cuh"
 #include "select.cuh"
 
@@ -36,11 +36,18 @@ inline int grid_of(risqgpu* h, int64_t n, int block = 256) {
     return (int)std::max<int64_t>(1, std::min(g, cap));
 }
 
+// Membership in the handle's determinant set, which is sorted by (up, dn).  One-word
+// strings: the alpha string's group by binary search over the unique alpha strings, then
+// one probe of the determinant table (most excited strings are in no group, which ends the
+// test there); two-word strings: binary search over the determinants.
 template <int W>
-struct SortedSet {  // the handle's determinant set, sorted by (up, dn)
+struct SortedSet {
     const uint64_t* __restrict__ up;
     const uint64_t* __restrict__ dn;
     int64_t N;
+    const uint64_t* __restrict__ alpha;  // unique alpha strings, ascending (one-word strings, or null)
+    int32_t G;
+    DetTable table;
     // lexicographic compare of (up, dn) with the most significant word of up first
     __device__ __forceinline__ int cmp(int64_t p, const Bits<W>& a, const Bits<W>& b) const {
 #pragma unroll
@@ -55,18 +62,40 @@ struct SortedSet {  // the handle's determinant set, sorted by (up, dn)
         }
         return 0;
     }
-    __device__ __forceinline__ bool contains(const Bits<W>& a, const Bits<W>& b) const {
-        int64_t lo = 0, hi = N;
+    // group of an alpha string, -1 if the set has none
+    __device__ __forceinline__ int group(uint64_t a) const {
+        int lo = 0, hi = G;
         while (lo < hi) {
-            int64_t mid = (lo + hi) >> 1;
-            int c = cmp(mid, a, b);
-            if (c == 0) return true;
-            if (c < 0) lo = mid + 1;
+            const int mid = (lo + hi) >> 1;
+            const uint64_t x = __ldg(alpha + mid);
+            if (x == a) return mid;
+            if (x < a) lo = mid + 1;
             else hi = mid;
         }
-        return false;
+        return -1;
+    }
+    __device__ __forceinline__ bool contains(const Bits<W>& a, const Bits<W>& b) const {
+        if constexpr (W == 1) {
+            const int g = group(a.w[0]);
+            return g >= 0 && table.find(g, b.w[0]) >= 0;
+        } else {
+            int64_t lo = 0, hi = N;
+            while (lo < hi) {
+                int64_t mid = (lo + hi) >> 1;
+                int c = cmp(mid, a, b);
+                if (c == 0) return true;
+                if (c < 0) lo = mid + 1;
+                else hi = mid;
+            }
+            return false;
+        }
     }
 };
+
+__global__ void k_unique_alpha(const uint64_t* __restrict__ up, const int32_t* __restrict__ ga_start, int32_t G,
+                               uint64_t* __restrict__ alpha) {
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < G; g += gridDim.x * blockDim.x) alpha[g] = up[ga_start[g]];
+}
 
 struct Tables {  // heat-bath lists on the device (see select.cuh)
     const int32_t* __restrict__ opp_off;   // n*n + 1
@@ -85,15 +114,24 @@ __device__ __forceinline__ uint32_t ecode(int kind, int i, int j, int r, int s) 
     return ((uint32_t)kind << 28) | ((uint32_t)i << 21) | ((uint32_t)j << 14) | ((uint32_t)r << 7) | (uint32_t)s;
 }
 
-// One warp per determinant (caller order).  FILL = false: count the candidates
-// of each determinant; FILL = true: write them at off[d].
+// One warp per determinant (caller order).  FILL = false: count the candidates of each
+// determinant; FILL = true: write them at off[d].  Lane l looks at the head of list
+// c0 + l, and the warp then goes through each list that has an entry above eps, 32
+// consecutive entries at a time, so that loads and tests are shared by the lanes (a list
+// per lane read its entries uncoalesced and waited for the longest: 3.3 ms for the fill of
+// 30,011 determinants at eps 1e-3, against 0.9 here).  Candidates keep the order in which
+// the reference visits them: by list, then by entry.
 template <int W, bool FILL>
 __global__ void __launch_bounds__(256) k_expand(const uint64_t* __restrict__ aos, const double* __restrict__ coeff,
                                                 int64_t N, double eps, int singles_on, Tables T, Bits<W> valence,
                                                 Ints I, SortedSet<W> set, int* __restrict__ row_counter,
                                                 int64_t* __restrict__ cnt, const int64_t* __restrict__ off,
                                                 uint64_t* __restrict__ out_cfg, int32_t* __restrict__ out_parent,
-                                                uint32_t* __restrict__ out_code, int64_t M) {
+                                                uint32_t* __restrict__ out_code, int64_t M, int cache) {
+    // cache: entries per warp for the alpha groups of this determinant's single excitations
+    // (i-th valence electron, orbital), looked up when first met; 0 when they do not fit
+    extern __shared__ int32_t s_group[];
+    int32_t* const my_group = s_group + (threadIdx.x >> 5) * cache;
     const int lane = threadIdx.x & 31;
     const int n = T.norb;
     for (;;) {
@@ -105,65 +143,87 @@ __global__ void __launch_bounds__(256) k_expand(const uint64_t* __restrict__ aos
 #pragma unroll
         for (int k = 0; k < W; k++) { up.w[k] = aos[(int64_t)d * 4 + k]; dn.w[k] = aos[(int64_t)d * 4 + 2 + k]; }
         const double local_eps = eps / fabs(coeff[d]);
-        int64_t base = FILL ? off[d] : 0;
+        const int64_t base = FILL ? off[d] : 0;
         int64_t count = 0;
+        int own_group = -1;  // this determinant's alpha group
+        if constexpr (W == 1) own_group = set.group(up.w[0]);
 
-        auto emit_chunk = [&](int my_n, auto&& gen) {
-            // lanes hold my_n candidates each; place them in lane order
-            int incl = my_n;
+        // One list [lo, hi): test(r, s, a2, b2) says whether the entry is a candidate and
+        // fills in its strings.
+        auto walk = [&](int lo, int hi, uint32_t code0, auto&& test) {
+            for (int k0 = lo; k0 < hi; k0 += 32) {
+                const int k = k0 + lane;
+                const bool above = k < hi && !(T.habs[k] < local_eps);
+                int r = 0, s = 0;
+                Bits<W> a2, b2;
+                bool keep = false;
+                if (above) {
+                    r = T.r[k];
+                    s = T.s[k];
+                    keep = test(r, s, a2, b2);
+                }
+                const unsigned m = __ballot_sync(FULL, keep);
+                if (FILL && keep) {
+                    const int64_t pos = base + count + __popc(m & ((1u << lane) - 1u));
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                int y = __shfl_up_sync(FULL, incl, o);
-                if (lane >= o) incl += y;
+                    for (int q = 0; q < W; q++) {
+                        out_cfg[q * M + pos] = a2.w[q];
+                        out_cfg[(W + q) * M + pos] = b2.w[q];
+                    }
+                    out_parent[pos] = d;
+                    out_code[pos] = code0 | ((uint32_t)r << 7) | (uint32_t)s;
+                }
+                count += __popc(m);
+                if (!__all_sync(FULL, above)) break;
             }
-            int total = __shfl_sync(FULL, incl, 31);
-            if (FILL && my_n > 0) gen(base + count + (incl - my_n));
-            count += total;
         };
 
         // (1) opposite-spin doubles (mod.rs:1487-1534)
         if (T.max_opp >= local_eps) {
-            Bits<W> vu = up & valence, vd = dn & valence;
+            const Bits<W> vu = up & valence, vd = dn & valence;
             const int nu = vu.popc(), nd = vd.popc();
             const int npair = nu * nd;
+            __syncwarp();
+            if (W == 1 && cache)
+                for (int k = lane; k < nu * n; k += 32) my_group[k] = -2;
+            __syncwarp();
             for (int c0 = 0; c0 < npair; c0 += 32) {
                 const int pidx = c0 + lane;
-                int i = -1, j = -1;
-                int my_n = 0;
+                int i = 0, j = 0, ii = 0, lo = 0, hi = 0;
                 if (pidx < npair) {
                     Bits<W> t = vu;
-                    for (int k = 0; k < pidx / nd; k++) t.pop_lowest();
+                    ii = pidx / nd;
+                    for (int k = 0; k < ii; k++) t.pop_lowest();
                     i = t.ctz();
                     Bits<W> u = vd;
                     for (int k = 0; k < pidx % nd; k++) u.pop_lowest();
                     j = u.ctz();
-                    const int lo = T.opp_off[i * n + j], hi = T.opp_off[i * n + j + 1];
-                    for (int k = lo; k < hi; k++) {
-                        if (T.habs[k] < local_eps) break;
-                        const int r = T.r[k], s = T.s[k];
-                        if (up.test(r) || dn.test(s)) continue;
-                        Bits<W> nu2 = up, nd2 = dn;
-                        nu2.clear(i); nu2.set(r);
-                        nd2.clear(j); nd2.set(s);
-                        if (!set.contains(nu2, nd2)) my_n++;
-                    }
+                    lo = T.opp_off[i * n + j];
+                    hi = T.opp_off[i * n + j + 1];
                 }
-                emit_chunk(my_n, [&](int64_t pos) {
-                    const int lo = T.opp_off[i * n + j], hi = T.opp_off[i * n + j + 1];
-                    for (int k = lo; k < hi; k++) {
-                        if (T.habs[k] < local_eps) break;
-                        const int r = T.r[k], s = T.s[k];
-                        if (up.test(r) || dn.test(s)) continue;
-                        Bits<W> nu2 = up, nd2 = dn;
-                        nu2.clear(i); nu2.set(r);
-                        nd2.clear(j); nd2.set(s);
-                        if (set.contains(nu2, nd2)) continue;
-                        for (int q = 0; q < W; q++) { out_cfg[q * M + pos] = nu2.w[q]; out_cfg[(W + q) * M + pos] = nd2.w[q]; }
-                        out_parent[pos] = d;
-                        out_code[pos] = ecode(0, i, j, r, s);
-                        pos++;
-                    }
-                });
+                unsigned todo = __ballot_sync(FULL, lo < hi && !(T.habs[lo] < local_eps));
+                while (todo) {
+                    const int src = __ffs(todo) - 1;
+                    todo &= todo - 1;
+                    const int wi = __shfl_sync(FULL, i, src), wj = __shfl_sync(FULL, j, src);
+                    const int wii = __shfl_sync(FULL, ii, src);
+                    walk(__shfl_sync(FULL, lo, src), __shfl_sync(FULL, hi, src), ecode(0, wi, wj, 0, 0),
+                         [&](int r, int s, Bits<W>& a2, Bits<W>& b2) -> bool {
+                             if (up.test(r) || dn.test(s)) return false;
+                             a2 = up;
+                             b2 = dn;
+                             a2.clear(wi); a2.set(r);
+                             b2.clear(wj); b2.set(s);
+                             if constexpr (W == 1) {
+                                 int g;
+                                 if (cache) {
+                                     g = my_group[wii * n + r];
+                                     if (g == -2) my_group[wii * n + r] = g = set.group(a2.w[0]);
+                                 } else g = set.group(a2.w[0]);
+                                 return g < 0 || set.table.find(g, b2.w[0]) < 0;
+                             } else return !set.contains(a2, b2);
+                         });
+                }
             }
         }
         // (2) same-spin doubles (mod.rs:1536-1580)
@@ -175,8 +235,7 @@ __global__ void __launch_bounds__(256) k_expand(const uint64_t* __restrict__ aos
                 const int npair = nv * (nv - 1) / 2;
                 for (int c0 = 0; c0 < npair; c0 += 32) {
                     const int pidx = c0 + lane;
-                    int i = -1, j = -1;
-                    int my_n = 0;
+                    int i = 0, j = 0, lo = 0, hi = 0;
                     if (pidx < npair) {
                         // bit_pairs order: (a, b) with a < b, a-major
                         int a = 0, rem = pidx;
@@ -187,32 +246,26 @@ __global__ void __launch_bounds__(256) k_expand(const uint64_t* __restrict__ aos
                         i = t.ctz();
                         for (int k = a; k < b; k++) t.pop_lowest();
                         j = t.ctz();
-                        const int lo = T.same_off[i * n + j], hi = T.same_off[i * n + j + 1];
-                        for (int k = lo; k < hi; k++) {
-                            if (T.habs[k] < local_eps) break;
-                            const int r = T.r[k], s = T.s[k];
-                            if (x.test(r) || x.test(s)) continue;
-                            Bits<W> nx = x;
-                            nx.clear(i); nx.clear(j); nx.set(r); nx.set(s);
-                            if (!(sp == 0 ? set.contains(nx, dn) : set.contains(up, nx))) my_n++;
-                        }
+                        lo = T.same_off[i * n + j];
+                        hi = T.same_off[i * n + j + 1];
                     }
-                    emit_chunk(my_n, [&](int64_t pos) {
-                        const int lo = T.same_off[i * n + j], hi = T.same_off[i * n + j + 1];
-                        for (int k = lo; k < hi; k++) {
-                            if (T.habs[k] < local_eps) break;
-                            const int r = T.r[k], s = T.s[k];
-                            if (x.test(r) || x.test(s)) continue;
-                            Bits<W> nx = x;
-                            nx.clear(i); nx.clear(j); nx.set(r); nx.set(s);
-                            const Bits<W> a2 = sp == 0 ? nx : up, b2 = sp == 0 ? dn : nx;
-                            if (set.contains(a2, b2)) continue;
-                            for (int q = 0; q < W; q++) { out_cfg[q * M + pos] = a2.w[q]; out_cfg[(W + q) * M + pos] = b2.w[q]; }
-                            out_parent[pos] = d;
-                            out_code[pos] = ecode(1 + sp, i, j, r, s);
-                            pos++;
-                        }
-                    });
+                    unsigned todo = __ballot_sync(FULL, lo < hi && !(T.habs[lo] < local_eps));
+                    while (todo) {
+                        const int src = __ffs(todo) - 1;
+                        todo &= todo - 1;
+                        const int wi = __shfl_sync(FULL, i, src), wj = __shfl_sync(FULL, j, src);
+                        walk(__shfl_sync(FULL, lo, src), __shfl_sync(FULL, hi, src), ecode(1 + sp, wi, wj, 0, 0),
+                             [&](int r, int s, Bits<W>& a2, Bits<W>& b2) -> bool {
+                                 if (x.test(r) || x.test(s)) return false;
+                                 Bits<W> nx = x;
+                                 nx.clear(wi); nx.clear(wj); nx.set(r); nx.set(s);
+                                 a2 = sp == 0 ? nx : up;
+                                 b2 = sp == 0 ? dn : nx;
+                                 if constexpr (W == 1)
+                                     if (sp == 1) return set.table.find(own_group, nx.w[0]) < 0;
+                                 return !set.contains(a2, b2);
+                             });
+                    }
                 }
             }
         }
@@ -221,45 +274,20 @@ __global__ void __launch_bounds__(256) k_expand(const uint64_t* __restrict__ aos
             for (int sp = 0; sp < 2; sp++) {
                 const Bits<W> x = sp == 0 ? up : dn;
                 const Bits<W> other = sp == 0 ? dn : up;
-                const Bits<W> vx = x & valence;
-                const int nv = vx.popc();
-                for (int c0 = 0; c0 < nv; c0 += 32) {
-                    const int pidx = c0 + lane;
-                    int i = -1;
-                    int my_n = 0;
-                    if (pidx < nv) {
-                        Bits<W> t = vx;
-                        for (int k = 0; k < pidx; k++) t.pop_lowest();
-                        i = t.ctz();
-                        const int lo = T.sing_off[i], hi = T.sing_off[i + 1];
-                        for (int k = lo; k < hi; k++) {
-                            if (T.habs[k] < local_eps) break;
-                            const int r = T.r[k];
-                            if (x.test(r)) continue;
-                            Bits<W> nx = x;
-                            nx.clear(i); nx.set(r);
-                            const Bits<W> a2 = sp == 0 ? nx : up, b2 = sp == 0 ? dn : nx;
-                            if (set.contains(a2, b2)) continue;
-                            if (fabs(sc_single<W>(I, x, nx, other)) > local_eps) my_n++;
-                        }
-                    }
-                    emit_chunk(my_n, [&](int64_t pos) {
-                        const int lo = T.sing_off[i], hi = T.sing_off[i + 1];
-                        for (int k = lo; k < hi; k++) {
-                            if (T.habs[k] < local_eps) break;
-                            const int r = T.r[k];
-                            if (x.test(r)) continue;
-                            Bits<W> nx = x;
-                            nx.clear(i); nx.set(r);
-                            const Bits<W> a2 = sp == 0 ? nx : up, b2 = sp == 0 ? dn : nx;
-                            if (set.contains(a2, b2)) continue;
-                            if (!(fabs(sc_single<W>(I, x, nx, other)) > local_eps)) continue;
-                            for (int q = 0; q < W; q++) { out_cfg[q * M + pos] = a2.w[q]; out_cfg[(W + q) * M + pos] = b2.w[q]; }
-                            out_parent[pos] = d;
-                            out_code[pos] = ecode(3 + sp, i, 0, r, 0);
-                            pos++;
-                        }
-                    });
+                Bits<W> vx = x & valence;
+                while (!vx.is_zero()) {
+                    const int i = vx.ctz();
+                    vx.pop_lowest();
+                    walk(T.sing_off[i], T.sing_off[i + 1], ecode(3 + sp, i, 0, 0, 0),
+                         [&](int r, int, Bits<W>& a2, Bits<W>& b2) -> bool {
+                             if (x.test(r)) return false;
+                             Bits<W> nx = x;
+                             nx.clear(i); nx.set(r);
+                             a2 = sp == 0 ? nx : up;
+                             b2 = sp == 0 ? dn : nx;
+                             if (set.contains(a2, b2)) return false;
+                             return fabs(sc_single<W>(I, x, nx, other)) > local_eps;
+                         });
                 }
             }
         }
@@ -518,48 +546,56 @@ int find_new_impl(risqgpu* h, const double* coeffs, double eps, bool singles, co
     RQ_TRY(dalloc(h, dgc, N));
     RQ_CUDA(h, cudaMemcpyAsync(aos, h->h_dets.data(), sizeof(uint64_t) * 4 * N, cudaMemcpyHostToDevice, h->stream));
     RQ_CUDA(h, cudaMemcpyAsync(cf, coeffs, sizeof(double) * N, cudaMemcpyHostToDevice, h->stream));
-    {
-        std::vector<double> dg_int(N), dg_c(N);
-        std::vector<int32_t> orig(N);
-        RQ_CUDA(h, cudaMemcpyAsync(dg_int.data(), h->d_diag, sizeof(double) * N, cudaMemcpyDeviceToHost, h->stream));
-        RQ_CUDA(h, cudaMemcpyAsync(orig.data(), h->d_orig, sizeof(int32_t) * N, cudaMemcpyDeviceToHost, h->stream));
-        RQ_TRY(sync(h, "select prep"));
-        for (int64_t p = 0; p < N; p++) dg_c[orig[p]] = dg_int[p];
-        RQ_CUDA(h, cudaMemcpy(dgc, dg_c.data(), sizeof(double) * N, cudaMemcpyHostToDevice));
-    }
-    // tables
+    RQ_TRY(permute_out(h, h->d_diag, dgc));
+    // tables: on the device already, or brought there for this call
     int32_t *oo = nullptr, *so = nullptr, *go = nullptr;
     uint8_t *tr = nullptr, *ts = nullptr;
     double* th = nullptr;
+    uint64_t* alpha = nullptr;
+    ScopedFree<7> release_tables(oo, so, go, tr, ts, th, alpha);
     RQ_TRY(dalloc(h, oo, tab.opp_off.size()));
     RQ_TRY(dalloc(h, so, tab.same_off.size()));
     RQ_TRY(dalloc(h, go, tab.sing_off.size()));
-    RQ_TRY(dalloc(h, tr, tab.r.size()));
-    RQ_TRY(dalloc(h, ts, tab.s.size()));
-    RQ_TRY(dalloc(h, th, tab.habs.size()));
     RQ_CUDA(h, cudaMemcpyAsync(oo, tab.opp_off.data(), 4 * tab.opp_off.size(), cudaMemcpyHostToDevice, h->stream));
     RQ_CUDA(h, cudaMemcpyAsync(so, tab.same_off.data(), 4 * tab.same_off.size(), cudaMemcpyHostToDevice, h->stream));
     RQ_CUDA(h, cudaMemcpyAsync(go, tab.sing_off.data(), 4 * tab.sing_off.size(), cudaMemcpyHostToDevice, h->stream));
-    RQ_CUDA(h, cudaMemcpyAsync(tr, tab.r.data(), tab.r.size(), cudaMemcpyHostToDevice, h->stream));
-    RQ_CUDA(h, cudaMemcpyAsync(ts, tab.s.data(), tab.s.size(), cudaMemcpyHostToDevice, h->stream));
-    RQ_CUDA(h, cudaMemcpyAsync(th, tab.habs.data(), 8 * tab.habs.size(), cudaMemcpyHostToDevice, h->stream));
-    Tables T{oo, so, go, tr, ts, th, h->norb, tab.max_opp, tab.max_same, tab.max_sing};
+    if (!tab.d_habs) {
+        RQ_TRY(dalloc(h, tr, tab.r.size()));
+        RQ_TRY(dalloc(h, ts, tab.s.size()));
+        RQ_TRY(dalloc(h, th, tab.habs.size()));
+        RQ_CUDA(h, cudaMemcpyAsync(tr, tab.r.data(), tab.r.size(), cudaMemcpyHostToDevice, h->stream));
+        RQ_CUDA(h, cudaMemcpyAsync(ts, tab.s.data(), tab.s.size(), cudaMemcpyHostToDevice, h->stream));
+        RQ_CUDA(h, cudaMemcpyAsync(th, tab.habs.data(), 8 * tab.habs.size(), cudaMemcpyHostToDevice, h->stream));
+    }
+    Tables T{oo, so, go, tab.d_habs ? tab.d_r : tr, tab.d_habs ? tab.d_s : ts, tab.d_habs ? tab.d_habs : th, h->norb,
+             tab.max_opp, tab.max_same, tab.max_sing};
     Bits<W> val;
     for (int q = 0; q < W; q++) val.w[q] = tab.valence[q];
     Ints I{h->d_h1, h->d_h2, h->nuc};
-    SortedSet<W> set{h->d_up, h->d_dn, N};
+    if (W == 1) {
+        RQ_TRY(dalloc(h, alpha, (size_t)h->G_a));
+        k_unique_alpha<<<grid_of(h, h->G_a), 256, 0, h->stream>>>(h->d_up, h->d_ga_start, h->G_a, alpha);
+        RQ_TRY(check_launch(h, "unique alpha strings"));
+    }
+    SortedSet<W> set{h->d_up, h->d_dn, N, alpha, h->G_a, DetTable{h->d_ht, h->ht_bits}};
+    // alpha groups of single excitations, per warp, when eight warps' fit 64 KiB
+    int cache = W == 1 ? h->n_up * h->norb : 0;
+    if ((size_t)cache * 8 * sizeof(int32_t) > ((size_t)64 << 10)) cache = 0;
+    const size_t smem = (size_t)cache * 8 * sizeof(int32_t);
+    RQ_CUDA(h, cudaFuncSetAttribute(k_expand<W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    RQ_CUDA(h, cudaFuncSetAttribute(k_expand<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int* counter = nullptr;
     int64_t *cnt = nullptr, *off = nullptr;
     RQ_TRY(dalloc(h, counter, 1));
     RQ_TRY(dalloc(h, cnt, N + 1));
     RQ_TRY(dalloc(h, off, N + 1));
     int occ = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_expand<W, true>, 256, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_expand<W, true>, 256, smem);
     const int blocks = num_sms(h) * std::max(occ, 1);
     RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
     RQ_CUDA(h, cudaMemsetAsync(cnt + N, 0, sizeof(int64_t), h->stream));
-    k_expand<W, false><<<blocks, 256, 0, h->stream>>>(aos, cf, N, eps, singles ? 1 : 0, T, val, I, set, counter, cnt,
-                                                      nullptr, nullptr, nullptr, nullptr, 0);
+    k_expand<W, false><<<blocks, 256, smem, h->stream>>>(aos, cf, N, eps, singles ? 1 : 0, T, val, I, set, counter, cnt,
+                                                      nullptr, nullptr, nullptr, nullptr, 0, cache);
     RQ_TRY(check_launch(h, "expand count"));
     {
         size_t tb = 0;
@@ -581,8 +617,8 @@ int find_new_impl(risqgpu* h, const double* coeffs, double eps, bool singles, co
         RQ_TRY(dalloc(h, parent, M));
         RQ_TRY(dalloc(h, code, M));
         RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
-        k_expand<W, true><<<blocks, 256, 0, h->stream>>>(aos, cf, N, eps, singles ? 1 : 0, T, val, I, set, counter,
-                                                         nullptr, off, cfg, parent, code, M);
+        k_expand<W, true><<<blocks, 256, smem, h->stream>>>(aos, cf, N, eps, singles ? 1 : 0, T, val, I, set, counter,
+                                                         nullptr, off, cfg, parent, code, M, cache);
         RQ_TRY(check_launch(h, "expand fill"));
         // first occurrence of each configuration
         int64_t* idx = nullptr;
@@ -627,12 +663,132 @@ int find_new_impl(risqgpu* h, const double* coeffs, double eps, bool singles, co
     } else if (st) {
         st->unique = st->added = 0;
     }
-    dfree(aos); dfree(cf); dfree(dgc); dfree(oo); dfree(so); dfree(go); dfree(tr); dfree(ts); dfree(th);
+    dfree(aos); dfree(cf); dfree(dgc);
     dfree(counter); dfree(cnt); dfree(off);
     return RISQGPU_OK;
 }
 
 }  // namespace
+
+namespace {
+
+// |H| of the opposite-spin doubles (p, q) -> (r, s), one block per (p, q), in the
+// reference's loop order: r over the valence orbitals but p, s over those but q.
+__global__ void k_opp_lists(Ints I, int n, int nv, const uint8_t* __restrict__ vo, const int32_t* __restrict__ off,
+                            double* __restrict__ key, uint16_t* __restrict__ rs) {
+    __shared__ uint8_t vr[128], vs[128];  // the valence orbitals without p, without q
+    const int p = blockIdx.x / n, q = blockIdx.x % n;
+    const int m = nv - 1, lo = off[blockIdx.x], len = off[blockIdx.x + 1] - lo;
+    if (len == 0) return;
+    for (int k = threadIdx.x; k < nv; k += blockDim.x) {
+        const int o = vo[k];
+        int kp = 0, kq = 0;
+        while (vo[kp] != p) kp++;
+        while (vo[kq] != q) kq++;
+        if (o != p) vr[k - (k > kp)] = (uint8_t)o;
+        if (o != q) vs[k - (k > kq)] = (uint8_t)o;
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < len; t += blockDim.x) {
+        const int r = vr[t / m], s = vs[t % m];
+        key[lo + t] = fabs(direct(I, p, q, r, s));
+        rs[lo + t] = (uint16_t)((r << 8) | s);
+    }
+}
+
+// |H| of the same-spin doubles (p < q) -> (r < s), one warp per (p, q): r, then s, over the
+// valence orbitals but p and q, pairs with r >= s left out.
+__global__ void k_same_lists(Ints I, int n, int nv, const uint8_t* __restrict__ vo, const int32_t* __restrict__ off,
+                             double* __restrict__ key, uint16_t* __restrict__ rs) {
+    const int p = blockIdx.x / n, q = blockIdx.x % n, lane = threadIdx.x;
+    int at = off[blockIdx.x];
+    if (off[blockIdx.x + 1] == at) return;
+    for (int t0 = 0; t0 < nv * nv; t0 += 32) {
+        const int t = t0 + lane;
+        int r = 0, s = 0;
+        bool ok = t < nv * nv;
+        if (ok) {
+            r = vo[t / nv];
+            s = vo[t % nv];
+            ok = r < s && r != p && r != q && s != p && s != q;
+        }
+        const unsigned m = __ballot_sync(FULL, ok);
+        if (ok) {
+            const int k = at + __popc(m & ((1u << lane) - 1u));
+            key[k] = fabs(dpe(I, p, q, r, s));
+            rs[k] = (uint16_t)((r << 8) | s);
+        }
+        at += __popc(m);
+    }
+}
+
+__global__ void k_split_rs(const uint16_t* __restrict__ rs, int64_t n, uint8_t* __restrict__ r, uint8_t* __restrict__ s) {
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        r[i] = (uint8_t)(rs[i] >> 8);
+        s[i] = (uint8_t)(rs[i] & 255);
+    }
+}
+
+// Largest |H| of sorted lists: of their first entries.
+__global__ void k_list_max(const double* __restrict__ key, const int32_t* __restrict__ off, int segs,
+                           unsigned long long* __restrict__ out) {
+    unsigned long long m = 0ull;  // bits of non-negative doubles order like the doubles
+    for (int k = threadIdx.x; k < segs; k += blockDim.x)
+        if (off[k + 1] > off[k]) m = max(m, (unsigned long long)__double_as_longlong(key[off[k]]));
+    atomicMax(out, m);
+}
+
+}  // namespace
+
+int sort_double_lists(risqgpu* h, SelectTables& t) {
+    const int n = h->norb, nv = (int)t.valence_orbs.size(), segs = n * n;
+    const int32_t total = t.same_off.back();
+    RQ_TRY(dalloc(h, t.d_r, t.entries));
+    RQ_TRY(dalloc(h, t.d_s, t.entries));
+    RQ_TRY(dalloc(h, t.d_habs, t.entries));
+    if (total == 0) return RISQGPU_OK;
+    // list starts of both kinds in one array: the opposite-spin lists, then the same-spin ones
+    std::vector<int32_t> off(t.opp_off.begin(), t.opp_off.end() - 1);
+    off.insert(off.end(), t.same_off.begin(), t.same_off.end());
+    std::vector<uint8_t> vo(t.valence_orbs.begin(), t.valence_orbs.end());
+    int32_t* doff = nullptr;
+    uint8_t* dvo = nullptr;
+    double* key = nullptr;
+    uint16_t *rs = nullptr, *rs2 = nullptr;
+    char* tmp = nullptr;
+    unsigned long long* mx = nullptr;
+    ScopedFree<7> release(doff, dvo, key, rs, rs2, tmp, mx);
+    RQ_TRY(dalloc(h, doff, off.size()));
+    RQ_TRY(dalloc(h, dvo, vo.size()));
+    RQ_TRY(dalloc(h, key, (size_t)total));
+    RQ_TRY(dalloc(h, rs, (size_t)total));
+    RQ_TRY(dalloc(h, rs2, (size_t)total));
+    RQ_TRY(dalloc(h, mx, 2));
+    RQ_CUDA(h, cudaMemcpyAsync(doff, off.data(), 4 * off.size(), cudaMemcpyHostToDevice, h->stream));
+    RQ_CUDA(h, cudaMemcpyAsync(dvo, vo.data(), vo.size(), cudaMemcpyHostToDevice, h->stream));
+    RQ_CUDA(h, cudaMemsetAsync(mx, 0, 16, h->stream));
+    Ints I{h->d_h1, h->d_h2, h->nuc};
+    k_opp_lists<<<segs, 128, 0, h->stream>>>(I, n, nv, dvo, doff, key, rs);
+    k_same_lists<<<segs, 32, 0, h->stream>>>(I, n, nv, dvo, doff + segs, key, rs);
+    RQ_TRY(check_launch(h, "double lists"));
+    // falling |H|, equal ones in loop order
+    size_t tb = 0;
+    cub::DeviceSegmentedSort::StableSortPairsDescending(nullptr, tb, key, t.d_habs, rs, rs2, total, 2 * segs, doff, doff + 1,
+                                                        h->stream);
+    RQ_TRY(dalloc(h, tmp, tb));
+    cub::DeviceSegmentedSort::StableSortPairsDescending(tmp, tb, key, t.d_habs, rs, rs2, total, 2 * segs, doff, doff + 1,
+                                                        h->stream);
+    k_split_rs<<<grid_of(h, total), 256, 0, h->stream>>>(rs2, total, t.d_r, t.d_s);
+    k_list_max<<<1, 1024, 0, h->stream>>>(t.d_habs, doff, segs, mx);
+    k_list_max<<<1, 1024, 0, h->stream>>>(t.d_habs, doff + segs, segs, mx + 1);
+    RQ_TRY(check_launch(h, "sorted double lists"));
+    double m[2] = {0.0, 0.0};
+    RQ_CUDA(h, cudaMemcpyAsync(m, mx, 16, cudaMemcpyDeviceToHost, h->stream));
+    RQ_TRY(sync(h, "double lists"));
+    t.max_opp = m[0];
+    t.max_same = m[1];
+    return RISQGPU_OK;
+}
 
 int find_new_dets_impl(risqgpu* h, const double* coeffs, double eps, bool singles, const SelectTables& tab,
                        std::vector<uint64_t>& new_dets, std::vector<double>& new_diag, SelectStats* st) {
