@@ -1000,13 +1000,21 @@ int fill_upper64(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int
     const int64_t own_lo = h->part_p_lo, own_hi = h->part_p_hi;
     // rows of other ranks' panels hold no stored pairs here
     RQ_CUDA(h, cudaMemsetAsync(h->d_row_len, 0, sizeof(int32_t) * n, h->stream));
-    // bytes of the tiled arrays (10 an element, an eighth more for padding and headers),
-    // per row tile data and accumulators, plus a margin that grows with the set
-    const size_t base_need = (size_t)(ps[own_hi] - ps[own_lo]) * 10 / 8 * 9 + (size_t)n * 40;
-    const size_t fixed = base_need + std::max((size_t)8 << 20, std::min((size_t)256 << 20, base_need / 32));
+    // bytes of the tiled arrays, per row tile data and accumulators, plus a margin that grows
+    // with the set.  An element takes 10 bytes, about an eighth more for its group's padding,
+    // and its share of the group's slots (136 bytes a group; 1.0 at the four elements a row
+    // and tile of a 9,150,723-determinant set): chunks are cut for 14, and for 11.25, below
+    // what any set takes, only where 14 would refuse a set that may fit.
+    const int64_t own_cap = ps[own_hi] - ps[own_lo];
+    auto fixed_for = [&](size_t quarters) {
+        const size_t need = (size_t)own_cap * quarters / 4 + (size_t)n * 40;
+        return need + std::max((size_t)8 << 20, std::min((size_t)256 << 20, need / 32));
+    };
     std::vector<int64_t> cuts;
     int64_t max_chunk = 0;
-    RQ_TRY(chunk_cuts(h, ps, own_lo, own_hi, fixed, 24, cuts, max_chunk));
+    if (chunk_cuts(h, ps, own_lo, own_hi, fixed_for(56), 24, cuts, max_chunk) != RISQGPU_OK)
+        RQ_TRY(chunk_cuts(h, ps, own_lo, own_hi, fixed_for(45), 24, cuts, max_chunk));
+    h->err.clear();
     int32_t* ccols = nullptr;
     uint32_t* code = nullptr;
     double *c64 = nullptr, *t64 = nullptr;
@@ -1024,6 +1032,8 @@ int fill_upper64(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int
                                           nullptr, nullptr, p_lo << rb, std::min(n, p_hi << rb), ps[p_lo])));
         RQ_TRY(tb.chunk(p_lo, p_hi, h->d_row_start, ps[p_lo], h->d_row_len, ccols, c64, code, t64, max_chunk));
     }
+    // the chunk's arrays go before the leftovers of all chunks are gathered
+    dfree(ccols); dfree(c64); dfree(code); dfree(t64);
     RQ_TRY(tb.finish());
     RQ_TRY(count_rows(h, nnz));
     // every stored element went into the tiles or the leftovers exactly once

@@ -137,9 +137,14 @@ int mem_alloc(risqgpu* h, void** p, size_t bytes) {
     cudaMemPool_t small = nullptr;
     if (!h->mem_limit && bytes < POOL_HUGE) {
         b.source = bytes < POOL_LARGE ? FROM_POOL : FROM_BLOCKS;
-        if (b.source == FROM_BLOCKS) b.held = block_size(bytes);
         std::lock_guard<std::mutex> lk(g_pool_mu);
         Pool& P = g_pools[h->device];
+        // A handle that holds more than is ever kept idle gets the bytes it asks for: the
+        // rounding of its many large buffers would take memory that the build counts on.
+        if (b.source == FROM_BLOCKS) {
+            if (h->mem_used + bytes > P.keep) b.source = FROM_DEVICE;
+            else b.held = block_size(bytes);
+        }
         small = P.small;
         auto best = P.blocks.end();
         if (b.source == FROM_BLOCKS)
