@@ -977,9 +977,9 @@ __global__ void k_panel_starts(const int64_t* __restrict__ row_start, int64_t n,
 // holds one chunk, each chunk regrouped into tiles before the next is filled.
 template <int W>
 int fill_upper64(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int* counter, int blocks, int threads,
-                 int64_t& nnz) {
+                 int64_t cap, int64_t& nnz) {
     const int64_t n = (int64_t)h->N;
-    if (tile_shape64(n, h->tile_rb, h->tile_cb) != RISQGPU_OK) {
+    if (tile_shape64(n, cap, h->tile_rb, h->tile_cb) != RISQGPU_OK) {
         h->err = "determinant set too large for the tiled upper-triangle layout";
         return RISQGPU_ERR_INVALID;
     }
@@ -1255,7 +1255,7 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
     if (upper) {
         int64_t nnz = 0;
         RQ_CUDA(h, cudaEventRecord(ev[2], h->stream));
-        RQ_TRY(fill_upper64<W>(h, v, I, thr, counter, blocks, threads, nnz));
+        RQ_TRY(fill_upper64<W>(h, v, I, thr, counter, blocks, threads, cap, nnz));
         RQ_CUDA(h, cudaEventRecord(ev[3], h->stream));
         return finish_build(h, precision, upper, cap, nnz, t0, t1, t1, ev, st);
     }

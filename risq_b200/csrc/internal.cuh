@@ -297,7 +297,7 @@ int permute_out(risqgpu* h, const double* yi, double* y);
 
 // tiled upper-triangle storage (tiles.cu)
 int tile_shape(int64_t N, int& rb, int& cb, int& kb);
-int tile_shape64(int64_t N, int& rb, int& cb);
+int tile_shape64(int64_t N, int64_t pairs, int& rb, int& cb);
 int sigma_tiles(risqgpu* h, const void* x, void* y, int kind);
 // FP64 sigma of a matrix-free build (build_h.cu), internal order
 int sigma_matrix_free(risqgpu* h, const double* x, double* y);

@@ -1298,9 +1298,14 @@ int tile_shape(int64_t N, int& rb, int& cb, int& kb) {
     return ((N + ((int64_t)1 << cb) - 1) >> cb) <= 65536 ? RISQGPU_OK : RISQGPU_ERR_INVALID;
 }
 
-int tile_shape64(int64_t N, int& rb, int& cb) {
+int tile_shape64(int64_t N, int64_t pairs, int& rb, int& cb) {
     rb = 10;  // 1024 rows per panel
-    cb = 11;  // 2048 columns per window
+    // 2048 columns per window; 4096 where a row has less than one pair in such a window on
+    // average, since a row's slot, x_p and row sum cost as much as several pairs: 9,150,723
+    // determinants (0.54 pairs), FP64 sigma 63.3 ms at 2048, 56.7 at 4096.  Sets of up to
+    // 551,147 determinants have 4 and more.
+    const int64_t half = ((N + 2047) >> 11) / 2;
+    cb = pairs < N * half ? 12 : 11;
     while (cb < 16 && ((N + ((int64_t)1 << cb) - 1) >> cb) > MAX_BINS) cb++;
     return ((N + ((int64_t)1 << cb) - 1) >> cb) <= MAX_BINS ? RISQGPU_OK : RISQGPU_ERR_INVALID;
 }
