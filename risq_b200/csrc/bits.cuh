@@ -1,7 +1,8 @@
 // Determinant strings and Slater-Condon matrix elements on the device.
 //
 // A spin string of up to 64*W orbitals lives in W 64-bit words (W = 1 for
-// norb <= 64, W = 2 up to the reference's u128 limit).  Every function below
+// norb <= 64, W = 2 up to the reference's u128 limit); W = 0 holds one of up to 32 in a
+// 32-bit register.  Every function below
 // reproduces the reference's FP64 arithmetic operation for operation, so the
 // elements it returns are bitwise equal to the CPU ones:
 //   ham_sing          src/ham/mod.rs:135-168
@@ -100,6 +101,27 @@ struct Bits {
         }
         return r;
     }
+};
+
+// Strings of up to 32 orbitals in one register, for the kernels that are bound by integer
+// instructions: the same operations take half of those of a 64-bit word or less (a set bit's
+// index or a shift takes a third).  Memory holds the words of Bits<1>.
+template <>
+struct Bits<0> {
+    uint32_t v;
+
+    __device__ __forceinline__ Bits operator^(const Bits& o) const { return {v ^ o.v}; }
+    __device__ __forceinline__ Bits operator&(const Bits& o) const { return {v & o.v}; }
+    __device__ __forceinline__ Bits operator|(const Bits& o) const { return {v | o.v}; }
+    __device__ __forceinline__ Bits andnot(const Bits& o) const { return {v & ~o.v}; }
+    __device__ __forceinline__ bool operator==(const Bits& o) const { return v == o.v; }
+    __device__ __forceinline__ bool operator!=(const Bits& o) const { return v != o.v; }
+    __device__ __forceinline__ bool is_zero() const { return v == 0; }
+    __device__ __forceinline__ int popc() const { return __popc(v); }
+    // index of the lowest set bit (caller guarantees non-zero)
+    __device__ __forceinline__ int ctz() const { return __ffs((int)v) - 1; }
+    __device__ __forceinline__ void pop_lowest() { v &= v - 1; }
+    __device__ __forceinline__ static Bits below(int b) { return {b >= 32 ? ~0u : (1u << b) - 1u}; }
 };
 
 // parity(n) of src/utils/bits.rs:171-180: +1 for an even popcount.

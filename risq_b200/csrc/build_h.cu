@@ -217,7 +217,8 @@ struct SetView {
     const int32_t* __restrict__ orig;
     int64_t nsh;
     int norb;
-    // (alpha group, beta string) -> internal index, or null (two-word strings)
+    // (alpha group, beta string) -> internal index, or null (two-word strings; W = 0 reads
+    // the low halves of one-word ones)
     const int4* __restrict__ ht;
     int ht_bits;
     // previous build (incremental extension)
@@ -231,24 +232,18 @@ struct SetView {
     const float* __restrict__ prev_v32;
     const float* __restrict__ prev_vlo;
 
-    __device__ __forceinline__ Bits<W> up_at(int64_t p) const {
+    __device__ __forceinline__ Bits<W> load(const uint64_t* __restrict__ s, int64_t p) const {
         Bits<W> b;
+        if constexpr (W == 0) b.v = __ldg(reinterpret_cast<const uint32_t*>(s) + 2 * p);
+        else {
 #pragma unroll
-        for (int k = 0; k < W; k++) b.w[k] = __ldg(up + k * N + p);
+            for (int k = 0; k < W; k++) b.w[k] = __ldg(s + k * N + p);
+        }
         return b;
     }
-    __device__ __forceinline__ Bits<W> dn_at(int64_t p) const {
-        Bits<W> b;
-#pragma unroll
-        for (int k = 0; k < W; k++) b.w[k] = __ldg(dn + k * N + p);
-        return b;
-    }
-    __device__ __forceinline__ Bits<W> upb_at(int64_t t) const {
-        Bits<W> b;
-#pragma unroll
-        for (int k = 0; k < W; k++) b.w[k] = __ldg(up_b + k * N + t);
-        return b;
-    }
+    __device__ __forceinline__ Bits<W> up_at(int64_t p) const { return load(up, p); }
+    __device__ __forceinline__ Bits<W> dn_at(int64_t p) const { return load(dn, p); }
+    __device__ __forceinline__ Bits<W> upb_at(int64_t t) const { return load(up_b, t); }
     __device__ __forceinline__ int find(int g, uint64_t beta) const { return DetTable{ht, ht_bits}.find(g, beta); }
 };
 
@@ -498,10 +493,13 @@ __global__ void __launch_bounds__(256) k_build_rows(SetView<W> v, Ints I, double
             const int ps = v.pa_start[g], pe = v.pa_start[g + 1];
             // this row's occupied / virtual beta orbitals, k-th of each in lane k % 32, word k / 32
             int occ0 = 64, occ1 = 64, vir0 = 64, vir1 = 64, n_occ = 0, n_vir = 0;
-            if constexpr (W == 1) {
+            uint64_t beta_p = 0;
+            if constexpr (W == 0) beta_p = b.v;
+            if constexpr (W == 1) beta_p = b.w[0];
+            if constexpr (W <= 1) {
                 if (v.ht) {
                     const uint64_t all = v.norb >= 64 ? ~0ull : ((1ull << v.norb) - 1ull);
-                    const uint64_t bo = b.w[0], bv = ~b.w[0] & all;
+                    const uint64_t bo = beta_p, bv = ~beta_p & all;
                     n_occ = __popcll(bo);
                     n_vir = __popcll(bv);
                     occ0 = nth_set_bit(bo, lane);
@@ -519,13 +517,13 @@ __global__ void __launch_bounds__(256) k_build_rows(SetView<W> v, Ints I, double
                     gs = v.ga_start[g2];
                     // groups are ordered by index: a lower group holds only q < p
                     gl = (upper && g2 < g) ? 0 : v.ga_start[g2 + 1] - gs;
-                    if (W == 1 && v.ht && gl > LOOKUP_MIN_GROUP) {
+                    if (W <= 1 && v.ht && gl > LOOKUP_MIN_GROUP) {
                         probe = true;
                         gl = 0;
                     }
                 }
                 // large groups: probe the table with the single excitations of beta_p
-                if constexpr (W == 1) {
+                if constexpr (W <= 1) {
                     unsigned big = __ballot_sync(FULL, probe);
                     while (big) {
                         const int src = __ffs(big) - 1;
@@ -542,7 +540,7 @@ __global__ void __launch_bounds__(256) k_build_rows(SetView<W> v, Ints I, double
                             const int v0 = __shfl_sync(FULL, vir0, iv & 31), v1 = __shfl_sync(FULL, vir1, iv & 31);
                             const int oi = io < 32 ? o0 : o1, vi = iv < 32 ? v0 : v1;
                             if (idx < total) {
-                                const uint64_t beta = b.w[0] ^ (1ull << oi) ^ (1ull << vi);
+                                const uint64_t beta = beta_p ^ (1ull << oi) ^ (1ull << vi);
                                 q = v.find(gg, beta);
                                 hit = q >= 0 && (p_new || v.orig[q] >= v.nsh);
                             }
@@ -863,6 +861,13 @@ int build_groups(risqgpu* h, const uint64_t* d_aos, const double* d_diag_in) {
     return RISQGPU_OK;
 }
 
+// Whether the search and the elements use strings in 32-bit registers: always where a
+// string fits, since the row kernels are bound by instruction issue.  131,611 determinants
+// of 12 orbitals, FP64 rows: search 1.67 -> 1.17 ms, fill 5.22 -> 3.33 ms; 551,147 of 20,
+// FP32 + remainder bins: 11.7 -> 9.2 and 24.8 -> 16.7 ms (fill: 843 -> 590 instructions per 32
+// elements of the first set, 50 % of the issue slots).
+bool narrow(const risqgpu* h) { return h->norb <= 32; }
+
 template <int W>
 SetView<W> make_view(risqgpu* h, bool with_prev, const int32_t* prev_inv_caller) {
     SetView<W> v;
@@ -885,14 +890,23 @@ __global__ void k_invert(const int32_t* __restrict__ orig, int64_t n, int32_t* _
         inv[orig[p]] = (int32_t)p;
 }
 
+// As many CTAs of a row kernel as the device holds at once: its warps take rows from a
+// counter.  (The search needs half the registers of the fill and runs twice its warps.)
+template <typename K>
+int resident(risqgpu* h, K kern, int threads) {
+    int occ = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, threads, 0);
+    return num_sms(h) * std::max(occ, 1);
+}
+
 template <int W, int OUT>
 int launch_fill(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, const TileOut& T, int precision,
-                int* counter, int blocks, int threads, int32_t* cols, double* v64, float* v32, float* vlo,
+                int* counter, int threads, int32_t* cols, double* v64, float* v32, float* vlo,
                 int64_t row_lo, int64_t row_hi, int64_t base) {
 #define RQ_FILL(MODE)                                                                                            \
-    k_build_rows<W, MODE, OUT><<<blocks, threads, 0, h->stream>>>(v, I, thr, T, counter, nullptr, h->d_row_start, \
-                                                                  h->d_row_len, cols, v64, v32, vlo, row_lo,      \
-                                                                  row_hi, base, SigmaIO{})
+    k_build_rows<W, MODE, OUT><<<resident(h, k_build_rows<W, MODE, OUT>, threads), threads, 0, h->stream>>>(     \
+        v, I, thr, T, counter, nullptr, h->d_row_start, h->d_row_len, cols, v64, v32, vlo, row_lo, row_hi, base, \
+        SigmaIO{})
     if constexpr (OUT != OUT_BINS)
         if (precision == RISQGPU_FP64) RQ_FILL(1);
     if constexpr (OUT != OUT_UPPER) {
@@ -976,7 +990,7 @@ __global__ void k_panel_starts(const int64_t* __restrict__ row_start, int64_t n,
 // FP64 upper triangle: rows filled chunk by chunk of whole panels into a CSR buffer that
 // holds one chunk, each chunk regrouped into tiles before the next is filled.
 template <int W>
-int fill_upper64(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int* counter, int blocks, int threads,
+int fill_upper64(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int* counter, int threads,
                  int64_t cap, int64_t& nnz) {
     const int64_t n = (int64_t)h->N;
     if (tile_shape64(n, cap, h->tile_rb, h->tile_cb) != RISQGPU_OK) {
@@ -1028,7 +1042,7 @@ int fill_upper64(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int
     for (size_t c = 0; c + 1 < cuts.size(); c++) {
         const int64_t p_lo = cuts[c], p_hi = cuts[c + 1];
         RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
-        RQ_TRY((launch_fill<W, OUT_UPPER>(h, v, I, thr, TileOut{}, RISQGPU_FP64, counter, blocks, threads, ccols, c64,
+        RQ_TRY((launch_fill<W, OUT_UPPER>(h, v, I, thr, TileOut{}, RISQGPU_FP64, counter, threads, ccols, c64,
                                           nullptr, nullptr, p_lo << rb, std::min(n, p_hi << rb), ps[p_lo])));
         RQ_TRY(tb.chunk(p_lo, p_hi, h->d_row_start, ps[p_lo], h->d_row_len, ccols, c64, code, t64, max_chunk));
     }
@@ -1061,8 +1075,8 @@ __global__ void k_bin_off(int64_t n_blocks, int64_t n_windows, int cb, int kb, i
 // tiles before the next is filled, so that the device holds the tiled arrays plus one
 // chunk rather than two copies of the matrix.
 template <int W>
-int build_tiled(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int precision, int* counter, int blocks,
-                int threads, cudaEvent_t* ev, std::chrono::steady_clock::time_point& t1, int64_t& cap, int64_t& nnz) {
+int build_tiled(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int precision, int* counter, int threads,
+                cudaEvent_t* ev, std::chrono::steady_clock::time_point& t1, int64_t& cap, int64_t& nnz) {
     const int64_t n = (int64_t)h->N;
     int rb = 0, cb = 0, kb = 0;
     if (tile_shape(n, rb, cb, kb) != RISQGPU_OK) {
@@ -1094,8 +1108,8 @@ int build_tiled(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int 
     T.hist = hist;
     RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
     RQ_CUDA(h, cudaEventRecord(ev[0], h->stream));
-    k_build_rows<W, 0, OUT_BINS><<<blocks, threads, 0, h->stream>>>(v, I, thr, T, counter, nullptr, nullptr, nullptr,
-                                                                nullptr, nullptr, nullptr, nullptr, 0, n, 0, SigmaIO{});
+    k_build_rows<W, 0, OUT_BINS><<<resident(h, k_build_rows<W, 0, OUT_BINS>, threads), threads, 0, h->stream>>>(
+        v, I, thr, T, counter, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, n, 0, SigmaIO{});
     RQ_CUDA(h, cudaEventRecord(ev[1], h->stream));
     RQ_TRY(check_launch(h, "count bins"));
     TileBuilder tb;
@@ -1141,7 +1155,7 @@ int build_tiled(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int 
         const int64_t p_lo = cuts[c], p_hi = cuts[c + 1];
         T.el0 = tb.base[(size_t)p_lo].el;
         RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
-        RQ_TRY((launch_fill<W, OUT_BINS>(h, v, I, thr, T, precision, counter, blocks, threads, nullptr, nullptr, c32, clo,
+        RQ_TRY((launch_fill<W, OUT_BINS>(h, v, I, thr, T, precision, counter, threads, nullptr, nullptr, c32, clo,
                                          p_lo << rb, std::min(n, p_hi << rb), 0)));
         RQ_TRY(tb.chunk(p_lo, p_hi, T.el0, cur, code, c32, clo));
     }
@@ -1206,12 +1220,6 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
     Ints I{h->d_h1, h->d_h2, h->nuc};
     RQ_TRY(dalloc(h, counter, 1));
     const int threads = 256;
-    int occ = 0;
-    if (upper && precision != RISQGPU_FP64)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_build_rows<W, 3, OUT_BINS>, threads, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_build_rows<W, 1, OUT_ROWS>, threads, 0);
-    const int blocks = num_sms(h) * std::max(occ, 1);
-
     RQ_TRY(sync(h, "pre-count"));
     BuildEvents be;
     cudaEvent_t* ev = be.ev;
@@ -1220,7 +1228,7 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
     if (upper && precision != RISQGPU_FP64) {
         auto t1 = t0;
         int64_t cap = 0, nnz = 0;
-        RQ_TRY(build_tiled<W>(h, v, I, thr, precision, counter, blocks, threads, ev, t1, cap, nnz));
+        RQ_TRY(build_tiled<W>(h, v, I, thr, precision, counter, threads, ev, t1, cap, nnz));
         return finish_build(h, precision, upper, cap, nnz, t0, t1, t1, ev, st);
     }
     RQ_TRY(dalloc(h, cnt, n + 1));
@@ -1228,14 +1236,13 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
     RQ_TRY(dalloc(h, h->d_row_len, n));
     RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
     RQ_CUDA(h, cudaEventRecord(ev[0], h->stream));
-    if (upper)
-        k_build_rows<W, 0, OUT_UPPER><<<blocks, threads, 0, h->stream>>>(v, I, thr, TileOut{}, counter, cnt, nullptr, nullptr,
-                                                                         nullptr, nullptr, nullptr, nullptr, 0, n, 0,
-                                                                         SigmaIO{});
-    else
-        k_build_rows<W, 0, OUT_ROWS><<<blocks, threads, 0, h->stream>>>(v, I, thr, TileOut{}, counter, cnt, nullptr, nullptr,
-                                                                        nullptr, nullptr, nullptr, nullptr, 0, n, 0,
-                                                                        SigmaIO{});
+    auto count = [&](auto kern) {
+        kern<<<resident(h, kern, threads), threads, 0, h->stream>>>(v, I, thr, TileOut{}, counter, cnt, nullptr, nullptr,
+                                                                    nullptr, nullptr, nullptr, nullptr, 0, n, 0,
+                                                                    SigmaIO{});
+    };
+    if (upper) count(k_build_rows<W, 0, OUT_UPPER>);
+    else count(k_build_rows<W, 0, OUT_ROWS>);
     RQ_CUDA(h, cudaEventRecord(ev[1], h->stream));
     RQ_TRY(check_launch(h, "count rows"));
     {
@@ -1255,7 +1262,7 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
     if (upper) {
         int64_t nnz = 0;
         RQ_CUDA(h, cudaEventRecord(ev[2], h->stream));
-        RQ_TRY(fill_upper64<W>(h, v, I, thr, counter, blocks, threads, cap, nnz));
+        RQ_TRY(fill_upper64<W>(h, v, I, thr, counter, threads, cap, nnz));
         RQ_CUDA(h, cudaEventRecord(ev[3], h->stream));
         return finish_build(h, precision, upper, cap, nnz, t0, t1, t1, ev, st);
     }
@@ -1279,7 +1286,7 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
     auto t2 = clk::now();
     RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
     RQ_CUDA(h, cudaEventRecord(ev[2], h->stream));
-    RQ_TRY((launch_fill<W, OUT_ROWS>(h, v, I, thr, TileOut{}, precision, counter, blocks, threads, h->d_cols, h->d_val64,
+    RQ_TRY((launch_fill<W, OUT_ROWS>(h, v, I, thr, TileOut{}, precision, counter, threads, h->d_cols, h->d_val64,
                                      h->d_val32, h->d_val_lo, 0, n, 0)));
     RQ_CUDA(h, cudaEventRecord(ev[3], h->stream));
     int64_t nnz = 0;
@@ -1297,15 +1304,15 @@ int sigma_mf(risqgpu* h, const double* x, double* y) {
     SetView<W> v = make_view<W>(h, false, nullptr);
     v.nsh = 0;  // every pair, old and new determinants alike
     Ints I{h->d_h1, h->d_h2, h->nuc};
-    static int cached_dev[2] = {-1, -1}, cached_blocks[2] = {0, 0};
-    if (cached_dev[W - 1] != h->device) {
+    static int cached_dev[3] = {-1, -1, -1}, cached_blocks[3] = {0, 0, 0};
+    if (cached_dev[W] != h->device) {
         int occ = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_build_rows<W, 5, OUT_ROWS>, 256, 0);
-        cached_blocks[W - 1] = num_sms(h) * std::max(occ, 1);
-        cached_dev[W - 1] = h->device;
+        cached_blocks[W] = num_sms(h) * std::max(occ, 1);
+        cached_dev[W] = h->device;
     }
     RQ_CUDA(h, cudaMemsetAsync(h->d_mf_counter, 0, sizeof(int), h->stream));
-    k_build_rows<W, 5, OUT_ROWS><<<cached_blocks[W - 1], 256, 0, h->stream>>>(
+    k_build_rows<W, 5, OUT_ROWS><<<cached_blocks[W], 256, 0, h->stream>>>(
         v, I, h->mf_thr, TileOut{}, h->d_mf_counter, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0,
         (int64_t)h->N, 0, SigmaIO{x, y, h->d_diag, h->stop_flag});
     return check_launch(h, "matrix-free sigma");
@@ -1314,6 +1321,7 @@ int sigma_mf(risqgpu* h, const double* x, double* y) {
 }  // namespace
 
 int sigma_matrix_free(risqgpu* h, const double* x, double* y) {
+    if (narrow(h)) return sigma_mf<0>(h, x, y);
     return h->W == 1 ? sigma_mf<1>(h, x, y) : sigma_mf<2>(h, x, y);
 }
 
@@ -1475,7 +1483,9 @@ int build_h_impl(risqgpu* h, int precision, int builder, risqgpu_hstats* st) {
     int vprec = precision == RISQGPU_FP64_UPPER ? RISQGPU_FP64
               : precision == RISQGPU_FP32_UPPER ? RISQGPU_FP32
               : precision == RISQGPU_MIXED_UPPER ? RISQGPU_MIXED : precision;
-    int rc = h->W == 1 ? build_rows<1>(h, vprec, upper, thr, st) : build_rows<2>(h, vprec, upper, thr, st);
+    int rc = narrow(h)   ? build_rows<0>(h, vprec, upper, thr, st)
+             : h->W == 1 ? build_rows<1>(h, vprec, upper, thr, st)
+                         : build_rows<2>(h, vprec, upper, thr, st);
     if (rc) return rc;
     h->built = true;
     if (h->nsh > 0) free_prev(h);

@@ -9,6 +9,7 @@ import pytest
 
 from oracle import oracle as O
 from risq_b200 import GpuHam, _capi
+from risq_b200.fcidump import synthetic_integrals
 from tests import helpers as H
 
 pytestmark = pytest.mark.gpu
@@ -58,3 +59,39 @@ def test_tiled_sigma_matches_oracle(norb, nel, n):
                 g.set_reproducible(False)
         orp, ocols, ovals, _ = g.export_upper()
         assert np.array_equal(orp, rp) and np.array_equal(ocols, cols)
+
+
+@pytest.mark.parametrize("n_alpha,run", [(3001, 3), (4099, 3), (2200, 4)])
+def test_wide_fp64_windows_of_sparse_sets(n_alpha, run):
+    """Runs of `run` determinants of one alpha string, each connected to the others and hardly
+    any to the rest: less than one pair per row and window, hence 4096-column windows."""
+    norb, nel = 24, 8
+    ints = synthetic_integrals(norb, 3)
+    rng = np.random.default_rng(n_alpha)
+    rows, seen = [], set()
+    while len(seen) < n_alpha:
+        up = sum(1 << int(o) for o in rng.choice(norb, nel, replace=False))
+        if up in seen:
+            continue
+        seen.add(up)
+        occ = rng.choice(norb, nel + run - 1, replace=False)
+        base = sum(1 << int(o) for o in occ[:nel - 1])
+        rows += [(up, 0, base | 1 << int(o), 0) for o in occ[nel - 1:]]
+    dets = np.array(rows, dtype=np.uint64)[rng.permutation(len(rows))]
+    x = rng.standard_normal(len(dets))
+    with GpuHam(ints) as g:
+        g.set_dets(dets)
+        st = g.build(_capi.FP64_UPPER)
+        assert st["n_tiles"] > 0 and st["nnz_dense"] > st["nnz_upper"] // 2
+        assert st["nnz_upper"] < len(dets) * (((len(dets) + 2047) >> 11) // 2)
+        rp, cols, vals, diag = g.export_upper()
+        y = g.matrix_vector_prod(x)
+        g.build(_capi.FP64_UPPER)
+        np.testing.assert_array_equal(g.matrix_vector_prod(x), y)
+    sp = O.Sparse().build(H.oracle_ham(ints), dets, diag, 0, builder=_capi.BUILDER_FAST)
+    orp, ocols, ovals, _ = sp.export()
+    np.testing.assert_array_equal(rp, orp)
+    np.testing.assert_array_equal(cols, ocols)
+    np.testing.assert_array_equal(vals, ovals)
+    ref = sp.mv(x)
+    assert np.max(np.abs(y - ref)) <= 1e-11 * np.max(np.abs(ref))
