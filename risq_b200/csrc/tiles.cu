@@ -484,7 +484,7 @@ __global__ void k_left_len(int64_t p_lo, int64_t p_hi, const unsigned long long*
 
 // ---------------------------------------------------------------- conversion, FP64 values
 //
-// The FP64 upper triangle is regrouped from CSR rows: its tiles (1024 x 2048), its split
+// The FP64 upper triangle is regrouped from CSR rows: its tiles (tile_shape64), its split
 // into dense tiles and leftovers and the order of a row's leftovers decide how its sigma
 // rounds, and solves with a thick restart turn a difference of 1e-13 into another course of
 // iterations, so these stay what they were.
