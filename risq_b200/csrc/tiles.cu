@@ -936,6 +936,8 @@ __global__ void __launch_bounds__(ST, sizeof(X) == 4 ? 6 : 3)
         if (gather)
             for (int i = threadIdx.x; i < (1 << T.rb); i += ST) yR[i] = 0ull;
         stage_window<X>(xJ, x + c0, w);
+        // padding has columns 0..31: in a narrower window they have to hold a finite x too
+        for (int i = w + threadIdx.x; i < 32; i += ST) xJ[i] = 0;
         for (int i = threadIdx.x; i < w; i += ST) {
             yJa[i] = 0;
             if constexpr (DBL) yJb[i] = 0u;
