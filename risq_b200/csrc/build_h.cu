@@ -1370,6 +1370,7 @@ void free_dets(risqgpu* h) {
     dfree(h->d_ga); dfree(h->d_ga_start); dfree(h->d_gb); dfree(h->d_gb_start); dfree(h->d_order_b);
     dfree(h->d_pos_b); dfree(h->d_pa_start); dfree(h->d_pa_list); dfree(h->d_ht);
     h->ht_bits = 0;
+    h->grouped = false;
     free_csr(h);
     free_prev(h);
     h->N = 0;
@@ -1430,6 +1431,7 @@ int set_dets_impl(risqgpu* h, const uint64_t* dets, size_t n, size_t nsh, const 
         dfree(h->d_ga); dfree(h->d_ga_start); dfree(h->d_gb); dfree(h->d_gb_start); dfree(h->d_order_b);
         dfree(h->d_pos_b); dfree(h->d_pa_start); dfree(h->d_pa_list); dfree(h->d_ht);
         h->ht_bits = 0;
+        h->grouped = false;
         h->N = 0;
     } else {
         free_dets(h);
@@ -1467,6 +1469,7 @@ int set_dets_impl(risqgpu* h, const uint64_t* dets, size_t n, size_t nsh, const 
     RQ_TRY(sync(h, "set_dets"));
     dfree(d_aos);
     dfree(d_dg);
+    h->grouped = rc == RISQGPU_OK;
     return rc;
 }
 
@@ -1474,6 +1477,7 @@ int build_h_impl(risqgpu* h, int precision, int builder, risqgpu_hstats* st) {
     if (precision < 0 || precision > RISQGPU_MATRIX_FREE) { h->err = "bad precision"; return RISQGPU_ERR_INVALID; }
     if (builder < 0 || builder > 2) { h->err = "bad builder"; return RISQGPU_ERR_INVALID; }
     if (h->N == 0) { h->err = "no determinants set"; return RISQGPU_ERR_INVALID; }
+    if (!h->d_pa_start) { h->err = "the last determinant set was refused"; return RISQGPU_ERR_INVALID; }
     if (h->nsh > 0 && (h->prev_precision != precision || precision >= RISQGPU_FP64_UPPER)) {
         h->err = "an incremental build must keep the previous build's full-row precision";
         return RISQGPU_ERR_INVALID;

@@ -92,6 +92,7 @@ struct risqgpu {
     // index -1 = empty
     int4* d_ht = nullptr;
     int ht_bits = 0;
+    bool grouped = false;  // the groups and the table above are complete (the set was accepted)
 
     // sparse H: both triangles, rows in internal order, diagonal separate
     int precision = -1;   // value storage: FP64, FP32, MIXED, COLS or MATRIX_FREE

@@ -39,7 +39,8 @@ inline int grid_of(risqgpu* h, int64_t n, int block = 256) {
 // Membership in the handle's determinant set, which is sorted by (up, dn).  One-word
 // strings: the alpha string's group by binary search over the unique alpha strings, then
 // one probe of the determinant table (most excited strings are in no group, which ends the
-// test there); two-word strings: binary search over the determinants.
+// test there); two-word strings, and sets without groups (`alpha` null: the set was refused
+// after it was sorted): binary search over the determinants.
 template <int W>
 struct SortedSet {
     const uint64_t* __restrict__ up;
@@ -75,20 +76,19 @@ struct SortedSet {
         return -1;
     }
     __device__ __forceinline__ bool contains(const Bits<W>& a, const Bits<W>& b) const {
-        if constexpr (W == 1) {
+        if (W == 1 && alpha) {
             const int g = group(a.w[0]);
             return g >= 0 && table.find(g, b.w[0]) >= 0;
-        } else {
-            int64_t lo = 0, hi = N;
-            while (lo < hi) {
-                int64_t mid = (lo + hi) >> 1;
-                int c = cmp(mid, a, b);
-                if (c == 0) return true;
-                if (c < 0) lo = mid + 1;
-                else hi = mid;
-            }
-            return false;
         }
+        int64_t lo = 0, hi = N;
+        while (lo < hi) {
+            int64_t mid = (lo + hi) >> 1;
+            int c = cmp(mid, a, b);
+            if (c == 0) return true;
+            if (c < 0) lo = mid + 1;
+            else hi = mid;
+        }
+        return false;
     }
 };
 
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(256) k_expand(const uint64_t* __restrict__ aos
         const int64_t base = FILL ? off[d] : 0;
         int64_t count = 0;
         int own_group = -1;  // this determinant's alpha group
-        if constexpr (W == 1) own_group = set.group(up.w[0]);
+        if (W == 1 && set.alpha) own_group = set.group(up.w[0]);
 
         // One list [lo, hi): test(r, s, a2, b2) says whether the entry is a candidate and
         // fills in its strings.
@@ -214,14 +214,12 @@ __global__ void __launch_bounds__(256) k_expand(const uint64_t* __restrict__ aos
                              b2 = dn;
                              a2.clear(wi); a2.set(r);
                              b2.clear(wj); b2.set(s);
-                             if constexpr (W == 1) {
-                                 int g;
-                                 if (cache) {
-                                     g = my_group[wii * n + r];
-                                     if (g == -2) my_group[wii * n + r] = g = set.group(a2.w[0]);
-                                 } else g = set.group(a2.w[0]);
+                             if (W == 1 && cache) {
+                                 int g = my_group[wii * n + r];
+                                 if (g == -2) my_group[wii * n + r] = g = set.group(a2.w[0]);
                                  return g < 0 || set.table.find(g, b2.w[0]) < 0;
-                             } else return !set.contains(a2, b2);
+                             }
+                             return !set.contains(a2, b2);
                          });
                 }
             }
@@ -261,8 +259,8 @@ __global__ void __launch_bounds__(256) k_expand(const uint64_t* __restrict__ aos
                                  nx.clear(wi); nx.clear(wj); nx.set(r); nx.set(s);
                                  a2 = sp == 0 ? nx : up;
                                  b2 = sp == 0 ? dn : nx;
-                                 if constexpr (W == 1)
-                                     if (sp == 1) return set.table.find(own_group, nx.w[0]) < 0;
+                                 if (W == 1 && set.alpha && sp == 1)
+                                     return set.table.find(own_group, nx.w[0]) < 0;
                                  return !set.contains(a2, b2);
                              });
                     }
@@ -572,14 +570,16 @@ int find_new_impl(risqgpu* h, const double* coeffs, double eps, bool singles, co
     Bits<W> val;
     for (int q = 0; q < W; q++) val.w[q] = tab.valence[q];
     Ints I{h->d_h1, h->d_h2, h->nuc};
-    if (W == 1) {
+    // a refused set has no groups, and its determinants may hold more electrons than n_up
+    const bool groups = W == 1 && h->grouped;
+    if (groups) {
         RQ_TRY(dalloc(h, alpha, (size_t)h->G_a));
         k_unique_alpha<<<grid_of(h, h->G_a), 256, 0, h->stream>>>(h->d_up, h->d_ga_start, h->G_a, alpha);
         RQ_TRY(check_launch(h, "unique alpha strings"));
     }
     SortedSet<W> set{h->d_up, h->d_dn, N, alpha, h->G_a, DetTable{h->d_ht, h->ht_bits}};
     // alpha groups of single excitations, per warp, when eight warps' fit 64 KiB
-    int cache = W == 1 ? h->n_up * h->norb : 0;
+    int cache = groups ? h->n_up * h->norb : 0;
     if ((size_t)cache * 8 * sizeof(int32_t) > ((size_t)64 << 10)) cache = 0;
     const size_t smem = (size_t)cache * 8 * sizeof(int32_t);
     RQ_CUDA(h, cudaFuncSetAttribute(k_expand<W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -792,7 +792,7 @@ int sort_double_lists(risqgpu* h, SelectTables& t) {
 
 int find_new_dets_impl(risqgpu* h, const double* coeffs, double eps, bool singles, const SelectTables& tab,
                        std::vector<uint64_t>& new_dets, std::vector<double>& new_diag, SelectStats* st) {
-    if (h->N == 0) { h->err = "no determinants set"; return RISQGPU_ERR_INVALID; }
+    if (h->N == 0 || !h->d_diag) { h->err = "no determinants set"; return RISQGPU_ERR_INVALID; }
     return h->W == 1 ? find_new_impl<1>(h, coeffs, eps, singles, tab, new_dets, new_diag, st)
                      : find_new_impl<2>(h, coeffs, eps, singles, tab, new_dets, new_diag, st);
 }
