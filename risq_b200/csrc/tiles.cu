@@ -22,7 +22,8 @@
 // turns every bin into groups of rows.
 //
 // Column windows sum in 32-bit fixed point (k_sigma_fx): each product is rounded, by a
-// fixed rule, at a scale chosen per tile from the tile's largest column sum of |H| and the
+// fixed rule, at a scale chosen per tile from the tile's largest column sum of |H| (the exact
+// largest one, rounded up) and the
 // largest |x| of the panel, and integer atomics are associative, so a window's sum does
 // not depend on the order in which the pairs land.  The FP64 sigma (and the FP32 sigma
 // when reproducible sums are asked for) sums the rows in integers too and adds all window
@@ -290,10 +291,11 @@ __global__ void __launch_bounds__(AT) k_tile_size(int64_t k_lo, int64_t k_hi, in
 // reached it.  A group holds, step by step, two elements of each of its 32 slots; what a
 // slot lacks to its group's length is padded with zeros (columns spread over the banks).
 // Bins that fit are put together in shared memory and written out coalesced; larger ones
-// are scattered.  Also the bin's largest row and column sum of |H|: FP32 values in
-// integers, every element rounded up, so they bound the exact sums and do not depend on
-// the order; FP64 values (whose bins are whole tiles) in FP32 with a margin, and the larger
-// of the two for both.
+// are scattered.  Also the bin's largest row sum of |H|: FP32 values in integers, every
+// element rounded up, so it bounds the exact sum and does not depend on the order (the
+// column sums of a tile run over its bins: k_tile_finish, which takes the bin's largest |H|
+// from col_bound); FP64 values (whose bins are whole tiles) in FP32 with a margin, and the
+// larger of the row and column sums for both.
 template <typename V, bool VLO>
 __global__ void __launch_bounds__(AT) k_tile_arrange(int64_t k_lo, int64_t k_hi, int rb, int cb, int kb, int64_t chunk_el0,
                                                      TileBlock* __restrict__ blocks, const uint32_t* __restrict__ code,
@@ -306,8 +308,8 @@ __global__ void __launch_bounds__(AT) k_tile_arrange(int64_t k_lo, int64_t k_hi,
     constexpr bool DBL = std::is_same<V, double>::value;
     extern __shared__ __align__(16) unsigned char sm[];
     const int B = 1 << kb, C = 1 << cb;
-    uint32_t* cabs = reinterpret_cast<uint32_t*>(sm);       // C: column sums
-    uint32_t* rabs = cabs + C;                              // B: row sums
+    uint32_t* cabs = reinterpret_cast<uint32_t*>(sm);       // FP64 values, C: column sums
+    uint32_t* rabs = cabs + (DBL ? C : 0);                  // B: row sums
     int* cnt = reinterpret_cast<int*>(rabs + B);            // B: row lengths
     int* next = cnt + B;                                    // B: next element of each row
     int* fpre = next + B;                                   // B
@@ -332,7 +334,8 @@ __global__ void __launch_bounds__(AT) k_tile_arrange(int64_t k_lo, int64_t k_hi,
         const TileBlock b = blocks[kk];
         const int64_t e0 = b.el - chunk_el0;
         const int E = b.len, row0 = b.row & ((1 << rb) - 1);
-        for (int i = tid; i < C; i += AT) cabs[i] = 0;
+        if constexpr (DBL)
+            for (int i = tid; i < C; i += AT) cabs[i] = 0;
         for (int i = tid; i < B; i += AT) {
             rabs[i] = 0;
             next[i] = 0;
@@ -368,10 +371,10 @@ __global__ void __launch_bounds__(AT) k_tile_arrange(int64_t k_lo, int64_t k_hi,
             if (c % SEG) slots[32 * b.group + rank[r]] = (uint32_t)(row0 + r) | ((uint32_t)(c % SEG) << 16);
         }
         __syncthreads();
-        // |H| in units of 2^-u, rounded up: at most max(B, C) elements of at most vmax + 2 units
+        // |H| in units of 2^-u, rounded up: at most C elements of at most vmax + 2 units
         int ex = 0;
         if (vmax > 0.f) frexpf(vmax, &ex);
-        const int u = 31 - max(kb, cb) - 1 - ex;
+        const int u = 31 - cb - 1 - ex;
         const double unit = ldexp(1.0, u);
         for (int i = tid; i < E; i += AT) {
             const uint32_t cd = code[e0 + i];
@@ -382,9 +385,7 @@ __global__ void __launch_bounds__(AT) k_tile_arrange(int64_t k_lo, int64_t k_hi,
                 atomicAdd(reinterpret_cast<float*>(rabs) + r, a);
                 atomicAdd(reinterpret_cast<float*>(cabs) + c, a);
             } else {
-                const uint32_t a = (uint32_t)__double2ll_ru(fabs((double)v) * unit) + (VLO ? 1u : 0u);
-                atomicAdd(rabs + r, a);
-                atomicAdd(cabs + c, a);
+                atomicAdd(rabs + r, (uint32_t)__double2ll_ru(fabs((double)v) * unit) + (VLO ? 1u : 0u));
             }
             const int k = atomicAdd(next + r, 1), seg = k / SEG, kk2 = k % SEG;
             const int s = seg < cnt[r] / SEG ? fpre[r] + seg : rank[r];
@@ -403,7 +404,8 @@ __global__ void __launch_bounds__(AT) k_tile_arrange(int64_t k_lo, int64_t k_hi,
         }
         uint32_t rm = 0, cm = 0;
         for (int i = tid; i < B; i += AT) rm = max(rm, rabs[i]);
-        for (int i = tid; i < C; i += AT) cm = max(cm, cabs[i]);
+        if constexpr (DBL)
+            for (int i = tid; i < C; i += AT) cm = max(cm, cabs[i]);
         rm = __reduce_max_sync(FULL, rm);
         cm = __reduce_max_sync(FULL, cm);
         if (lane == 0) {
@@ -417,35 +419,72 @@ __global__ void __launch_bounds__(AT) k_tile_arrange(int64_t k_lo, int64_t k_hi,
                 blocks[kk].row_bound = blocks[kk].col_bound = m;
             } else {
                 blocks[kk].row_bound = __double2float_ru(ldexp((double)s_rm, -u));
-                blocks[kk].col_bound = __double2float_ru(ldexp((double)s_cm, -u));
+                blocks[kk].col_bound = vmax;
             }
         }
         __syncthreads();
     }
 }
 
-// Per tile, from its row blocks: pairs, the largest row sum of |H|, and a bound on its
-// column sums (the blocks' largest ones added); and into sums (units of 2^-20, rounded
-// up) the row bounds per panel and the column bounds per window.
-__global__ void k_tile_finish(int64_t t_lo, int64_t t_hi, int64_t b_hi, int rb, int64_t n_panels, int32_t chunk,
-                              TileBlock* __restrict__ blocks, const int32_t* __restrict__ tile_blk,
-                              const int32_t* __restrict__ tile_win, float2* __restrict__ tile_bound, unsigned long long* __restrict__ sums,
-                              unsigned long long* __restrict__ n_dense) {
-    for (int64_t t = t_lo + blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < t_hi; t += (int64_t)gridDim.x * blockDim.x) {
+// Per tile of a chunk (its first bin element: el0), one CTA each: pairs, the largest row sum
+// of |H| of its row blocks, and its largest column sum, over all of them (integers as in
+// k_tile_arrange: the largest of the blocks' own column sums, added, belongs to different
+// columns and was 2.7 to 8 times the tile's, two to three bits of every product).  And into
+// sums (units of 2^-20, rounded up) the row bounds per panel and the column bounds per
+// window.  Bound by the read of code and value, 8 bytes a pair.
+template <bool VLO>
+__global__ void __launch_bounds__(TT) k_tile_finish(int64_t t_lo, int64_t t_hi, int64_t b_hi, int rb, int cb,
+                                                    int64_t n_panels, int32_t chunk, int64_t el0,
+                                                    TileBlock* __restrict__ blocks, const int32_t* __restrict__ tile_blk,
+                                                    const int32_t* __restrict__ tile_win, const uint32_t* __restrict__ code,
+                                                    const float* __restrict__ val, float2* __restrict__ tile_bound,
+                                                    unsigned long long* __restrict__ sums,
+                                                    unsigned long long* __restrict__ n_dense) {
+    extern __shared__ __align__(16) unsigned char sm[];
+    uint32_t* cabs = reinterpret_cast<uint32_t*>(sm);  // C column sums
+    __shared__ uint32_t s_cm;
+    const int C = 1 << cb;
+    const uint32_t cmask = (uint32_t)C - 1u;
+    for (int64_t t = t_lo + blockIdx.x; t < t_hi; t += gridDim.x) {
         const int64_t ka = tile_blk[t], kz = t + 1 < t_hi ? tile_blk[t + 1] : b_hi;
+        for (int i = threadIdx.x; i < C; i += TT) cabs[i] = 0;
+        if (threadIdx.x == 0) s_cm = 0;
         int len = 0;
-        float rbnd = 0.f, cbnd = 0.f;
+        float rbnd = 0.f, vmax = 0.f;
         for (int64_t k = ka; k < kz; k++) {
-            blocks[k].chunk = chunk;
             len += blocks[k].len;
             rbnd = fmaxf(rbnd, blocks[k].row_bound);
-            cbnd = __fadd_ru(cbnd, blocks[k].col_bound);
+            vmax = fmaxf(vmax, blocks[k].col_bound);
         }
-        tile_bound[t] = make_float2(rbnd, cbnd);
-        atomicAdd(n_dense, (unsigned long long)len);
-        const int64_t P = blocks[ka].row >> rb;
-        atomicAdd(sums + P, (unsigned long long)__double2ll_ru((double)rbnd * 1048576.0));
-        atomicAdd(sums + n_panels + tile_win[t], (unsigned long long)__double2ll_ru((double)cbnd * 1048576.0));
+        __syncthreads();
+        // units of 2^-u: at most 2^rb elements of at most vmax + 2 units in a column
+        int ex = 0;
+        if (vmax > 0.f) frexpf(vmax, &ex);
+        const int u = 31 - rb - 1 - ex;
+        const double unit = ldexp(1.0, u);
+        for (int64_t k = ka; k < kz; k++) {
+            const int64_t e0 = blocks[k].el - el0;
+            const int E = blocks[k].len;
+            for (int i = threadIdx.x; i < E; i += TT)
+                atomicAdd(cabs + (code[e0 + i] & cmask),
+                          (uint32_t)__double2ll_ru(fabs((double)val[e0 + i]) * unit) + (VLO ? 1u : 0u));
+        }
+        __syncthreads();
+        uint32_t cm = 0;
+        for (int i = threadIdx.x; i < C; i += TT) cm = max(cm, cabs[i]);
+        cm = __reduce_max_sync(FULL, cm);
+        if ((threadIdx.x & 31) == 0) atomicMax(&s_cm, cm);
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            const float cbnd = __double2float_ru(ldexp((double)s_cm, -u));
+            tile_bound[t] = make_float2(rbnd, cbnd);
+            atomicAdd(n_dense, (unsigned long long)len);
+            const int64_t P = blocks[ka].row >> rb;
+            atomicAdd(sums + P, (unsigned long long)__double2ll_ru((double)rbnd * 1048576.0));
+            atomicAdd(sums + n_panels + tile_win[t], (unsigned long long)__double2ll_ru((double)cbnd * 1048576.0));
+            for (int64_t k = ka; k < kz; k++) blocks[k].chunk = chunk;
+        }
+        __syncthreads();
     }
 }
 
@@ -1427,7 +1466,7 @@ int arrange_bins(risqgpu* h, TileBlock* blocks, int64_t k_lo, int64_t k_hi, int6
     ch.val = val;
     if (lin) RQ_TRY(dalloc(h, ch.lo, (size_t)c[0] * 2));
     RQ_CUDA(h, cudaMemsetAsync(counters + 2, 0, sizeof(unsigned long long), h->stream));
-    const size_t fixed = sizeof(uint32_t) * (size_t)(C + 5 * B + B / 32 + 4);
+    const size_t fixed = sizeof(uint32_t) * (size_t)((sizeof(V) == 8 ? C : 0) + 5 * B + B / 32 + 4);
     const size_t per = 2 + sizeof(V) + (lin ? 4 : 0);
     // two CTAs per SM
     const int cap = (int)((((size_t)110 << 10) - std::min(fixed, (size_t)100 << 10)) / per) & ~63;
@@ -1456,10 +1495,16 @@ int TileBuilder::chunk(int64_t p_lo, int64_t p_hi, int64_t chunk_el0, const unsi
     const int32_t id = (int32_t)h->chunks.size() - 1;
     for (int64_t P = p_lo; P < p_hi; P++) panel_chunk[(size_t)P] = id;
     if (z.tile > a.tile) {
-        k_tile_finish<<<grid_n(h, z.tile - a.tile), 256, 0, h->stream>>>(
-            a.tile, z.tile, z.block, h->tile_rb, h->n_panels, id, h->d_tile_blocks, h->d_tile_blk, h->d_tile_win,
-            h->d_tile_bound, sums, counters + 3);
-        RQ_TRY(check_launch(h, "tile bounds"));
+        const int64_t nt = z.tile - a.tile;
+        const size_t smem = sizeof(uint32_t) << h->tile_cb;
+        auto go = [&](auto kern) -> int {
+            RQ_CUDA(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            kern<<<(int)std::min<int64_t>(nt, (int64_t)num_sms(h) * 64), TT, smem, h->stream>>>(
+                a.tile, z.tile, z.block, h->tile_rb, h->tile_cb, h->n_panels, id, chunk_el0, h->d_tile_blocks, h->d_tile_blk,
+                h->d_tile_win, code, vin, h->d_tile_bound, sums, counters + 3);
+            return check_launch(h, "tile bounds");
+        };
+        RQ_TRY(lin ? go(k_tile_finish<true>) : go(k_tile_finish<false>));
     }
     k_left_len<<<grid_n(h, np), 256, 0, h->stream>>>(p_lo, p_hi, left_cur, h->d_left_off, h->d_left_len);
     const int grid = (int)std::min<int64_t>(np, (int64_t)num_sms(h) * 8);
