@@ -1148,7 +1148,7 @@ int build_tiled(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int 
     const size_t vb = precision == RISQGPU_MIXED ? 8 : 4;
     // bytes of the tiled arrays (an eighth more for their padding), plus a margin that grows with the set (at most 256 MiB)
     // for what the allocator rounds up
-    size_t need = sizeof(unsigned long long) * (size_t)n_bins + (size_t)n * 8 + (size_t)np * 64;
+    size_t need = sizeof(unsigned long long) * (size_t)n_bins + (size_t)n * 12 + (size_t)np * 64;
     for (int64_t P = own_lo; P < own_hi; P++) {
         const PanelCount& c = tb.counts[(size_t)P];
         need += (size_t)c.vecs * 2 * (2 + vb) / 8 * 9 + (size_t)c.groups * 136 + (size_t)c.left * (6 + vb) +

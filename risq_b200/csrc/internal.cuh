@@ -139,7 +139,8 @@ struct risqgpu {
     int32_t* d_row_nleft = nullptr;   // d_left_col), and their number
     double* d_left64 = nullptr;
     double h_row_abs_max = 0.0;       // bound on sum_q |H_pq| (both triangles) of any row, for the fixed-point scale
-    // sigma work space, allocated with the matrix: the accumulator (N int64), max |x| per
+    // sigma work space, allocated with the matrix: the accumulator (N int64; FP32 values: N
+    // more, row sums from entry (N + 1) / 2 on, where the columns are summed in FP32), max |x| per
     // run of entries, and the scalars of k_sigma_prep
     long long* d_acc = nullptr;
     double* d_wmax = nullptr;

@@ -740,7 +740,7 @@ __global__ void k_tile_finish64(int64_t nt, int32_t chunk, TileBlock* __restrict
 // scalars[0] max |x|, [1] 2^s, [2] 2^-s, [3] the work-unit counter; [4] counts the blocks.
 template <typename X, typename Y>
 __global__ void __launch_bounds__(256) k_sigma_prep(const X* __restrict__ x, int64_t N, int wb, Y* __restrict__ acc,
-                                                    double* __restrict__ wmax, double row_abs_max, int smax, int top,
+                                                    long long* __restrict__ acc_row, double* __restrict__ wmax, double row_abs_max, int smax, int top,
                                                     double* __restrict__ scalars, const int* __restrict__ stop) {
     if (stop && *stop) return;
     __shared__ double s_m[8];
@@ -760,6 +760,7 @@ __global__ void __launch_bounds__(256) k_sigma_prep(const X* __restrict__ x, int
     for (int64_t i = i0 + threadIdx.x; i < i1; i += 256) {
         m = fmax(m, fabs((double)x[i]));
         acc[i] = 0;
+        if (acc_row) acc_row[i] = 0;
     }
     m = block_max(m);
     unsigned long long* const done = reinterpret_cast<unsigned long long*>(scalars) + 4;
@@ -847,26 +848,33 @@ struct TileView {
     const int32_t* __restrict__ row_nleft;
 };
 
-// Power of two that takes sums of at most b to at most 2^30, as an exponent.
-__device__ __forceinline__ int fixed_shift(double b, int most) {
+// Power of two, as an exponent, that takes sums of at most b below 2^(top + 1).
+__device__ __forceinline__ int fixed_shift(double b, int most, int top) {
     int sh = 0;
-    if (b > 0.0 && isfinite(b)) sh = 29 - ilogb(b);
+    if (b > 0.0 && isfinite(b)) sh = top - ilogb(b);
     return max(-most, min(most, sh));
 }
+
+// The largest such for 32-bit sums: the margin of 2^-13 (2^18 units) covers what the up to
+// 2^11 products of a sum are rounded by.
+__device__ __forceinline__ int fixed_shift32(double b, int most) { return fixed_shift(b * (1.0 + 0x1p-13), most, 30); }
 
 // Fixed-point tile sigma.  Shared-memory integer atomics are single instructions,
 // where FP32 shared atomics are compare-and-swap loops and 64-bit ones slower still
 // (measured on B200: 7.9, 2.6 and 1.5 per clock per SM), so each tile's column sums are
 // formed in 32-bit integers: every product is scaled by 2^s_t, s_t chosen from the tile's
-// bound on its column sums of |H| times the panel's max |x| so that no sum exceeds 2^30,
+// largest column sum of |H| times the panel's max |x| so that no sum reaches 2^31,
 // and rounded to an integer (FP32 vectors) or, at 2^lb times that scale, to a 64-bit
-// integer whose high part and low lb = 32 - rb bits are added apart (FP64 vectors: 49 or
-// more significant bits; the 2^rb rows of a panel cannot overflow the low parts).  Row
-// sums stay in the register of the lane that holds the row: FP32 for FP32 vectors, 64-bit
-// integers at the scale 2^S of the whole sigma for FP64 ones, 32-bit integers for EXACT
-// FP32.  EXACT: all sums are shifted to the scale 2^S and added with 64-bit global
-// atomics, so sigma is bitwise reproducible and ranks' partial sums add exactly;
-// otherwise they are added in FP32.
+// integer whose high part and low lb = 32 - rb bits are added apart (FP64 vectors: 51 or
+// more bits below the largest sum; the 2^rb rows of a panel cannot overflow the low parts).
+// Row sums stay in the register of the lane that holds the row: 32-bit integers, scaled
+// like the columns by the tile's largest row sum and the window's max |x|, for FP32
+// vectors, 64-bit integers at the scale 2^S of the whole sigma for FP64 ones.  EXACT: all
+// sums are shifted to the scale 2^S and added with 64-bit global atomics, so sigma is
+// bitwise reproducible and ranks' partial sums add exactly; otherwise (FP32 vectors) the
+// rows' are (in FP32, a row's sums from every tile of its panel were what rounded most on a
+// vector without signs: 6.6e-8 of |y|, against 4.1e-8), and a window's are added in FP32,
+// four columns at a time.
 //
 // FP64 values: rows and columns of a tile share one scale, 2^20 times finer than the one
 // that takes the tile's bound times max |x| to 2^30, and a sum that the scale 2^S cannot
@@ -878,12 +886,13 @@ __device__ __forceinline__ int fixed_shift(double b, int most) {
 template <typename X, typename V, bool VLO, bool EXACT>
 __global__ void __launch_bounds__(ST, sizeof(X) == 4 ? 6 : 3)
     k_sigma_fx(int64_t N, int64_t n_units, const SigmaUnit* __restrict__ units, TileView<V> T, const X* __restrict__ x,
-               const double* __restrict__ wmax, void* __restrict__ acc_out, double* __restrict__ scalars,
-               const int* __restrict__ stop) {
+               const double* __restrict__ wmax, void* __restrict__ acc_out, unsigned long long* __restrict__ acc_row,
+               double* __restrict__ scalars, const int* __restrict__ stop) {
     if (stop && *stop) return;
     constexpr bool DBL = std::is_same<X, double>::value;
     constexpr bool V64 = std::is_same<V, double>::value;
     using RS = typename std::conditional<DBL, long long, typename std::conditional<EXACT, int, float>::type>::type;
+    constexpr int PARTS = DBL || EXACT ? 1 : 4;  // of an FP32 row sum: a quarter of the elements each
     constexpr int U = DBL ? 2 : 4;  // steps in flight
     extern __shared__ __align__(16) unsigned char sm[];
     const int C = 1 << T.cb, lb = 32 - T.rb;
@@ -894,8 +903,8 @@ __global__ void __launch_bounds__(ST, sizeof(X) == 4 ? 6 : 3)
     __shared__ long long s_unit;
     __shared__ int s_next;
     const int lane = threadIdx.x & 31;
-    const double gscale = scalars[1];  // 2^S (EXACT)
-    const int S = EXACT ? ilogb(gscale) : 0;
+    const double gscale = scalars[1];  // 2^S
+    const int S = ilogb(gscale);
     unsigned long long* counter = reinterpret_cast<unsigned long long*>(scalars) + 3;
     unsigned long long* acc_ll = reinterpret_cast<unsigned long long*>(acc_out);
     X* acc_x = reinterpret_cast<X*>(acc_out);
@@ -948,7 +957,7 @@ __global__ void __launch_bounds__(ST, sizeof(X) == 4 ? 6 : 3)
                     atomicAdd(acc_ll + p, (unsigned long long)llrint((double)pr * gscale));
                     atomicAdd(acc_ll + q, (unsigned long long)llrint((double)pc * gscale));
                 } else {
-                    atomicAdd(acc_x + p, pr);
+                    atomicAdd(acc_row + p, (unsigned long long)llrint((double)pr * gscale));
                     atomicAdd(acc_x + q, pc);
                 }
             }
@@ -962,15 +971,15 @@ __global__ void __launch_bounds__(ST, sizeof(X) == 4 ? 6 : 3)
         // it without rounding and neither the cut into slots and units nor the order matters
         int sh, rsh = S;  // of the column sums (FP64 vectors: lb bits finer) and of the row sums
         if constexpr (V64) {
-            sh = fixed_shift((double)bound.y * scalars[0], 200) + 20 - lb;
+            sh = fixed_shift((double)bound.y * scalars[0], 200, 29) + 20 - lb;
             rsh = sh + lb;
         } else {
-            sh = fixed_shift((double)bound.y * max_of(r0, min(N, r0 + ((int64_t)1 << T.rb))), DBL ? 800 : 120);
+            sh = fixed_shift32((double)bound.y * max_of(r0, min(N, r0 + ((int64_t)1 << T.rb))), DBL ? 800 : 120);
             if constexpr (EXACT) sh = min(sh, DBL ? S - lb : S);
-            if constexpr (EXACT && !DBL) rsh = min(S, fixed_shift((double)bound.x * max_of(c0, c0 + w), 120));
+            if constexpr (EXACT && !DBL) rsh = min(S, fixed_shift32((double)bound.x * max_of(c0, c0 + w), 120));
         }
         const X csc = (X)ldexp(1.0, DBL ? sh + lb : sh);
-        const X rsc = (X)(EXACT ? ldexp(1.0, rsh) : 1.0);
+        const X rsc = (X)ldexp(1.0, rsh);
         const bool gather = V64 && rsh > S;  // row sums round to 2^S: together, once
         if (gather)
             for (int i = threadIdx.x; i < (1 << T.rb); i += ST) yR[i] = 0ull;
@@ -1016,8 +1025,8 @@ __global__ void __launch_bounds__(ST, sizeof(X) == 4 ? 6 : 3)
             const int len = (int)(hd >> 16);
             const int64_t row = r0 + (hd & 0xffffu);
             const X xr = len > 0 ? __ldg(x + row) * csc : (X)0;
-            RS rs = 0;
-            auto add = [&](int cc, X vv) {
+            RS rs[PARTS] = {};
+            auto add = [&](RS& rs, int cc, X vv) {
                 if constexpr (DBL) {
                     rs += __double2ll_rn(vv * xJ[cc] * rsc);
                     const long long q = __double2ll_rn(vv * xr);
@@ -1047,8 +1056,8 @@ __global__ void __launch_bounds__(ST, sizeof(X) == 4 ? 6 : 3)
                 if constexpr (VLO) pl += 64 * U;
 #pragma unroll
                 for (int k = 0; k < U; k++) {
-                    add(c[k].x, v[k][0]);
-                    add(c[k].y, v[k][1]);
+                    add(rs[2 * k % PARTS], c[k].x, v[k][0]);
+                    add(rs[(2 * k + 1) % PARTS], c[k].y, v[k][1]);
                 }
             }
             for (; j < steps; j++) {
@@ -1058,13 +1067,18 @@ __global__ void __launch_bounds__(ST, sizeof(X) == 4 ? 6 : 3)
                 pc += 32;
                 pv += 64;
                 if constexpr (VLO) pl += 64;
-                add(c.x, v[0]);
-                add(c.y, v[1]);
+                add(rs[0], c.x, v[0]);
+                add(rs[1 % PARTS], c.y, v[1]);
             }
             if (len > 0) {
-                if (gather) atomicAdd(yR + (row - r0), (unsigned long long)rs);
-                else if constexpr (EXACT) atomicAdd(acc_ll + row, (unsigned long long)((long long)rs << (S - rsh)));
-                else atomicAdd(acc_x + row, rs);
+                if (gather) atomicAdd(yR + (row - r0), (unsigned long long)rs[0]);
+                else if constexpr (EXACT) atomicAdd(acc_row + row, (unsigned long long)((long long)rs[0] << (S - rsh)));
+                else {
+                    double sum = 0.0;
+#pragma unroll
+                    for (int k = 0; k < PARTS; k++) sum += (double)rs[k];
+                    atomicAdd(acc_row + row, (unsigned long long)llrint(sum * gscale));
+                }
             }
             hd = hd_next;
             off = off_next;
@@ -1104,14 +1118,15 @@ __global__ void __launch_bounds__(ST, sizeof(X) == 4 ? 6 : 3)
     }
 }
 
-// y = diag x + acc (fixed point: acc 2^-s)
+// y = diag x + acc 2^-s, or with FP32 column sums diag x + acc + acc_row 2^-s
 template <typename X, typename T>
 __global__ void k_fixed_finish(int64_t N, const double* __restrict__ diag, const X* __restrict__ x,
-                               const T* __restrict__ acc, const double* __restrict__ scalars,
-                               X* __restrict__ y) {
-    const double inv = std::is_same<T, long long>::value ? scalars[2] : 1.0;
+                               const T* __restrict__ acc, const long long* __restrict__ acc_row,
+                               const double* __restrict__ scalars, X* __restrict__ y) {
+    constexpr bool FX = std::is_same<T, long long>::value;
+    const double inv = scalars[2];
     for (int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; p < N; p += (int64_t)gridDim.x * blockDim.x)
-        y[p] = (X)(diag[p] * (double)x[p] + (double)acc[p] * inv);
+        y[p] = (X)(diag[p] * (double)x[p] + (FX ? (double)acc[p] * inv : (double)acc[p] + (double)acc_row[p] * inv));
 }
 
 // Calls f(p, q, v) for every stored pair (p < q, internal indices, FP64 value): one CTA
@@ -1259,18 +1274,22 @@ int launch_fx(risqgpu* h, const X* x, X* y, const TileView<V>& T) {
     RQ_CUDA(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, ST, smem);
+    // FP32 sums: N columns, then the rows' in fixed point
+    long long* const acc_row = EXACT ? nullptr : h->d_acc + (N + 1) / 2;
     const int grid =
         (int)std::max<int64_t>(1, std::min<int64_t>(h->n_units, (int64_t)num_sms(h) * std::max(occ, 1)));
     k_sigma_prep<X, Y><<<(int)(((N - 1) >> T.wb) + 1), 256, 0, h->stream>>>(
-        x, N, T.wb, reinterpret_cast<Y*>(h->d_acc), h->d_wmax, h->h_row_abs_max,
+        x, N, T.wb, reinterpret_cast<Y*>(h->d_acc), acc_row, h->d_wmax, h->h_row_abs_max,
         std::is_same<X, float>::value ? 100 : 1000, 61, h->d_sig_scalars, h->stop_flag);
-    kern<<<grid, ST, smem, h->stream>>>(N, h->n_units, h->d_units, T, x, h->d_wmax, h->d_acc, h->d_sig_scalars, h->stop_flag);
+    kern<<<grid, ST, smem, h->stream>>>(N, h->n_units, h->d_units, T, x, h->d_wmax, h->d_acc,
+                                        reinterpret_cast<unsigned long long*>(EXACT ? h->d_acc : acc_row),
+                                        h->d_sig_scalars, h->stop_flag);
     RQ_TRY(check_launch(h, "sigma (tiles)"));
     // with a row-block partition every rank summed its own panels: the exact integer
     // sums are added across the ranks
     if (EXACT && h->part_n > 1) RQ_TRY(part_allreduce(h, h->d_acc, (size_t)N));
     k_fixed_finish<X, Y><<<grid_n(h, N), 256, 0, h->stream>>>(N, h->d_diag, x, reinterpret_cast<const Y*>(h->d_acc),
-                                                             h->d_sig_scalars, y);
+                                                             acc_row, h->d_sig_scalars, y);
     return check_launch(h, "sigma (tiles)");
 }
 
@@ -1402,7 +1421,7 @@ int TileBuilder::begin(int64_t p_lo, int64_t p_hi, int precision, const uint32_t
     RQ_TRY(dalloc(h, h->d_left_row, (size_t)left));
     RQ_TRY(dalloc(h, h->d_left32, (size_t)left));
     if (lo) RQ_TRY(dalloc(h, h->d_left_lo, (size_t)left));
-    RQ_TRY(dalloc(h, h->d_acc, (size_t)N));
+    RQ_TRY(dalloc(h, h->d_acc, (size_t)(N + (N + 1) / 2)));
     RQ_TRY(dalloc(h, h->d_sig_scalars, 5));
     RQ_TRY(dalloc(h, h->d_wmax, (size_t)((N - 1) >> std::min(h->tile_rb, h->tile_cb)) + 1));
     RQ_TRY(dalloc(h, left_cur, (size_t)np));
