@@ -113,7 +113,7 @@ typedef struct {
     double ms_count;          /* candidate count pass */
     double ms_fill;           /* Slater-Condon + CSR fill pass */
     double ms_total;
-    uint64_t bytes_csr;       /* bytes written for columns + values */
+    uint64_t bytes_csr;       /* bytes of the stored columns + values (tiles: without their padding) */
     double gpu_ms_count;      /* CUDA-event durations on the handle's stream */
     double gpu_ms_fill;       /* fill (and, for upper-triangle storage, the regrouping into tiles) */
     uint64_t n_tiles;         /* upper-triangle storage: dense (row panel, column window) tiles */
@@ -259,8 +259,18 @@ RISQGPU_API int risqgpu_set_partition(risqgpu_t* h, int rank, int nranks, risqgp
  * it lets a caller share one GPU between the library and its own work, and lets
  * tests drive the out-of-memory paths without exhausting a shared device. */
 RISQGPU_API int risqgpu_set_memory_limit(risqgpu_t* h, size_t bytes);
-/* Device memory the handle holds now (used) and its bound (limit, 0 = none). */
+/* Device memory the handle's buffers hold now (used) and its bound (limit, 0 = none).
+ * Beyond that, while handles without a bound live, the process keeps up to 6 GiB of freed
+ * large blocks and 2 GiB of small ones per device (a sixteenth and a thirty-second of the
+ * device, if less) for the next buffers, and between risqgpu_set_dets and the end of the next
+ * build a handle keeps the large blocks of the matrix it dropped.  All of it is given back
+ * when an allocation of the library would fail otherwise, when the last handle on the
+ * device is destroyed, when a handle gets a bound, and by risqgpu_release_memory. */
 RISQGPU_API int risqgpu_memory_used(const risqgpu_t* h, size_t* used, size_t* limit);
+/* Give the idle device memory described above back to the device (every idle block on this
+ * handle's device, whichever handle used it), for a caller that is about to allocate its
+ * own.  Waits for the handle's stream. */
+RISQGPU_API int risqgpu_release_memory(risqgpu_t* h);
 
 /* Run the handle's work on `stream` (a cudaStream_t on the handle's device; NULL
  * restores the handle's own stream), so that a caller can order and time it with

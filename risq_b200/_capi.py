@@ -97,6 +97,7 @@ SIGNATURES = [
     ("risqgpu_set_partition", C.c_int, [_handle, C.c_int, C.c_int, ALLREDUCE_FN, C.c_void_p]),
     ("risqgpu_set_memory_limit", C.c_int, [_handle, C.c_size_t]),
     ("risqgpu_memory_used", C.c_int, [_handle, C.POINTER(C.c_size_t), C.POINTER(C.c_size_t)]),
+    ("risqgpu_release_memory", C.c_int, [_handle]),
     ("risqgpu_set_stream", C.c_int, [_handle, C.c_void_p]),
     ("risqgpu_sigma_noalloc", C.c_int, [_handle, C.c_void_p, C.c_void_p]),
     ("risqgpu_ham_diag", C.c_int, [_handle, _u64p, C.c_size_t, _dp]),

@@ -973,14 +973,21 @@ void own_panels(const risqgpu* h, const std::vector<int64_t>& ps, int64_t& lo, i
     hi = std::max(hi, lo);
 }
 
-// Chunks of the panels [own_lo, own_hi): the fewest whose largest one, at per_el bytes an
-// element, fits beside `fixed` bytes; chunk k ends at the panel boundary nearest to k/K of
-// the pairs, so the chunks hold about equal shares.
+// Chunks of the panels [own_lo, own_hi): of about CHUNK_BYTES at per_el bytes an element, or
+// at most 16, or the fewest more whose largest one fits beside `fixed` bytes; chunk k ends at
+// the panel boundary nearest to k/K of the pairs, so the chunks hold about equal shares.
+// CHUNK_BYTES keeps what a chunk needs within the idle memory kept between builds; not more
+// than 16 of them for that, since the FP64 conversion has one CTA per panel and two per SM
+// (8,300,003 determinants: 2.04 s of kernels in 75 chunks of 108 panels, 1.69 s in 16).
+constexpr size_t CHUNK_BYTES = (size_t)5 << 30;
+
 int chunk_cuts(risqgpu* h, const std::vector<int64_t>& ps, int64_t own_lo, int64_t own_hi, size_t fixed, size_t per_el,
                std::vector<int64_t>& cuts, int64_t& max_chunk) {
     const int64_t own_cap = ps[own_hi] - ps[own_lo], own_np = own_hi - own_lo;
     const size_t avail = mem_available(h, fixed + (size_t)own_cap * per_el);
-    for (int64_t K = 1;; K = K < 8 ? K + 1 : K * 2) {
+    const int64_t want = std::min<int64_t>(16, (int64_t)((size_t)own_cap * per_el / CHUNK_BYTES) + 1);
+    for (int64_t K = std::max<int64_t>(1, std::min(own_np, want));;
+         K = K < 8 ? K + 1 : K * 2) {
         cuts.assign(1, own_lo);
         for (int64_t k = 1; k < K; k++) {
             const int64_t goal = ps[own_lo] + (int64_t)((double)own_cap * k / K);
@@ -1049,8 +1056,12 @@ int fill_upper64(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int
     };
     std::vector<int64_t> cuts;
     int64_t max_chunk = 0;
-    if (chunk_cuts(h, ps, own_lo, own_hi, fixed_for(56), 24, cuts, max_chunk) != RISQGPU_OK)
-        RQ_TRY(chunk_cuts(h, ps, own_lo, own_hi, fixed_for(45), 24, cuts, max_chunk));
+    // (60 quarters of a byte: 14 bytes and the sixteenth by which blocks may be larger)
+    if (chunk_cuts(h, ps, own_lo, own_hi, fixed_for(60), 24, cuts, max_chunk) != RISQGPU_OK) {
+        h->exact = true;
+        if (chunk_cuts(h, ps, own_lo, own_hi, fixed_for(56), 24, cuts, max_chunk) != RISQGPU_OK)
+            RQ_TRY(chunk_cuts(h, ps, own_lo, own_hi, fixed_for(45), 24, cuts, max_chunk));
+    }
     h->err.clear();
     int32_t* ccols = nullptr;
     uint32_t* code = nullptr;
@@ -1157,7 +1168,11 @@ int build_tiled(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int 
     const size_t fixed = need + std::max((size_t)8 << 20, std::min((size_t)256 << 20, need / 32));
     std::vector<int64_t> cuts;
     int64_t max_chunk = 0;
-    RQ_TRY(chunk_cuts(h, ps, own_lo, own_hi, fixed, 4 + vb, cuts, max_chunk));
+    if (chunk_cuts(h, ps, own_lo, own_hi, fixed + fixed / 16, 4 + vb, cuts, max_chunk) != RISQGPU_OK) {
+        h->exact = true;
+        RQ_TRY(chunk_cuts(h, ps, own_lo, own_hi, fixed, 4 + vb, cuts, max_chunk));
+        h->err.clear();
+    }
     RQ_TRY(dalloc(h, cur, (size_t)n_bins));
     RQ_TRY(tb.begin(own_lo, own_hi, precision, hist, bin_off, cur));
     dfree(hist);
@@ -1295,6 +1310,7 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
         const size_t arrays = (size_t)cap * (4 + vb);
         size_t need = arrays + std::max((size_t)8 << 20, std::min((size_t)64 << 20, arrays / 16));
         const size_t fr = mem_available(h, need);
+        h->exact = need + arrays / 16 > fr;
         if (need > fr) {
             h->err = "sparse H needs " + std::to_string(need >> 20) + " MiB, " + std::to_string(fr >> 20) +
                      " MiB available";
@@ -1366,6 +1382,7 @@ static void free_prev(risqgpu* h) {
 }
 
 void free_dets(risqgpu* h) {
+    Parking park(h);
     dfree(h->d_up); dfree(h->d_dn); dfree(h->d_up_b); dfree(h->d_orig); dfree(h->d_inv); dfree(h->d_diag);
     dfree(h->d_ga); dfree(h->d_ga_start); dfree(h->d_gb); dfree(h->d_gb_start); dfree(h->d_order_b);
     dfree(h->d_pos_b); dfree(h->d_pa_start); dfree(h->d_pa_list); dfree(h->d_ht);
@@ -1473,7 +1490,7 @@ int set_dets_impl(risqgpu* h, const uint64_t* dets, size_t n, size_t nsh, const 
     return rc;
 }
 
-int build_h_impl(risqgpu* h, int precision, int builder, risqgpu_hstats* st) {
+static int build_matrix(risqgpu* h, int precision, int builder, risqgpu_hstats* st) {
     if (precision < 0 || precision > RISQGPU_MATRIX_FREE) { h->err = "bad precision"; return RISQGPU_ERR_INVALID; }
     if (builder < 0 || builder > 2) { h->err = "bad builder"; return RISQGPU_ERR_INVALID; }
     if (h->N == 0) { h->err = "no determinants set"; return RISQGPU_ERR_INVALID; }
@@ -1485,7 +1502,10 @@ int build_h_impl(risqgpu* h, int precision, int builder, risqgpu_hstats* st) {
     bool fast = builder == RISQGPU_BUILDER_FAST || (builder == RISQGPU_BUILDER_AUTO && h->N > 100);
     double thr = fast ? 1e-12 : 0.0;
     auto t0 = std::chrono::steady_clock::now();
-    free_csr(h);
+    {
+        Parking park(h);
+        free_csr(h);
+    }
     if (precision == RISQGPU_MATRIX_FREE) {
         // nothing to store: sigma finds and evaluates every row's elements itself
         if (h->part_n > 1) {
@@ -1524,6 +1544,13 @@ int build_h_impl(risqgpu* h, int precision, int builder, risqgpu_hstats* st) {
         st->ms_total = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
     }
     return RISQGPU_OK;
+}
+
+int build_h_impl(risqgpu* h, int precision, int builder, risqgpu_hstats* st) {
+    const int rc = build_matrix(h, precision, builder, st);
+    h->exact = false;
+    drop_parked(h, true);
+    return rc;
 }
 
 int export_upper_impl(risqgpu* h, int64_t* rowptr, int64_t* cols, double* vals, size_t cap, double* diag) {

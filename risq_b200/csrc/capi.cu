@@ -13,15 +13,14 @@ namespace risq {
 
 namespace {
 
-// Where a buffer came from.  Buffers below POOL_LARGE: the device's stream-ordered pool.
-// From there to POOL_HUGE: whole blocks kept for reuse, sizes rounded up to a quarter of
-// their power of two, so that one set's matrix fits the blocks another one left; a pool
-// that cuts small buffers, or the first of two large ones, from a freed matrix's hole has
-// to map new memory for the rest (131,611 determinants, three handles in turn: 13 ms a
-// build, against 8 here).  Larger ones, and those of handles with a memory bound: the
-// device.
+// Where a buffer came from.  Below POOL_LARGE: the device's stream-ordered pool.  From there
+// on: whole blocks, kept for reuse when they are freed, in sizes that differ by a sixteenth of
+// their power of two, so that one set's matrix fits the blocks another one left; a pool that
+// cuts small buffers, or the first of two large ones, from a freed matrix's hole has to map
+// new memory for the rest (131,611 determinants, three handles in turn: 13 ms a build,
+// against 8 here).  Those of handles with a memory bound: the device.
 enum Source { FROM_DEVICE, FROM_POOL, FROM_BLOCKS };
-constexpr size_t POOL_LARGE = (size_t)64 << 20, POOL_HUGE = (size_t)6 << 30;
+constexpr size_t POOL_LARGE = (size_t)64 << 20;
 
 struct Buffer {
     risqgpu* h;
@@ -35,7 +34,6 @@ std::unordered_map<void*, Buffer> g_ledger;
 struct Block {  // an idle block: free once `done` has passed on the stream it was used on
     void* p;
     size_t bytes;
-    cudaStream_t stream;
     cudaEvent_t done;
 };
 struct Pool {
@@ -43,7 +41,6 @@ struct Pool {
     std::vector<Block> blocks;  // oldest first
     size_t idle = 0;            // bytes of blocks
     size_t keep = 0;            // most of them
-    size_t freed = 0;           // bytes returned to the small pool since it was looked at
     int users = 0;
 };
 std::mutex g_pool_mu;
@@ -52,9 +49,12 @@ std::unordered_map<int, Pool> g_pools;
 size_t block_size(size_t bytes) {
     size_t unit = POOL_LARGE;
     while (unit * 2 <= bytes) unit *= 2;
-    unit /= 4;
+    unit = std::min(unit / 16, (size_t)64 << 20);
     return (bytes + unit - 1) / unit * unit;
 }
+
+// Whether a block may serve a request: at most an eighth of it unused.
+bool fits(size_t block, size_t bytes) { return block >= bytes && block - bytes <= bytes / 8; }
 
 void drop_oldest(Pool& P) {  // cudaFree waits for the work that uses the block
     const Block b = P.blocks.front();
@@ -72,6 +72,24 @@ bool pool_bytes(cudaMemPool_t pool, uint64_t& reserved, uint64_t& used) {
     return false;
 }
 
+// Hands a block that work on h's stream may still use to the device's idle ones.
+void keep_block(risqgpu* h, void* p, size_t bytes) {
+    DeviceGuard g(h->device);
+    std::lock_guard<std::mutex> lk(g_pool_mu);
+    Pool& P = g_pools[h->device];
+    Block k{p, bytes, nullptr};
+    if (bytes > P.keep || cudaEventCreateWithFlags(&k.done, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventRecord(k.done, h->stream) != cudaSuccess) {
+        cudaGetLastError();
+        if (k.done) cudaEventDestroy(k.done);
+        cudaFree(p);
+        return;
+    }
+    P.blocks.push_back(k);
+    P.idle += bytes;
+    while (P.idle > P.keep) drop_oldest(P);
+}
+
 }  // namespace
 
 int pool_acquire(int device) {
@@ -87,12 +105,12 @@ int pool_acquire(int device) {
             P.small = nullptr;
             return RISQGPU_ERR_CUDA;
         }
-        // the pool's own threshold counts the bytes in use too; mem_free bounds the idle ones
-        uint64_t all = UINT64_MAX;
-        cudaMemPoolSetAttribute(P.small, cudaMemPoolAttrReleaseThreshold, &all);
+        // above this size the pool itself returns what is idle, at each wait
         size_t fr = 0, tot = 0;
         cudaMemGetInfo(&fr, &tot);
-        P.keep = std::min(POOL_KEEP, tot / 8);
+        uint64_t small = std::min(SMALL_KEEP, tot / 32);
+        cudaMemPoolSetAttribute(P.small, cudaMemPoolAttrReleaseThreshold, &small);
+        P.keep = std::min(POOL_KEEP, tot / 16);
     }
     P.users++;
     return RISQGPU_OK;
@@ -126,6 +144,14 @@ size_t pool_idle(int device) {
     return idle;
 }
 
+void drop_parked(risqgpu* h, bool reuse) {
+    for (const auto& b : h->parked) {
+        if (reuse) keep_block(h, b.first, b.second);
+        else cudaFree(b.first);
+    }
+    h->parked.clear();
+}
+
 int mem_alloc(risqgpu* h, void** p, size_t bytes) {
     *p = nullptr;
     if (h->mem_limit && h->mem_used + bytes > h->mem_limit) {
@@ -135,26 +161,36 @@ int mem_alloc(risqgpu* h, void** p, size_t bytes) {
     }
     Buffer b{h, bytes, FROM_DEVICE, bytes};
     cudaMemPool_t small = nullptr;
-    if (!h->mem_limit && bytes < POOL_HUGE) {
+    if (!h->mem_limit) {
         b.source = bytes < POOL_LARGE ? FROM_POOL : FROM_BLOCKS;
-        std::lock_guard<std::mutex> lk(g_pool_mu);
-        Pool& P = g_pools[h->device];
-        // A handle that holds more than is ever kept idle gets the bytes it asks for: the
-        // rounding of its many large buffers would take memory that the build counts on.
         if (b.source == FROM_BLOCKS) {
-            if (h->mem_used + bytes > P.keep) b.source = FROM_DEVICE;
-            else b.held = block_size(bytes);
+            // the smallest block that fits: of the handle's previous matrix, then of the idle ones
+            b.held = h->exact ? bytes : block_size(bytes);
+            auto best = h->parked.end();
+            for (auto k = h->parked.begin(); k != h->parked.end(); ++k)
+                if (fits(k->second, bytes) && (best == h->parked.end() || k->second < best->second)) best = k;
+            if (best != h->parked.end()) {
+                *p = best->first;
+                b.held = best->second;
+                h->parked.erase(best);
+            }
         }
-        small = P.small;
-        auto best = P.blocks.end();
-        if (b.source == FROM_BLOCKS)
-            best = std::find_if(P.blocks.begin(), P.blocks.end(), [&](const Block& k) { return k.bytes == b.held; });
-        if (best != P.blocks.end()) {
-            if (best->stream != h->stream) cudaStreamWaitEvent(h->stream, best->done, 0);
-            cudaEventDestroy(best->done);
-            *p = best->p;
-            P.idle -= best->bytes;
-            P.blocks.erase(best);
+        if (!*p) {
+            std::lock_guard<std::mutex> lk(g_pool_mu);
+            Pool& P = g_pools[h->device];
+            small = P.small;
+            auto best = P.blocks.end();
+            if (b.source == FROM_BLOCKS)
+                for (auto k = P.blocks.begin(); k != P.blocks.end(); ++k)
+                    if (fits(k->bytes, bytes) && (best == P.blocks.end() || k->bytes < best->bytes)) best = k;
+            if (best != P.blocks.end()) {
+                cudaStreamWaitEvent(h->stream, best->done, 0);
+                cudaEventDestroy(best->done);
+                *p = best->p;
+                b.held = best->bytes;
+                P.idle -= best->bytes;
+                P.blocks.erase(best);
+            }
         }
     }
     if (!*p) {
@@ -166,6 +202,7 @@ int mem_alloc(risqgpu* h, void** p, size_t bytes) {
             // idle memory may be all that is missing
             cudaGetLastError();
             cudaStreamSynchronize(h->stream);
+            drop_parked(h, false);
             pool_trim(h->device);
             b.held = bytes;
             e = take();
@@ -177,9 +214,10 @@ int mem_alloc(risqgpu* h, void** p, size_t bytes) {
             return e == cudaErrorMemoryAllocation ? RISQGPU_ERR_OOM : RISQGPU_ERR_CUDA;
         }
     }
+    b.bytes = b.held;
     std::lock_guard<std::mutex> lk(g_ledger_mu);
     g_ledger[*p] = b;
-    h->mem_used += bytes;
+    h->mem_used += b.bytes;
     return RISQGPU_OK;
 }
 
@@ -193,33 +231,10 @@ void mem_free(void* p) {
         b.h->mem_used -= b.bytes;
         g_ledger.erase(it);
     }
-    if (b.source == FROM_DEVICE) {
-        cudaFree(p);
-        return;
-    }
-    if (b.source == FROM_POOL) cudaFreeAsync(p, b.h->stream);
-    std::lock_guard<std::mutex> lk(g_pool_mu);
-    Pool& P = g_pools[b.h->device];
-    if (b.source == FROM_POOL) {
-        // every eighth of the allowance: give the device what is idle beyond it
-        P.freed += b.held;
-        if (P.freed < P.keep / 8) return;
-        P.freed = 0;
-        uint64_t reserved = 0, used = 0;
-        if (pool_bytes(P.small, reserved, used) && reserved > used + P.keep / 8) cudaMemPoolTrimTo(P.small, used + P.keep / 8);
-        return;
-    }
-    Block k{p, b.held, b.h->stream, nullptr};
-    if (cudaEventCreateWithFlags(&k.done, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventRecord(k.done, k.stream) != cudaSuccess) {
-        cudaGetLastError();
-        if (k.done) cudaEventDestroy(k.done);
-        cudaFree(p);
-        return;
-    }
-    P.blocks.push_back(k);
-    P.idle += k.bytes;
-    while (P.idle > P.keep) drop_oldest(P);
+    if (b.source == FROM_DEVICE) cudaFree(p);
+    else if (b.source == FROM_POOL) cudaFreeAsync(p, b.h->stream);
+    else if (b.h->parking) b.h->parked.emplace_back(p, b.held);
+    else keep_block(b.h, p, b.held);
 }
 
 }  // namespace risq
@@ -227,20 +242,6 @@ void mem_free(void* p) {
 using namespace risq;
 
 namespace {
-
-// Make the handle's device current for the duration of a call.
-struct DeviceGuard {
-    int prev = -1;
-    explicit DeviceGuard(int dev) {
-        cudaGetDevice(&prev);
-        if (prev != dev) cudaSetDevice(dev);
-    }
-    ~DeviceGuard() {
-        int cur = -1;
-        cudaGetDevice(&cur);
-        if (prev >= 0 && cur != prev) cudaSetDevice(prev);
-    }
-};
 
 size_t combine_2_host(long p, long q) {
     long i = p < 0 ? -p : p, j = q < 0 ? -q : q;
@@ -315,6 +316,7 @@ void risqgpu_destroy(risqgpu_t* h) {
     if (h->stream) cudaStreamSynchronize(h->stream);
     h->stream = h->own_stream;  // the frees are ordered on the handle's own stream
     free_dets(h);
+    drop_parked(h, true);
     free_mlp(h);
     dfree(h->d_h1);
     dfree(h->d_h2);
@@ -333,7 +335,9 @@ int risqgpu_set_dets(risqgpu_t* h, const uint64_t* dets, size_t n, size_t n_stor
     if (!h) return RISQGPU_ERR_INVALID;
     DeviceGuard g(h->device);
     h->err.clear();
-    return set_dets_impl(h, dets, n, n_stored_h, diag);
+    const int rc = set_dets_impl(h, dets, n, n_stored_h, diag);
+    if (rc) drop_parked(h, true);  // no build will follow
+    return rc;
 }
 
 int risqgpu_build_h(risqgpu_t* h, int precision, int builder, risqgpu_hstats* stats) {
@@ -454,6 +458,7 @@ int risqgpu_set_memory_limit(risqgpu_t* h, size_t bytes) {
         // the caller shares the device: hand back what no buffer uses
         DeviceGuard g(h->device);
         cudaStreamSynchronize(h->stream);
+        drop_parked(h, false);
         pool_trim(h->device);
     }
     return RISQGPU_OK;
@@ -463,6 +468,15 @@ int risqgpu_memory_used(const risqgpu_t* h, size_t* used, size_t* limit) {
     if (!h) return RISQGPU_ERR_INVALID;
     if (used) *used = h->mem_used;
     if (limit) *limit = h->mem_limit;
+    return RISQGPU_OK;
+}
+
+int risqgpu_release_memory(risqgpu_t* h) {
+    if (!h) return RISQGPU_ERR_INVALID;
+    DeviceGuard g(h->device);
+    RQ_TRY(sync(h, "release memory"));
+    drop_parked(h, false);
+    pool_trim(h->device);
     return RISQGPU_OK;
 }
 

@@ -174,6 +174,12 @@ struct risqgpu {
     int dav_space = 0;
     int dav_keep = 0;
 
+    // large blocks of a matrix that went, for the build that follows; whether freed ones join
+    // them; and whether large buffers take no more than they need
+    std::vector<std::pair<void*, size_t>> parked;
+    bool parking = false;
+    bool exact = false;
+
     // page-locked results of a Davidson iteration, and the device flag that a sigma looks at
     // before it starts (null, or set by a solve that has ended)
     double* pinned = nullptr;
@@ -191,22 +197,50 @@ struct risqgpu {
 
 namespace risq {
 
+// Make the handle's device current for the duration of a call.
+struct DeviceGuard {
+    int prev = -1;
+    explicit DeviceGuard(int dev) {
+        cudaGetDevice(&prev);
+        if (prev != dev) cudaSetDevice(dev);
+    }
+    ~DeviceGuard() {
+        int cur = -1;
+        cudaGetDevice(&cur);
+        if (prev >= 0 && cur != prev) cudaSetDevice(prev);
+    }
+};
+
 // Device memory of the handles.  Every buffer comes from dalloc and goes back through
-// dfree; a ledger records each one's handle and size (mem_used).  A handle without a
-// memory bound takes its buffers from memory that the process keeps per device (capi.cu):
-// a build or a solve makes and drops 50 to 90 buffers, and with cudaMalloc / cudaFree those
-// cost more than its kernels (131,611 determinants: 11.4 ms of a 20 ms build; 551,147: 49
-// of 113 ms).  At most POOL_KEEP idle bytes and an eighth more (and an eighth of the device
-// and an eighth more) are kept; all are given back when the last handle on the device goes,
-// and before any allocation is reported as failed.  A handle with a memory bound allocates
-// from the device directly, so that what it holds is what its bound counts.
-constexpr size_t POOL_KEEP = (size_t)12 << 30;
+// dfree; a ledger records each one's handle and size (mem_used, with what a block is larger
+// than was asked for).  A handle without a memory bound takes its buffers from memory that
+// the process keeps per device (capi.cu): a build or a solve makes and drops 50 to 90 buffers,
+// and with cudaMalloc / cudaFree those cost more than its kernels (131,611 determinants:
+// 11.4 ms of a 20 ms build; 551,147: 49 of 113 ms).  At most POOL_KEEP bytes of idle large
+// blocks (a sixteenth of the device) and a pool of at most SMALL_KEEP bytes, or what is in
+// use of it, are kept; all are given back when the last handle on the device goes, when a
+// caller asks (risqgpu_release_memory), and before any allocation is reported as failed.  A
+// handle with a memory bound allocates from the device directly, so that what it holds is
+// what its bound counts.
+//
+// The large blocks of a matrix that goes because another set or build follows stay with the
+// handle (`parked`) until that build returns: unmapping and mapping them again took from 0.1
+// to 2.5 s for 120 GB on a host whose GPUs are shared.
+constexpr size_t POOL_KEEP = (size_t)6 << 30, SMALL_KEEP = (size_t)2 << 30;
 int mem_alloc(risqgpu* h, void** p, size_t bytes);  // RISQGPU status; sets h->err
 void mem_free(void* p);
+void drop_parked(risqgpu* h, bool reuse);  // to the idle blocks, or to the device
 int pool_acquire(int device);  // one call per handle made on the device
 void pool_release(int device);  // one call per handle destroyed, after its buffers
 void pool_trim(int device);
 size_t pool_idle(int device);  // idle bytes kept
+
+// While it lives, large blocks that the handle frees are parked.
+struct Parking {
+    risqgpu* h;
+    explicit Parking(risqgpu* h_) : h(h_) { h->parking = true; }
+    ~Parking() { h->parking = false; }
+};
 
 // Free a device pointer (ignores null) and reset it.  Stream-ordered: work already issued
 // on the handle's stream may still use the buffer.
@@ -223,19 +257,20 @@ inline int dalloc(risqgpu* h, T*& p, size_t count) {
     return mem_alloc(h, (void**)&p, count * sizeof(T));
 }
 
-// Device bytes that new allocations may take: free device memory and what is kept idle,
-// bounded by the handle's limit.  The device is asked only when the idle memory does not
+// Device bytes that new allocations may take: free device memory and what is kept idle or
+// parked, bounded by the handle's limit.  The device is asked only when the latter does not
 // cover `need`: on a host whose GPUs are shared cudaMemGetInfo was seen to take from 0.1 to
 // 75 ms (a build of 551,147 determinants: 47 ms).
 inline size_t mem_available(risqgpu* h, size_t need) {
-    const size_t idle = h->mem_limit ? 0 : pool_idle(h->device);
-    if (idle >= need) return idle;
+    size_t idle = pool_idle(h->device);
+    for (const auto& b : h->parked) idle += b.second;
+    if (!h->mem_limit && idle >= need) return idle;
     size_t fr = 0, tot = 0;
     if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
         cudaGetLastError();
         fr = 0;
     }
-    fr += pool_idle(h->device);
+    fr += idle;
     if (h->mem_limit) fr = std::min(fr, h->mem_limit > h->mem_used ? h->mem_limit - h->mem_used : (size_t)0);
     return fr;
 }

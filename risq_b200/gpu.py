@@ -247,6 +247,11 @@ class GpuHam:
         A.check(A.lib().risqgpu_memory_used(self._h, C.byref(u), C.byref(l)), self._h)
         return u.value, l.value
 
+    def release_memory(self):
+        """Give the device memory the library keeps for reuse back to the device
+        (risqgpu_release_memory)."""
+        A.check(A.lib().risqgpu_release_memory(self._h), self._h)
+
     def set_stream(self, stream_ptr):
         """Issue the handle's work on a caller cudaStream_t (int address); None = own stream."""
         A.check(A.lib().risqgpu_set_stream(self._h, C.c_void_p(stream_ptr) if stream_ptr else None), self._h)
