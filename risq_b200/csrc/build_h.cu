@@ -932,10 +932,8 @@ int launch_fill(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, cons
         SigmaIO{})
     if constexpr (OUT != OUT_BINS)
         if (precision == RISQGPU_FP64) RQ_FILL(1);
-    if constexpr (OUT != OUT_UPPER) {
-        if (precision == RISQGPU_FP32) RQ_FILL(2);
-        if (precision == RISQGPU_MIXED) RQ_FILL(3);
-    }
+    if (precision == RISQGPU_FP32) RQ_FILL(2);
+    if (precision == RISQGPU_MIXED) RQ_FILL(3);
     if constexpr (OUT == OUT_ROWS)
         if (precision == RISQGPU_COLS) RQ_FILL(4);
 #undef RQ_FILL
@@ -1017,11 +1015,52 @@ __global__ void k_panel_starts(const int64_t* __restrict__ row_start, int64_t n,
         out[P] = row_start[min(n, P << rb)];
 }
 
+// Candidates of every row (the upper triangle's): row starts, and their number.
+template <int W, int OUT>
+int count_candidates(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int* counter, int threads,
+                     cudaEvent_t* ev, int64_t& cap) {
+    const int64_t n = (int64_t)h->N;
+    int64_t* cnt = nullptr;
+    char* tmp = nullptr;
+    ScopedFree<2> release(cnt, tmp);
+    RQ_TRY(dalloc(h, cnt, n + 1));
+    RQ_TRY(dalloc(h, h->d_row_start, n + 1));
+    RQ_TRY(dalloc(h, h->d_row_len, n));
+    RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
+    RQ_CUDA(h, cudaEventRecord(ev[0], h->stream));
+    k_build_rows<W, 0, OUT><<<resident(h, k_build_rows<W, 0, OUT>, threads), threads, 0, h->stream>>>(
+        v, I, thr, TileOut{}, counter, cnt, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, n, 0, SigmaIO{});
+    RQ_CUDA(h, cudaEventRecord(ev[1], h->stream));
+    RQ_TRY(check_launch(h, "count rows"));
+    size_t tb = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, h->d_row_start, (int)(n + 1), h->stream);
+    RQ_TRY(dalloc(h, tmp, tb));
+    RQ_CUDA(h, cudaMemsetAsync(cnt + n, 0, sizeof(int64_t), h->stream));
+    cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, h->d_row_start, (int)(n + 1), h->stream);
+    RQ_CUDA(h, cudaMemcpyAsync(&cap, h->d_row_start + n, sizeof(int64_t), cudaMemcpyDeviceToHost, h->stream));
+    return sync(h, "count rows");
+}
+
+// This handle's panels of 2^rb rows, and the candidates before each panel of all.
+int panel_starts(risqgpu* h, int rb, std::vector<int64_t>& ps) {
+    const int64_t n = (int64_t)h->N, np = (n + ((int64_t)1 << rb) - 1) >> rb;
+    h->n_panels = np;
+    ps.resize((size_t)np + 1);
+    int64_t* dps = nullptr;
+    ScopedFree<1> release(dps);
+    RQ_TRY(dalloc(h, dps, (size_t)np + 1));
+    k_panel_starts<<<grid_for(h, np + 1), 256, 0, h->stream>>>(h->d_row_start, n, rb, np, dps);
+    RQ_CUDA(h, cudaMemcpyAsync(ps.data(), dps, sizeof(int64_t) * (np + 1), cudaMemcpyDeviceToHost, h->stream));
+    RQ_TRY(sync(h, "panel starts"));
+    own_panels(h, ps, h->part_p_lo, h->part_p_hi);
+    return RISQGPU_OK;
+}
+
 // FP64 upper triangle: rows filled chunk by chunk of whole panels into a CSR buffer that
 // holds one chunk, each chunk regrouped into tiles before the next is filled.
 template <int W>
 int fill_upper64(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int* counter, int threads,
-                 int64_t cap, int64_t& nnz) {
+                 int64_t cap, Tiles64Builder& tb) {
     const int64_t n = (int64_t)h->N;
     if (tile_shape64(n, cap, h->tile_rb, h->tile_cb) != RISQGPU_OK) {
         h->err = "determinant set too large for the tiled upper-triangle layout";
@@ -1029,26 +1068,17 @@ int fill_upper64(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int
     }
     const int rb = h->tile_rb;
     h->tile_kb = rb;
-    const int64_t np = (n + ((int64_t)1 << rb) - 1) >> rb;
-    h->n_panels = np;
-    std::vector<int64_t> ps((size_t)np + 1);
-    {
-        int64_t* dps = nullptr;
-        ScopedFree<1> release(dps);
-        RQ_TRY(dalloc(h, dps, (size_t)np + 1));
-        k_panel_starts<<<grid_for(h, np + 1), 256, 0, h->stream>>>(h->d_row_start, n, rb, np, dps);
-        RQ_CUDA(h, cudaMemcpyAsync(ps.data(), dps, sizeof(int64_t) * (np + 1), cudaMemcpyDeviceToHost, h->stream));
-        RQ_TRY(sync(h, "panel starts"));
-    }
-    own_panels(h, ps, h->part_p_lo, h->part_p_hi);
+    std::vector<int64_t> ps;
+    RQ_TRY(panel_starts(h, rb, ps));
     const int64_t own_lo = h->part_p_lo, own_hi = h->part_p_hi;
     // rows of other ranks' panels hold no stored pairs here
     RQ_CUDA(h, cudaMemsetAsync(h->d_row_len, 0, sizeof(int32_t) * n, h->stream));
     // bytes of the tiled arrays, per row tile data and accumulators, plus a margin that grows
     // with the set.  An element takes 10 bytes, about an eighth more for its group's padding,
     // and its share of the group's slots (136 bytes a group; 1.0 at the four elements a row
-    // and tile of a 9,150,723-determinant set): chunks are cut for 14, and for 11.25, below
-    // what any set takes, only where 14 would refuse a set that may fit.
+    // and tile of a 9,150,723-determinant set, up to 24 bytes in all with one): chunks are cut
+    // for 14, and for 11.25, below what any set takes, only where 14 would refuse a set that
+    // may fit.  A set that then does not fit after all is stored as pair lists.
     const int64_t own_cap = ps[own_hi] - ps[own_lo];
     auto fixed_for = [&](size_t quarters) {
         const size_t need = (size_t)own_cap * quarters / 4 + (size_t)n * 40;
@@ -1071,7 +1101,6 @@ int fill_upper64(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int
     RQ_TRY(dalloc(h, c64, (size_t)max_chunk));
     RQ_TRY(dalloc(h, code, (size_t)max_chunk));
     RQ_TRY(dalloc(h, t64, (size_t)max_chunk));
-    Tiles64Builder tb;
     RQ_TRY(tb.begin(h));
     for (size_t c = 0; c + 1 < cuts.size(); c++) {
         const int64_t p_lo = cuts[c], p_hi = cuts[c + 1];
@@ -1082,16 +1111,62 @@ int fill_upper64(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int
     }
     // the chunk's arrays go before the leftovers of all chunks are gathered
     dfree(ccols); dfree(c64); dfree(code); dfree(t64);
-    RQ_TRY(tb.finish());
+    return tb.gather();
+}
+
+// The stored elements, every one of which went into the tiles or the leftovers exactly once.
+int check_stored(risqgpu* h, int64_t stored, int64_t& nnz) {
     RQ_TRY(count_rows(h, nnz));
-    // every stored element went into the tiles or the leftovers exactly once
-    if (nnz != tb.stored) {
-        h->err = "tiled layout holds " + std::to_string(tb.stored) + " elements for " + std::to_string(nnz) + " stored";
+    if (nnz != stored) {
+        h->err = "tiled layout holds " + std::to_string(stored) + " elements for " + std::to_string(nnz) + " stored";
         return RISQGPU_ERR_INVALID;
     }
     dfree(h->d_row_start);
     dfree(h->d_row_len);
     return RISQGPU_OK;
+}
+
+// The upper triangle as pair lists, from CSR rows that hold one chunk.
+template <int W>
+int fill_list(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int precision, int* counter, int threads,
+              TileListBuilder& tb) {
+    const int64_t n = (int64_t)h->N;
+    if (tile_shape_list(n, h->tile_rb, h->tile_cb) != RISQGPU_OK) {
+        h->err = "determinant set too large for the tiled upper-triangle layout";
+        return RISQGPU_ERR_INVALID;
+    }
+    h->exact = true;
+    const int rb = h->tile_rb;
+    std::vector<int64_t> ps;
+    RQ_TRY(panel_starts(h, rb, ps));
+    const int64_t own_lo = h->part_p_lo, own_hi = h->part_p_hi, own_cap = ps[own_hi] - ps[own_lo];
+    RQ_CUDA(h, cudaMemsetAsync(h->d_row_len, 0, sizeof(int32_t) * n, h->stream));
+    // the lists, per row tile data and accumulators, and a margin that grows with the set (at
+    // most 256 MiB) for the tiles' records
+    const size_t per_el = 4 + (precision == RISQGPU_FP32 ? 4 : 8);
+    const size_t need = (size_t)own_cap * per_el + (size_t)n * 32;
+    const size_t fixed = need + std::max((size_t)8 << 20, std::min((size_t)256 << 20, need / 32));
+    std::vector<int64_t> cuts;
+    int64_t max_chunk = 0;
+    RQ_TRY(chunk_cuts(h, ps, own_lo, own_hi, fixed, per_el, cuts, max_chunk));
+    int32_t* ccols = nullptr;
+    double* c64 = nullptr;
+    float *c32 = nullptr, *clo = nullptr;
+    ScopedFree<4> release(ccols, c64, c32, clo);
+    RQ_TRY(tb.begin(h, precision, own_cap));
+    RQ_TRY(dalloc(h, ccols, (size_t)max_chunk));
+    if (precision == RISQGPU_FP64) RQ_TRY(dalloc(h, c64, (size_t)max_chunk));
+    else RQ_TRY(dalloc(h, c32, (size_t)max_chunk));
+    if (precision == RISQGPU_MIXED) RQ_TRY(dalloc(h, clo, (size_t)max_chunk));
+    for (size_t c = 0; c + 1 < cuts.size(); c++) {
+        const int64_t p_lo = cuts[c], p_hi = cuts[c + 1];
+        RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
+        RQ_TRY((launch_fill<W, OUT_UPPER>(h, v, I, thr, TileOut{}, precision, counter, threads, ccols, c64, c32, clo,
+                                          p_lo << rb, std::min(n, p_hi << rb), ps[p_lo])));
+        RQ_TRY(tb.chunk(p_lo, p_hi, h->d_row_start, ps[p_lo], h->d_row_len, ccols, c64, c32, clo));
+    }
+    dfree(ccols); dfree(c64); dfree(c32); dfree(clo);
+    return tb.gather();
 }
 
 // First bin of every block of rows: block b holds the windows from its own column on.
@@ -1110,7 +1185,7 @@ __global__ void k_bin_off(int64_t n_blocks, int64_t n_windows, int cb, int kb, i
 // chunk rather than two copies of the matrix.
 template <int W>
 int build_tiled(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int precision, int* counter, int threads,
-                cudaEvent_t* ev, std::chrono::steady_clock::time_point& t1, int64_t& cap, int64_t& nnz) {
+                cudaEvent_t* ev, std::chrono::steady_clock::time_point& t1, int64_t& cap, TileBuilder& tb) {
     const int64_t n = (int64_t)h->N;
     int rb = 0, cb = 0, kb = 0;
     if (tile_shape(n, rb, cb, kb) != RISQGPU_OK) {
@@ -1146,7 +1221,6 @@ int build_tiled(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int 
         v, I, thr, T, counter, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, n, 0, SigmaIO{});
     RQ_CUDA(h, cudaEventRecord(ev[1], h->stream));
     RQ_TRY(check_launch(h, "count bins"));
-    TileBuilder tb;
     RQ_TRY(tb.plan(h, hist, bin_off, nblk));
     t1 = std::chrono::steady_clock::now();
     RQ_CUDA(h, cudaEventRecord(ev[2], h->stream));
@@ -1197,8 +1271,60 @@ int build_tiled(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int 
                                          p_lo << rb, std::min(n, p_hi << rb), 0)));
         RQ_TRY(tb.chunk(p_lo, p_hi, T.el0, cur, code, c32, clo));
     }
-    RQ_TRY(tb.finish());
-    nnz = tb.stored;
+    return RISQGPU_OK;
+}
+
+// RISQGPU_TEST_TILE_OOM: the tests' way to the pair lists on sets that fit in groups.
+bool test_oom() { return std::getenv("RISQGPU_TEST_TILE_OOM") != nullptr; }
+
+// Upper-triangle storage: in groups, or where memory runs out on some rank, as pair lists.
+template <int W>
+int build_upper(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int precision, int* counter, int threads,
+                cudaEvent_t* ev, std::chrono::steady_clock::time_point& t1, int64_t& cap, int64_t& nnz) {
+    ScopedFree<1> release(h->d_agree);
+    if (h->part_n > 1) RQ_TRY(dalloc(h, h->d_agree, 1));
+    auto counted = [&]() -> int {
+        RQ_TRY((count_candidates<W, OUT_UPPER>(h, v, I, thr, counter, threads, ev, cap)));
+        t1 = std::chrono::steady_clock::now();
+        RQ_CUDA(h, cudaEventRecord(ev[2], h->stream));
+        return RISQGPU_OK;
+    };
+    bool agreed = false;
+    auto groups = [&]() -> int {
+        if (precision == RISQGPU_FP64) {
+            Tiles64Builder tb;
+            int rc = counted();
+            if (!rc) rc = fill_upper64<W>(h, v, I, thr, counter, threads, cap, tb);
+            RQ_TRY(part_agree(h, !rc && test_oom() ? RISQGPU_ERR_OOM : rc));
+            agreed = true;
+            RQ_TRY(tb.finish());
+            return check_stored(h, tb.stored, nnz);
+        }
+        TileBuilder tb;
+        const int rc = build_tiled<W>(h, v, I, thr, precision, counter, threads, ev, t1, cap, tb);
+        RQ_TRY(part_agree(h, !rc && test_oom() ? RISQGPU_ERR_OOM : rc));
+        agreed = true;
+        RQ_TRY(tb.finish());
+        nnz = tb.stored;
+        return RISQGPU_OK;
+    };
+    int rc = groups();
+    if (rc == RISQGPU_ERR_OOM && !(agreed && h->part_n > 1)) {
+        const std::string first = h->err;
+        free_tiles(h);
+        TileListBuilder tb;
+        rc = counted();
+        if (!rc) rc = fill_list<W>(h, v, I, thr, precision, counter, threads, tb);
+        rc = part_agree(h, rc);
+        if (rc) {
+            if (!first.empty()) h->err = first + "; as pair lists: " + h->err;
+            return rc;
+        }
+        RQ_TRY(tb.finish());
+        RQ_TRY(check_stored(h, tb.stored, nnz));
+        h->err.clear();
+    }
+    RQ_TRY(rc);
     RQ_CUDA(h, cudaEventRecord(ev[3], h->stream));
     return RISQGPU_OK;
 }
@@ -1225,7 +1351,7 @@ int finish_build(risqgpu* h, int precision, int upper, int64_t cap, int64_t nnz,
         st->ms_count = std::chrono::duration<double, std::milli>(t1 - t0).count();
         st->ms_fill = std::chrono::duration<double, std::milli>(t3 - t2).count();
         size_t vb = precision == RISQGPU_FP64 ? 8 : (precision == RISQGPU_FP32 ? 4 : (precision == RISQGPU_COLS ? 0 : 8));
-        st->bytes_csr = (uint64_t)nnz * ((upper ? 2 : 4) + vb);
+        st->bytes_csr = (uint64_t)nnz * ((upper && !h->tile_list ? 2 : 4) + vb);
         st->n_tiles = (uint64_t)h->n_tiles;
         st->nnz_dense = h->n_dense_el;
     }
@@ -1248,8 +1374,7 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
     const bool incremental = h->nsh > 0 && h->d_prev_row_start != nullptr;
     int32_t* prev_inv = nullptr;
     int* counter = nullptr;
-    int64_t* cnt = nullptr;
-    ScopedFree<3> release(prev_inv, counter, cnt);
+    ScopedFree<2> release(prev_inv, counter);
     if (incremental) {
         RQ_TRY(dalloc(h, prev_inv, h->prev_N));
         k_invert<<<grid_for(h, h->prev_N), 256, 0, h->stream>>>(h->d_prev_orig, (int64_t)h->prev_N, prev_inv);
@@ -1263,47 +1388,15 @@ int build_rows(risqgpu* h, int precision, int upper, double thr, risqgpu_hstats*
     cudaEvent_t* ev = be.ev;
     for (int k = 0; k < 4; k++) RQ_CUDA(h, cudaEventCreate(&ev[k]));
     auto t0 = clk::now();
-    if (upper && precision != RISQGPU_FP64) {
+    if (upper) {
         auto t1 = t0;
         int64_t cap = 0, nnz = 0;
-        RQ_TRY(build_tiled<W>(h, v, I, thr, precision, counter, threads, ev, t1, cap, nnz));
+        RQ_TRY(build_upper<W>(h, v, I, thr, precision, counter, threads, ev, t1, cap, nnz));
         return finish_build(h, precision, upper, cap, nnz, t0, t1, t1, ev, st);
-    }
-    RQ_TRY(dalloc(h, cnt, n + 1));
-    RQ_TRY(dalloc(h, h->d_row_start, n + 1));
-    RQ_TRY(dalloc(h, h->d_row_len, n));
-    RQ_CUDA(h, cudaMemsetAsync(counter, 0, sizeof(int), h->stream));
-    RQ_CUDA(h, cudaEventRecord(ev[0], h->stream));
-    auto count = [&](auto kern) {
-        kern<<<resident(h, kern, threads), threads, 0, h->stream>>>(v, I, thr, TileOut{}, counter, cnt, nullptr, nullptr,
-                                                                    nullptr, nullptr, nullptr, nullptr, 0, n, 0,
-                                                                    SigmaIO{});
-    };
-    if (upper) count(k_build_rows<W, 0, OUT_UPPER>);
-    else count(k_build_rows<W, 0, OUT_ROWS>);
-    RQ_CUDA(h, cudaEventRecord(ev[1], h->stream));
-    RQ_TRY(check_launch(h, "count rows"));
-    {
-        size_t tb = 0;
-        cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, h->d_row_start, (int)(n + 1), h->stream);
-        char* tmp = nullptr;
-        ScopedFree<1> release_tmp(tmp);
-        RQ_TRY(dalloc(h, tmp, tb));
-        RQ_CUDA(h, cudaMemsetAsync(cnt + n, 0, sizeof(int64_t), h->stream));
-        cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, h->d_row_start, (int)(n + 1), h->stream);
     }
     int64_t cap = 0;
-    RQ_CUDA(h, cudaMemcpyAsync(&cap, h->d_row_start + n, sizeof(int64_t), cudaMemcpyDeviceToHost, h->stream));
-    RQ_TRY(sync(h, "count rows"));
-    dfree(cnt);
+    RQ_TRY((count_candidates<W, OUT_ROWS>(h, v, I, thr, counter, threads, ev, cap)));
     auto t1 = clk::now();
-    if (upper) {
-        int64_t nnz = 0;
-        RQ_CUDA(h, cudaEventRecord(ev[2], h->stream));
-        RQ_TRY(fill_upper64<W>(h, v, I, thr, counter, threads, cap, nnz));
-        RQ_CUDA(h, cudaEventRecord(ev[3], h->stream));
-        return finish_build(h, precision, upper, cap, nnz, t0, t1, t1, ev, st);
-    }
     {
         // refuse up front when the rows cannot be stored, leaving the handle unchanged
         size_t vb = precision == RISQGPU_FP64 ? 8 : (precision == RISQGPU_FP32 ? 4 : (precision == RISQGPU_COLS ? 0 : 8));
@@ -1533,7 +1626,10 @@ static int build_matrix(risqgpu* h, int precision, int builder, risqgpu_hstats* 
     int rc = narrow(h)   ? build_rows<0>(h, vprec, upper, thr, st)
              : h->W == 1 ? build_rows<1>(h, vprec, upper, thr, st)
                          : build_rows<2>(h, vprec, upper, thr, st);
-    if (rc) return rc;
+    if (rc) {
+        free_csr(h);  // what the build had allocated
+        return rc;
+    }
     h->built = true;
     if (h->nsh > 0) free_prev(h);
     h->nsh = 0;

@@ -116,6 +116,7 @@ struct risqgpu {
     // blocks of 2^tile_kb rows.  A dense (panel, window) tile holds its blocks' rows in
     // groups of 32; the pairs of sparse tiles are the panel's leftovers.
     bool tiled = false;
+    bool tile_list = false;           // as pair lists, see tiles_list.cuh
     int tile_rb = 0, tile_cb = 0, tile_kb = 0;
     int64_t n_panels = 0;
     int64_t n_tiles = 0;
@@ -127,6 +128,9 @@ struct risqgpu {
     int32_t* d_tile_blk = nullptr;    // n_tiles + 1: first block record of each tile
     float2* d_tile_bound = nullptr;   // largest row sum of |H| in each tile, bound on its column sums
     risq::TileBlock* d_tile_blocks = nullptr;
+    int64_t* d_tile_off = nullptr;    // pair lists: first pair and pairs of each tile; the codes,
+    int32_t* d_tile_len = nullptr;    // a panel's leftovers after its tiles (values: d_val64, ...)
+    uint32_t* d_el_idx = nullptr;
     std::vector<risq::TileChunk> chunks;  // the element arrays, chunk of panels by chunk
     risq::TileChunk* d_chunk_tab = nullptr;
     int64_t* d_left_off = nullptr;    // per panel: first leftover, their number; then their
@@ -153,6 +157,7 @@ struct risqgpu {
     int part_rank = 0, part_n = 1;
     risqgpu_allreduce_fn part_reduce = nullptr;
     void* part_user = nullptr;
+    unsigned long long* d_agree = nullptr;  // while a partitioned build runs: see part_agree
     int64_t part_p_lo = 0, part_p_hi = 0;
 
     // previous build kept for an incremental extension
@@ -335,12 +340,16 @@ int permute_out(risqgpu* h, const double* yi, double* y);
 // tiled upper-triangle storage (tiles.cu)
 int tile_shape(int64_t N, int& rb, int& cb, int& kb);
 int tile_shape64(int64_t N, int64_t pairs, int& rb, int& cb);
+int tile_shape_list(int64_t N, int& rb, int& cb);
 int sigma_tiles(risqgpu* h, const void* x, void* y, int kind);
 // FP64 sigma of a matrix-free build (build_h.cu), internal order
 int sigma_matrix_free(risqgpu* h, const double* x, double* y);
 // Sum `count` int64 values in place across the partition's ranks (the caller's all-reduce,
 // on the handle's stream).
 int part_allreduce(risqgpu* h, void* buf_dev, size_t count);
+// The ranks' common result of a step that each took for itself: out of memory anywhere is
+// out of memory everywhere, so that all go on to the same collectives.
+int part_agree(risqgpu* h, int rc);
 int tiles_coo(risqgpu* h, int32_t* p, int32_t* q, double* v);
 int tiles_self_energy(risqgpu* h, double energy, double gmin, double* out);
 int tiles_rows(risqgpu* h, const uint32_t* mark, int64_t* out_r, int64_t* out_c, double* out_v,
@@ -390,8 +399,33 @@ struct Tiles64Builder {
     int begin(risqgpu* h);
     int chunk(int64_t p_lo, int64_t p_hi, const int64_t* row_start, int64_t base, const int32_t* row_len,
               const int32_t* cols, const double* vin, uint32_t* code, double* val, int64_t cap);
+    int gather();
     int finish();
     ~Tiles64Builder();
+};
+
+// The upper triangle as pair lists (tiles_list.cuh), from CSR rows, chunk by chunk of panels.
+struct TileListBuilder {
+    risqgpu* h = nullptr;
+    int precision = 0;
+    unsigned long long* row_abs = nullptr;          // N: sum_q |H_pq| over both triangles, units of 2^-32
+    unsigned long long* absmax = nullptr;
+    struct Part {                                   // the tiles of a chunk
+        int64_t tiles;
+        int32_t* win;
+        int64_t* off;
+        int32_t* len;
+        float2* bound;
+    };
+    std::vector<Part> parts;
+    std::vector<int64_t> panel_tile;
+    int64_t tiles = 0, dense = 0, stored = 0, cap = 0;
+    int begin(risqgpu* h, int precision, int64_t cap);
+    int chunk(int64_t p_lo, int64_t p_hi, const int64_t* row_start, int64_t base, const int32_t* row_len,
+              const int32_t* cols, const double* v64, const float* v32, const float* vlo);
+    int gather();
+    int finish();
+    ~TileListBuilder();
 };
 
 // davidson (davidson.cu)

@@ -583,17 +583,18 @@ __global__ void __launch_bounds__(CT) k_tile_count(int64_t N, int64_t p_lo, int6
     }
 }
 
-// Scatter the chunk's pairs: those of dense tiles, tile by tile, into code / val, the
-// leftovers in row order.  off: first element, tile and leftover of every panel, in the
-// chunk's arrays.  Also adds |H_pq| to the row sums of both p and q (units of 2^-32:
+// Scatter the chunk's pairs: those of dense tiles, tile by tile, into code / val / lo, the
+// leftovers in row order into lcol / lval / llo.  off: first element, tile and leftover of
+// every panel.  A tile's place goes into its block, or into t_off / t_len.  Also adds |H_pq| to the row sums of both p and q (units of 2^-32:
 // integer sums are exact, so the sums and the fixed-point scale derived from them do not
 // depend on the order of the additions, nor on how the rows are split between ranks).
+template <typename V, bool VLO>
 __global__ void __launch_bounds__(CT) k_tile_scatter(
     int64_t N, int64_t p_lo, int64_t p_hi, int rb, int cb, const int64_t* __restrict__ row_start, int64_t base,
-    const int32_t* __restrict__ row_len, const int32_t* __restrict__ cols, const double* __restrict__ vin,
-    const PanelBase* __restrict__ off, int64_t left0, const int32_t* __restrict__ left_len, int32_t* __restrict__ tile_win,
-    TileBlock* __restrict__ blocks, int64_t* __restrict__ row_left, uint32_t* __restrict__ code,
-    double* __restrict__ val, uint32_t* __restrict__ lcol, double* __restrict__ lval,
+    const int32_t* __restrict__ row_len, const int32_t* __restrict__ cols, const V* __restrict__ vin,
+    const float* __restrict__ lin, const PanelBase* __restrict__ off, int64_t left0, const int32_t* __restrict__ left_len,
+    int32_t* __restrict__ tile_win, TileBlock* __restrict__ blocks, int64_t* __restrict__ t_off, int32_t* __restrict__ t_len,
+    int64_t* __restrict__ row_left, uint32_t* code, V* val, float* lo, uint32_t* lcol, V* lval, float* llo,
     unsigned long long* __restrict__ row_abs) {
     extern __shared__ int32_t sm_i[];
     int32_t* cursor = sm_i;              // per window: next dense slot (panel-relative), or -1
@@ -639,9 +640,14 @@ __global__ void __launch_bounds__(CT) k_tile_scatter(
             if (c > 0 && dense_tile(c, window_width(N, J0 + b, cb))) {
                 const long long t = pb.tile + ex_t;
                 tile_win[t] = (int32_t)(J0 + b);
-                blocks[t].el = pb.el + ex_el;
-                blocks[t].len = c;
-                blocks[t].row = (int32_t)r0;
+                if (blocks) {
+                    blocks[t].el = pb.el + ex_el;
+                    blocks[t].len = c;
+                    blocks[t].row = (int32_t)r0;
+                } else {
+                    t_off[t] = pb.el + ex_el;
+                    t_len[t] = c;
+                }
                 cursor[b] = (int32_t)ex_el;
                 ex_el += c;
                 ex_t++;
@@ -690,17 +696,19 @@ __global__ void __launch_bounds__(CT) k_tile_scatter(
                 if (dense && lane == leader) slot = atomicAdd(&cursor[bin], __popc(grp));
                 slot = __shfl_sync(FULL, slot, leader);
                 if (act) {
-                    const double v = vin[s + k];
+                    const V v = vin[s + k];
                     if (left) {
                         const int64_t pos = pb.block + lnext + __popc(ml & lt);
                         lcol[pos] = (uint32_t)q;
                         lval[pos] = v;
+                        if constexpr (VLO) llo[pos] = lin[s + k];
                     } else {
                         const int64_t pos = pb.el + slot + __popc(grp & lt);
                         code[pos] = (lr << cb) | ((uint32_t)q & cmask);
                         val[pos] = v;
+                        if constexpr (VLO) lo[pos] = lin[s + k];
                     }
-                    const unsigned long long ai = (unsigned long long)llrint(fabs(v) * 4294967296.0);
+                    const unsigned long long ai = (unsigned long long)llrint(fabs((double)v) * 4294967296.0);
                     rsum += ai;
                     atomicAdd(row_abs + q, ai);
                 }
@@ -1129,6 +1137,8 @@ __global__ void k_fixed_finish(int64_t N, const double* __restrict__ diag, const
         y[p] = (X)(diag[p] * (double)x[p] + (FX ? (double)acc[p] * inv : (double)acc[p] + (double)acc_row[p] * inv));
 }
 
+#include "tiles_list.cuh"
+
 // Calls f(p, q, v) for every stored pair (p < q, internal indices, FP64 value): one CTA
 // per panel, a warp per group of rows of its tiles, then its leftovers.
 template <typename V, bool VLO, typename F>
@@ -1248,6 +1258,15 @@ template <typename F>
 int tiles_each(risqgpu* h, F f) {
     const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(h->part_p_hi - h->part_p_lo, (int64_t)num_sms(h) * 8));
     const int64_t N = (int64_t)h->N, lo = h->part_p_lo, hi = h->part_p_hi;
+    if (h->tile_list) {
+        if (h->precision == RISQGPU_FP64)
+            k_list_each<double, false, F><<<grid, TT, 0, h->stream>>>(N, lo, hi, list_view<double>(h), f);
+        else if (h->precision == RISQGPU_MIXED)
+            k_list_each<float, true, F><<<grid, TT, 0, h->stream>>>(N, lo, hi, list_view<float>(h), f);
+        else
+            k_list_each<float, false, F><<<grid, TT, 0, h->stream>>>(N, lo, hi, list_view<float>(h), f);
+        return check_launch(h, "tiled pairs");
+    }
     if (h->precision == RISQGPU_FP64)
         k_tiles_each<double, false, F><<<grid, TT, 0, h->stream>>>(
             N, lo, hi, tile_view<double>(h, h->d_left64, nullptr), f);
@@ -1264,13 +1283,10 @@ inline int grid_n(risqgpu* h, int64_t n) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, (int64_t)num_sms(h) * 16));
 }
 
-template <typename X, typename V, bool VLO, bool EXACT>
-int launch_fx(risqgpu* h, const X* x, X* y, const TileView<V>& T) {
+template <typename X, typename V, bool EXACT, typename K, typename T_>
+int launch_sigma(risqgpu* h, const X* x, X* y, K kern, size_t smem, const T_& T) {
     using Y = typename std::conditional<EXACT, long long, X>::type;
     const int64_t N = (int64_t)h->N;
-    // x and the accumulators of a window; FP64 values: the row sums of a panel
-    const size_t smem = (((size_t)2 * sizeof(X)) << h->tile_cb) + (sizeof(V) == 8 ? (size_t)8 << h->tile_rb : 0);
-    auto kern = k_sigma_fx<X, V, VLO, EXACT>;
     RQ_CUDA(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, ST, smem);
@@ -1293,6 +1309,17 @@ int launch_fx(risqgpu* h, const X* x, X* y, const TileView<V>& T) {
     return check_launch(h, "sigma (tiles)");
 }
 
+template <typename X, typename V, bool VLO, bool EXACT>
+int launch_fx(risqgpu* h, const X* x, X* y, const V* lval, const float* llo) {
+    if (h->tile_list) {
+        const size_t smem = ((size_t)(8 + 2 * sizeof(X)) << h->tile_rb) + ((size_t)(2 * sizeof(X)) << h->tile_cb);
+        return launch_sigma<X, V, EXACT>(h, x, y, k_sigma_list<X, V, VLO, EXACT>, smem, list_view<V>(h));
+    }
+    // x and the accumulators of a window; FP64 values: the row sums of a panel
+    const size_t smem = (((size_t)2 * sizeof(X)) << h->tile_cb) + (sizeof(V) == 8 ? (size_t)8 << h->tile_rb : 0);
+    return launch_sigma<X, V, EXACT>(h, x, y, k_sigma_fx<X, V, VLO, EXACT>, smem, tile_view<V>(h, lval, llo));
+}
+
 }  // namespace
 
 int part_allreduce(risqgpu* h, void* buf_dev, size_t count) {
@@ -1305,6 +1332,21 @@ int part_allreduce(risqgpu* h, void* buf_dev, size_t count) {
         return RISQGPU_ERR_CUDA;
     }
     return check_launch(h, "all-reduce");
+}
+
+int part_agree(risqgpu* h, int rc) {
+    if (h->part_n <= 1) return rc;
+    // out of memory counts one, any other failure 2^32
+    const unsigned long long mine = rc == RISQGPU_OK ? 0ull : rc == RISQGPU_ERR_OOM ? 1ull : 1ull << 32;
+    unsigned long long all = 0;
+    RQ_CUDA(h, cudaMemcpyAsync(h->d_agree, &mine, sizeof(mine), cudaMemcpyHostToDevice, h->stream));
+    RQ_TRY(part_allreduce(h, h->d_agree, 1));
+    RQ_CUDA(h, cudaMemcpyAsync(&all, h->d_agree, sizeof(all), cudaMemcpyDeviceToHost, h->stream));
+    RQ_TRY(sync(h, "agreement of the ranks"));
+    if (rc != RISQGPU_OK && rc != RISQGPU_ERR_OOM) return rc;
+    if (all >> 32) { h->err = "another rank's build failed"; return RISQGPU_ERR_INVALID; }
+    if (all && rc == RISQGPU_OK) h->err = "another rank is out of device memory";
+    return all ? RISQGPU_ERR_OOM : RISQGPU_OK;
 }
 
 namespace {
@@ -1337,6 +1379,23 @@ int set_units(risqgpu* h, const std::vector<SigmaUnit>& us, const std::vector<in
     return RISQGPU_OK;
 }
 
+// Units of the leftovers of panel P's rows (nl of each row), about a quarter of the target
+// each, since one costs about four dense pairs.
+void left_units(std::vector<SigmaUnit>& us, std::vector<int64_t>& weight, const std::vector<int32_t>& nl, int64_t P,
+                int64_t R, int64_t N, int64_t target) {
+    const int64_t r0 = P * R, r1 = std::min(N, r0 + R);
+    int64_t lo = r0, acc = 0;
+    for (int64_t r = r0; r < r1; r++) {
+        acc += nl[(size_t)r];
+        if ((acc >= target / 4 || r + 1 == r1) && acc > 0) {
+            us.push_back({-1, (int32_t)P, (int32_t)(lo - r0), (int32_t)(r + 1 - r0), 0});
+            weight.push_back(4 * acc);
+            lo = r + 1;
+            acc = 0;
+        }
+    }
+}
+
 }  // namespace
 
 int tile_shape(int64_t N, int& rb, int& cb, int& kb) {
@@ -1366,6 +1425,13 @@ int tile_shape64(int64_t N, int64_t pairs, int& rb, int& cb) {
     // 551,147 determinants have 4 and more.
     const int64_t half = ((N + 2047) >> 11) / 2;
     cb = pairs < N * half ? 12 : 11;
+    while (cb < 16 && ((N + ((int64_t)1 << cb) - 1) >> cb) > MAX_BINS) cb++;
+    return ((N + ((int64_t)1 << cb) - 1) >> cb) <= MAX_BINS ? RISQGPU_OK : RISQGPU_ERR_INVALID;
+}
+
+int tile_shape_list(int64_t N, int& rb, int& cb) {
+    rb = 10;
+    cb = 11;
     while (cb < 16 && ((N + ((int64_t)1 << cb) - 1) >> cb) > MAX_BINS) cb++;
     return ((N + ((int64_t)1 << cb) - 1) >> cb) <= MAX_BINS ? RISQGPU_OK : RISQGPU_ERR_INVALID;
 }
@@ -1630,7 +1696,8 @@ int Tiles64Builder::chunk(int64_t p_lo, int64_t p_hi, const int64_t* row_start, 
     const size_t smem_count = sizeof(int32_t) * MAX_BINS;
     const size_t smem_scatter = sizeof(int32_t) * (MAX_BINS + ((size_t)1 << rb));
     RQ_CUDA(h, cudaFuncSetAttribute(k_tile_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_count));
-    RQ_CUDA(h, cudaFuncSetAttribute(k_tile_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_scatter));
+    RQ_CUDA(h, cudaFuncSetAttribute(k_tile_scatter<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)smem_scatter));
     const int grid = (int)std::min<int64_t>(np, (int64_t)num_sms(h) * 2);
     k_tile_count<<<grid, CT, smem_count, h->stream>>>(N, p_lo, p_hi, rb, cb, row_start, base, row_len, cols, dc,
                                                       h->d_row_nleft);
@@ -1660,9 +1727,9 @@ int Tiles64Builder::chunk(int64_t p_lo, int64_t p_hi, const int64_t* row_start, 
     RQ_TRY(dalloc(h, c.bound, (size_t)b.tile));
     RQ_TRY(dalloc(h, c.lcol, (size_t)b.block));
     RQ_TRY(dalloc(h, c.lval, (size_t)b.block));
-    k_tile_scatter<<<grid, CT, smem_scatter, h->stream>>>(N, p_lo, p_hi, rb, cb, row_start, base, row_len, cols, vin, db,
-                                                          left, h->d_row_nleft, c.win, c.blocks, h->d_row_left, code, val,
-                                                          c.lcol, c.lval, row_abs);
+    k_tile_scatter<double, false><<<grid, CT, smem_scatter, h->stream>>>(
+        N, p_lo, p_hi, rb, cb, row_start, base, row_len, cols, vin, nullptr, db, left, h->d_row_nleft, c.win, c.blocks, nullptr,
+        nullptr, h->d_row_left, code, val, nullptr, c.lcol, c.lval, nullptr, row_abs);
     RQ_TRY(check_launch(h, "tile scatter"));
     RQ_TRY(arrange_bins<double>(h, c.blocks, 0, b.tile, 0, nullptr, code, val, nullptr, counters));
     if (b.tile > 0) {
@@ -1675,8 +1742,8 @@ int Tiles64Builder::chunk(int64_t p_lo, int64_t p_hi, const int64_t* row_start, 
     return RISQGPU_OK;
 }
 
-int Tiles64Builder::finish() {
-    const int64_t N = (int64_t)h->N, np = h->n_panels;
+int Tiles64Builder::gather() {
+    const int64_t np = h->n_panels;
     for (int64_t P = h->part_p_hi; P <= np; P++) panel_tile[(size_t)P] = tiles;
     if (tiles >= INT32_MAX) { h->err = "too many tiles"; return RISQGPU_ERR_INVALID; }
     h->n_tiles = tiles;
@@ -1703,7 +1770,11 @@ int Tiles64Builder::finish() {
     RQ_TRY(gather(h->d_tile_win, &Chunk::win, tiles, &Chunk::tiles));
     RQ_TRY(gather(h->d_tile_bound, &Chunk::bound, tiles, &Chunk::tiles));
     RQ_TRY(gather(h->d_left_col, &Chunk::lcol, left, &Chunk::left));
-    RQ_TRY(gather(h->d_left64, &Chunk::lval, left, &Chunk::left));
+    return gather(h->d_left64, &Chunk::lval, left, &Chunk::left);
+}
+
+int Tiles64Builder::finish() {
+    const int64_t N = (int64_t)h->N, np = h->n_panels;
     std::vector<int32_t> tblk((size_t)tiles + 1);
     for (int64_t t = 0; t <= tiles; t++) tblk[(size_t)t] = (int32_t)t;  // a tile is one block
     RQ_TRY(dalloc(h, h->d_panel_tile, (size_t)np + 1));
@@ -1744,17 +1815,7 @@ int Tiles64Builder::finish() {
             us.push_back({(int32_t)t, (int32_t)P, (int32_t)t, (int32_t)t + 1, tb[(size_t)t].chunk});
             weight.push_back(tb[(size_t)t].len);
         }
-        const int64_t r0 = P * R, r1 = std::min(N, r0 + R);
-        int64_t lo = r0, acc = 0;
-        for (int64_t r = r0; r < r1; r++) {
-            acc += nl[(size_t)r];
-            if ((acc >= target / 4 || r + 1 == r1) && acc > 0) {
-                us.push_back({-1, (int32_t)P, (int32_t)(lo - r0), (int32_t)(r + 1 - r0), 0});
-                weight.push_back(4 * acc);
-                lo = r + 1;
-                acc = 0;
-            }
-        }
+        left_units(us, weight, nl, P, R, N, target);
     }
     return set_units(h, us, weight, target);
 }
@@ -1772,6 +1833,170 @@ Tiles64Builder::~Tiles64Builder() {
     }
 }
 
+int TileListBuilder::begin(risqgpu* h_, int precision_, int64_t cap_) {
+    h = h_;
+    precision = precision_;
+    cap = cap_;
+    const int64_t N = (int64_t)h->N;
+    panel_tile.assign((size_t)h->n_panels + 1, 0);
+    RQ_TRY(dalloc(h, h->d_row_left, (size_t)N));
+    RQ_TRY(dalloc(h, h->d_row_nleft, (size_t)N));
+    RQ_TRY(dalloc(h, row_abs, (size_t)N));
+    RQ_TRY(dalloc(h, absmax, 1));
+    RQ_TRY(dalloc(h, h->d_el_idx, (size_t)cap));
+    if (precision == RISQGPU_FP64) RQ_TRY(dalloc(h, h->d_val64, (size_t)cap));
+    else RQ_TRY(dalloc(h, h->d_val32, (size_t)cap));
+    if (precision == RISQGPU_MIXED) RQ_TRY(dalloc(h, h->d_val_lo, (size_t)cap));
+    RQ_CUDA(h, cudaMemsetAsync(h->d_row_nleft, 0, sizeof(int32_t) * N, h->stream));
+    RQ_CUDA(h, cudaMemsetAsync(row_abs, 0, sizeof(unsigned long long) * N, h->stream));
+    RQ_CUDA(h, cudaMemsetAsync(absmax, 0, sizeof(unsigned long long), h->stream));
+    return RISQGPU_OK;
+}
+
+int TileListBuilder::chunk(int64_t p_lo, int64_t p_hi, const int64_t* row_start, int64_t base, const int32_t* row_len,
+                           const int32_t* cols, const double* v64, const float* v32, const float* vlo) {
+    const int64_t N = (int64_t)h->N, np = p_hi - p_lo;
+    if (np <= 0) return RISQGPU_OK;
+    PanelCount* dc = nullptr;
+    PanelBase* db = nullptr;
+    ScopedFree<2> release(dc, db);
+    RQ_TRY(dalloc(h, dc, (size_t)np));
+    RQ_TRY(dalloc(h, db, (size_t)np));
+    const int rb = h->tile_rb, cb = h->tile_cb;
+    const size_t smem_count = sizeof(int32_t) * MAX_BINS;
+    const size_t smem_scatter = sizeof(int32_t) * (MAX_BINS + ((size_t)1 << rb));
+    RQ_CUDA(h, cudaFuncSetAttribute(k_tile_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_count));
+    const int grid = (int)std::min<int64_t>(np, (int64_t)num_sms(h) * 2);
+    k_tile_count<<<grid, CT, smem_count, h->stream>>>(N, p_lo, p_hi, rb, cb, row_start, base, row_len, cols, dc,
+                                                      h->d_row_nleft);
+    RQ_TRY(check_launch(h, "tile count"));
+    std::vector<PanelCount> pc((size_t)np);
+    RQ_CUDA(h, cudaMemcpyAsync(pc.data(), dc, sizeof(PanelCount) * np, cudaMemcpyDeviceToHost, h->stream));
+    RQ_TRY(sync(h, "tile count"));
+    // a panel: its tiles' pairs, then its leftovers (their first one as `block`)
+    std::vector<PanelBase> pb((size_t)np);
+    int64_t nt = 0;
+    for (int64_t P = 0; P < np; P++) {
+        const PanelCount& c = pc[(size_t)P];
+        pb[(size_t)P] = PanelBase{stored, nt, stored + c.dense};
+        panel_tile[(size_t)(p_lo + P)] = tiles + nt;
+        stored += c.dense + c.left;
+        dense += c.dense;
+        nt += c.tiles;
+    }
+    if (stored > cap) {
+        h->err = "tiled layout: " + std::to_string(stored) + " elements exceed the " + std::to_string(cap) + " slots counted";
+        return RISQGPU_ERR_INVALID;
+    }
+    RQ_CUDA(h, cudaMemcpyAsync(db, pb.data(), sizeof(PanelBase) * np, cudaMemcpyHostToDevice, h->stream));
+    parts.push_back({nt, nullptr, nullptr, nullptr, nullptr});
+    Part& c = parts.back();
+    RQ_TRY(dalloc(h, c.win, (size_t)nt));
+    RQ_TRY(dalloc(h, c.off, (size_t)nt));
+    RQ_TRY(dalloc(h, c.len, (size_t)nt));
+    RQ_TRY(dalloc(h, c.bound, (size_t)nt));
+    auto go = [&](auto scatter, auto bounds, auto* vin, auto* val) -> int {
+        RQ_CUDA(h, cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_scatter));
+        scatter<<<grid, CT, smem_scatter, h->stream>>>(N, p_lo, p_hi, rb, cb, row_start, base, row_len, cols, vin, vlo, db, 0,
+                                                       h->d_row_nleft, c.win, nullptr, c.off, c.len, h->d_row_left,
+                                                       h->d_el_idx, val, h->d_val_lo, h->d_el_idx, val, h->d_val_lo, row_abs);
+        RQ_TRY(check_launch(h, "tile scatter"));
+        if (nt == 0) return RISQGPU_OK;
+        const size_t smem = (sizeof(uint32_t) << rb) + (sizeof(uint32_t) << cb);
+        RQ_CUDA(h, cudaFuncSetAttribute(bounds, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        bounds<<<(int)std::min<int64_t>(nt, (int64_t)num_sms(h) * 64), TT, smem, h->stream>>>(nt, rb, cb, c.off, c.len,
+                                                                                          h->d_el_idx, val, c.bound);
+        return check_launch(h, "tile bounds");
+    };
+    if (precision == RISQGPU_FP64) RQ_TRY(go(k_tile_scatter<double, false>, k_list_bounds<double, false>, v64, h->d_val64));
+    else if (precision == RISQGPU_MIXED)
+        RQ_TRY(go(k_tile_scatter<float, true>, k_list_bounds<float, true>, v32, h->d_val32));
+    else RQ_TRY(go(k_tile_scatter<float, false>, k_list_bounds<float, false>, v32, h->d_val32));
+    tiles += nt;
+    return RISQGPU_OK;
+}
+
+// The chunks' tile records in one array each, and the work space of sigma.
+int TileListBuilder::gather() {
+    const int64_t N = (int64_t)h->N, np = h->n_panels;
+    for (int64_t P = h->part_p_hi; P <= np; P++) panel_tile[(size_t)P] = tiles;
+    if (tiles >= INT32_MAX) { h->err = "too many tiles"; return RISQGPU_ERR_INVALID; }
+    h->n_tiles = tiles;
+    auto gather = [&](auto*& dst, auto Part::*src) -> int {
+        using E = typename std::remove_pointer<typename std::remove_reference<decltype(dst)>::type>::type;
+        RQ_TRY(dalloc(h, dst, (size_t)tiles));
+        int64_t at = 0;
+        for (Part& c : parts) {
+            if (c.tiles > 0)
+                RQ_CUDA(h, cudaMemcpyAsync(dst + at, c.*src, sizeof(E) * c.tiles, cudaMemcpyDeviceToDevice, h->stream));
+            at += c.tiles;
+            dfree(c.*src);
+        }
+        return RISQGPU_OK;
+    };
+    RQ_TRY(gather(h->d_tile_win, &Part::win));
+    RQ_TRY(gather(h->d_tile_off, &Part::off));
+    RQ_TRY(gather(h->d_tile_len, &Part::len));
+    RQ_TRY(gather(h->d_tile_bound, &Part::bound));
+    RQ_TRY(dalloc(h, h->d_panel_tile, (size_t)np + 1));
+    const bool f64 = precision == RISQGPU_FP64;
+    RQ_TRY(dalloc(h, h->d_acc, (size_t)(f64 ? N : N + (N + 1) / 2)));
+    RQ_TRY(dalloc(h, h->d_sig_scalars, 5));
+    return dalloc(h, h->d_wmax, (size_t)((N - 1) >> std::min(h->tile_rb, h->tile_cb)) + 1);
+}
+
+int TileListBuilder::finish() {
+    const int64_t N = (int64_t)h->N, np = h->n_panels;
+    RQ_CUDA(h, cudaMemcpyAsync(h->d_panel_tile, panel_tile.data(), sizeof(int64_t) * (np + 1), cudaMemcpyHostToDevice,
+                               h->stream));
+    RQ_CUDA(h, cudaMemsetAsync(h->d_sig_scalars, 0, sizeof(double) * 5, h->stream));
+    // row sums of |H| over both triangles: with a partition each rank holds part of every
+    // row's sum, so the exact integer sums are added across the ranks first
+    if (h->part_n > 1) RQ_TRY(part_allreduce(h, row_abs, (size_t)N));
+    k_max_u64<<<grid_n(h, N), 256, 0, h->stream>>>(row_abs, N, absmax);
+    RQ_TRY(check_launch(h, "row sums"));
+    unsigned long long mi = 0;
+    std::vector<int32_t> len((size_t)tiles), nl((size_t)N);
+    RQ_CUDA(h, cudaMemcpyAsync(&mi, absmax, sizeof(mi), cudaMemcpyDeviceToHost, h->stream));
+    RQ_CUDA(h, cudaMemcpyAsync(len.data(), h->d_tile_len, sizeof(int32_t) * tiles, cudaMemcpyDeviceToHost, h->stream));
+    RQ_CUDA(h, cudaMemcpyAsync(nl.data(), h->d_row_nleft, sizeof(int32_t) * N, cudaMemcpyDeviceToHost, h->stream));
+    RQ_TRY(sync(h, "row sums"));
+    // each |H_pq| was rounded to a multiple of 2^-32: the margin covers that rounding
+    h->h_row_abs_max = 1.01 * ((double)mi / 4294967296.0) + 1e-6;
+    h->n_dense_el = (uint64_t)dense;
+    h->tiled = h->tile_list = true;
+    // units: runs of a panel's tiles of about `target` pairs, and rows with leftovers
+    std::vector<SigmaUnit> us;
+    std::vector<int64_t> weight;
+    const int64_t R = (int64_t)1 << h->tile_rb, target = std::max<int64_t>(32768, stored / ((int64_t)num_sms(h) * 64));
+    for (int64_t P = h->part_p_lo; P < h->part_p_hi; P++) {
+        int64_t acc = 0;
+        int32_t lo = (int32_t)panel_tile[(size_t)P];
+        const int32_t end = (int32_t)panel_tile[(size_t)P + 1];
+        for (int32_t t = lo; t < end; t++) {
+            acc += len[(size_t)t];
+            if (acc < target && t + 1 < end) continue;
+            us.push_back({lo, (int32_t)P, lo, t + 1, 0});
+            weight.push_back(acc);
+            lo = t + 1;
+            acc = 0;
+        }
+        left_units(us, weight, nl, P, R, N, target);
+    }
+    return set_units(h, us, weight, target);
+}
+
+TileListBuilder::~TileListBuilder() {
+    dfree(row_abs);
+    dfree(absmax);
+    for (Part& c : parts) {
+        dfree(c.win);
+        dfree(c.off);
+        dfree(c.len);
+        dfree(c.bound);
+    }
+}
+
 TileBuilder::~TileBuilder() {
     dfree(left_cur);
     dfree(sums);
@@ -1784,12 +2009,9 @@ TileBuilder::~TileBuilder() {
 int sigma_tiles(risqgpu* h, const void* x, void* y, int kind) {
     if (kind == 0) {
         if (h->precision == RISQGPU_FP64)
-            return launch_fx<double, double, false, true>(
-                h, (const double*)x, (double*)y, tile_view<double>(h, h->d_left64, nullptr));
+            return launch_fx<double, double, false, true>(h, (const double*)x, (double*)y, h->d_left64, nullptr);
         if (h->precision == RISQGPU_MIXED)
-            return launch_fx<double, float, true, true>(
-                h, (const double*)x, (double*)y,
-                tile_view<float>(h, h->d_left32, h->d_left_lo));
+            return launch_fx<double, float, true, true>(h, (const double*)x, (double*)y, h->d_left32, h->d_left_lo);
         h->err = "FP64 sigma needs FP64 or FP32 + remainder values";
         return RISQGPU_ERR_INVALID;
     }
@@ -1797,10 +2019,9 @@ int sigma_tiles(risqgpu* h, const void* x, void* y, int kind) {
         h->err = "FP32 sigma needs FP32 values";
         return RISQGPU_ERR_INVALID;
     }
-    const TileView<float> T = tile_view<float>(h, h->d_left32, nullptr);
     if (!h->reproducible && h->part_n == 1)
-        return launch_fx<float, float, false, false>(h, (const float*)x, (float*)y, T);
-    return launch_fx<float, float, false, true>(h, (const float*)x, (float*)y, T);
+        return launch_fx<float, float, false, false>(h, (const float*)x, (float*)y, h->d_left32, nullptr);
+    return launch_fx<float, float, false, true>(h, (const float*)x, (float*)y, h->d_left32, nullptr);
 }
 
 // Every stored pair of a tiled build as (p, q, value), internal indices, in no particular
@@ -1831,6 +2052,9 @@ void free_tiles(risqgpu* h) {
     dfree(h->d_tile_win);
     dfree(h->d_tile_blk);
     dfree(h->d_tile_blocks);
+    dfree(h->d_tile_off);
+    dfree(h->d_tile_len);
+    dfree(h->d_el_idx);
     for (TileChunk& ch : h->chunks) {
         dfree(ch.grp_off);
         dfree(ch.slots);
@@ -1852,7 +2076,7 @@ void free_tiles(risqgpu* h) {
     dfree(h->d_acc);
     dfree(h->d_wmax);
     dfree(h->d_sig_scalars);
-    h->tiled = false;
+    h->tiled = h->tile_list = false;
     h->n_panels = h->n_tiles = 0;
     h->n_dense_el = 0;
     h->h_row_abs_max = 0.0;
