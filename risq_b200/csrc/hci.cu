@@ -99,6 +99,45 @@ Eps init_eps(const SelectTables& t, int n, const uint64_t* hf, double eps_var) {
 
 }  // namespace
 
+// The doubles' lists in the order of sort_double_lists, on the host.
+static void host_double_lists(const HostInts& I, int n, const std::vector<int>& vo, SelectTables& t) {
+    std::vector<Entry> v;
+    t.r.clear();
+    t.s.clear();
+    t.habs.clear();
+    t.max_opp = t.max_same = 0.0;
+    auto add = [&](double& most) {
+        stable_desc(v);
+        if (!v.empty()) most = std::fmax(most, v[0].h);
+        for (const Entry& e : v) {
+            t.r.push_back((uint8_t)e.r);
+            t.s.push_back((uint8_t)e.s);
+            t.habs.push_back(e.h);
+        }
+    };
+    // lists by p, then q; entries in the order of the valence orbitals
+    std::vector<char> is_v(n, 0);
+    for (int p : vo) is_v[p] = 1;
+    for (int k = 0; k < n * n; k++) {
+        const int p = k / n, q = k % n;
+        if (!is_v[p] || !is_v[q]) continue;
+        v.clear();
+        for (int r : vo)
+            for (int s : vo)
+                if (r != p && s != q) v.push_back({r, s, std::fabs(I.direct(p, q, r, s))});
+        add(t.max_opp);
+    }
+    for (int k = 0; k < n * n; k++) {
+        const int p = k / n, q = k % n;
+        if (p >= q || !is_v[p] || !is_v[q]) continue;
+        v.clear();
+        for (int r : vo)
+            for (int s : vo)
+                if (r < s && r != p && r != q && s != p && s != q) v.push_back({r, s, std::fabs(I.dpe(p, q, r, s))});
+        add(t.max_same);
+    }
+}
+
 int build_select_tables(risqgpu* h, int ncore, int n_up, int n_dn, SelectTables& t) {
     const int n = h->norb;
     if (ncore < 0 || ncore >= n) { h->err = "ncore must be in [0, norb)"; return RISQGPU_ERR_INVALID; }
@@ -176,7 +215,20 @@ int build_select_tables(risqgpu* h, int ncore, int n_up, int n_dn, SelectTables&
     }
     t.sing_off[n] = at + (int32_t)sr.size();
     t.entries = (size_t)at + sr.size();
-    RQ_TRY(sort_double_lists(h, t));
+    const int rc = sort_double_lists(h, t);
+    if (rc == RISQGPU_ERR_OOM) {
+        // no room to sort on the device (the sort takes twice what the lists do): on the host
+        dfree(t.d_r);
+        dfree(t.d_s);
+        dfree(t.d_habs);
+        h->err.clear();
+        host_double_lists(I, n, vo, t);
+        t.r.insert(t.r.end(), sr.begin(), sr.end());
+        t.s.resize(t.entries, 0);
+        t.habs.insert(t.habs.end(), sh.begin(), sh.end());
+        return sync(h, "excitation tables");
+    }
+    RQ_TRY(rc);
     if (!sr.empty()) {
         RQ_CUDA(h, cudaMemcpyAsync(t.d_r + at, sr.data(), sr.size(), cudaMemcpyHostToDevice, h->stream));
         RQ_CUDA(h, cudaMemsetAsync(t.d_s + at, 0, sr.size(), h->stream));
@@ -186,6 +238,7 @@ int build_select_tables(risqgpu* h, int ncore, int n_up, int n_dn, SelectTables&
 }
 
 int tables_to_host(risqgpu* h, SelectTables& t) {
+    if (!t.d_habs) return RISQGPU_OK;
     t.r.resize(t.entries);
     t.s.resize(t.entries);
     t.habs.resize(t.entries);

@@ -46,7 +46,7 @@ struct SortedSet {
     const uint64_t* __restrict__ up;
     const uint64_t* __restrict__ dn;
     int64_t N;
-    const uint64_t* __restrict__ alpha;  // unique alpha strings, ascending (one-word strings, or null)
+    const uint64_t* __restrict__ alpha;  // unique alpha strings, ascending (one-word strings), or null
     int32_t G;
     DetTable table;
     // lexicographic compare of (up, dn) with the most significant word of up first
@@ -431,6 +431,8 @@ int sort_by_cfg(risqgpu* h, const uint64_t* cfg, int64_t M, int64_t* perm, int64
     if (n <= 1) return RISQGPU_OK;
     uint64_t *k0 = nullptr, *k1 = nullptr;
     int64_t* v1 = nullptr;
+    char* tmp = nullptr;
+    ScopedFree<4> release(k0, k1, v1, tmp);
     RQ_TRY(dalloc(h, k0, n));
     RQ_TRY(dalloc(h, k1, n));
     RQ_TRY(dalloc(h, v1, n));
@@ -440,7 +442,6 @@ int sort_by_cfg(risqgpu* h, const uint64_t* cfg, int64_t M, int64_t* perm, int64
         cub::DoubleBuffer<int64_t> dv(perm, v1);
         cub::DeviceRadixSort::SortPairs(nullptr, tb, dk, dv, (int)n, 0, 64, h->stream);
     }
-    char* tmp = nullptr;
     RQ_TRY(dalloc(h, tmp, tb));
     int64_t* cur = perm;
     int64_t* alt = v1;
@@ -458,42 +459,36 @@ int sort_by_cfg(risqgpu* h, const uint64_t* cfg, int64_t M, int64_t* perm, int64
     }
     if (cur != perm) RQ_CUDA(h, cudaMemcpyAsync(perm, cur, sizeof(int64_t) * n, cudaMemcpyDeviceToDevice, h->stream));
     RQ_TRY(check_launch(h, "sort_by_cfg"));
-    RQ_TRY(sync(h, "sort_by_cfg"));
-    dfree(k0); dfree(k1); dfree(v1); dfree(tmp);
-    return RISQGPU_OK;
+    return sync(h, "sort_by_cfg");
 }
 
 // Select flagged elements of `in` (keeping order) into `out`; returns the count.
 int compact_i64(risqgpu* h, const int64_t* in, const int32_t* flags, int64_t n, int64_t* out, int64_t& nout) {
     int64_t* dn = nullptr;
+    char* tmp = nullptr;
+    ScopedFree<2> release(dn, tmp);
     RQ_TRY(dalloc(h, dn, 1));
     size_t tb = 0;
     cub::DeviceSelect::Flagged(nullptr, tb, in, flags, out, dn, (int)n, h->stream);
-    char* tmp = nullptr;
     RQ_TRY(dalloc(h, tmp, tb));
     cub::DeviceSelect::Flagged(tmp, tb, in, flags, out, dn, (int)n, h->stream);
     RQ_CUDA(h, cudaMemcpyAsync(&nout, dn, sizeof(int64_t), cudaMemcpyDeviceToHost, h->stream));
-    RQ_TRY(sync(h, "compact"));
-    dfree(tmp);
-    dfree(dn);
-    return RISQGPU_OK;
+    return sync(h, "compact");
 }
 
 int sort_i64(risqgpu* h, int64_t* keys, int64_t n) {
     if (n <= 1) return RISQGPU_OK;
     int64_t* alt = nullptr;
+    char* tmp = nullptr;
+    ScopedFree<2> release(alt, tmp);
     RQ_TRY(dalloc(h, alt, n));
     size_t tb = 0;
     cub::DoubleBuffer<int64_t> dk(keys, alt);
     cub::DeviceRadixSort::SortKeys(nullptr, tb, dk, (int)n, 0, 64, h->stream);
-    char* tmp = nullptr;
     RQ_TRY(dalloc(h, tmp, tb));
     cub::DeviceRadixSort::SortKeys(tmp, tb, dk, (int)n, 0, 64, h->stream);
     if (dk.Current() != keys) RQ_CUDA(h, cudaMemcpyAsync(keys, dk.Current(), sizeof(int64_t) * n, cudaMemcpyDeviceToDevice, h->stream));
-    RQ_TRY(sync(h, "sort_i64"));
-    dfree(alt);
-    dfree(tmp);
-    return RISQGPU_OK;
+    return sync(h, "sort_i64");
 }
 
 // Unique by configuration keeping the smallest index: `idx` (n entries, values
@@ -504,6 +499,7 @@ int unique_first(risqgpu* h, const uint64_t* cfg, int64_t M, int64_t* idx, int64
     RQ_TRY(sort_by_cfg<W>(h, cfg, M, idx, n));
     int32_t* head = nullptr;
     int64_t* out = nullptr;
+    ScopedFree<2> release(head, out);
     RQ_TRY(dalloc(h, head, n));
     RQ_TRY(dalloc(h, out, n));
     k_heads<W><<<grid_of(h, n), 256, 0, h->stream>>>(cfg, M, idx, n, head);
@@ -511,10 +507,7 @@ int unique_first(risqgpu* h, const uint64_t* cfg, int64_t M, int64_t* idx, int64
     RQ_TRY(compact_i64(h, idx, head, n, out, nk));
     RQ_TRY(sort_i64(h, out, nk));
     RQ_CUDA(h, cudaMemcpyAsync(idx, out, sizeof(int64_t) * nk, cudaMemcpyDeviceToDevice, h->stream));
-    RQ_TRY(sync(h, "unique"));
-    dfree(head);
-    dfree(out);
-    return RISQGPU_OK;
+    return sync(h, "unique");
 }
 
 __global__ void k_gather_out(const int64_t* __restrict__ idx, int64_t K, const uint64_t* __restrict__ cfg, int64_t L,
@@ -532,13 +525,14 @@ __global__ void k_gather_out(const int64_t* __restrict__ idx, int64_t K, const u
 
 template <int W>
 int find_new_impl(risqgpu* h, const double* coeffs, double eps, bool singles, const SelectTables& tab,
-                  std::vector<uint64_t>& new_dets, std::vector<double>& new_diag, SelectStats* st) {
+                  std::vector<uint64_t>& new_dets, std::vector<double>& new_diag, SelectStats* st, bool groups) {
     const int64_t N = (int64_t)h->N;
     new_dets.clear();
     new_diag.clear();
     // caller-order determinants, coefficients and diagonals on the device
     uint64_t* aos = nullptr;
     double *cf = nullptr, *dgc = nullptr;
+    ScopedFree<3> release(aos, cf, dgc);
     RQ_TRY(dalloc(h, aos, 4 * N));
     RQ_TRY(dalloc(h, cf, N));
     RQ_TRY(dalloc(h, dgc, N));
@@ -570,8 +564,6 @@ int find_new_impl(risqgpu* h, const double* coeffs, double eps, bool singles, co
     Bits<W> val;
     for (int q = 0; q < W; q++) val.w[q] = tab.valence[q];
     Ints I{h->d_h1, h->d_h2, h->nuc};
-    // a refused set has no groups, and its determinants may hold more electrons than n_up
-    const bool groups = W == 1 && h->grouped;
     if (groups) {
         RQ_TRY(dalloc(h, alpha, (size_t)h->G_a));
         k_unique_alpha<<<grid_of(h, h->G_a), 256, 0, h->stream>>>(h->d_up, h->d_ga_start, h->G_a, alpha);
@@ -586,6 +578,7 @@ int find_new_impl(risqgpu* h, const double* coeffs, double eps, bool singles, co
     RQ_CUDA(h, cudaFuncSetAttribute(k_expand<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     int* counter = nullptr;
     int64_t *cnt = nullptr, *off = nullptr;
+    ScopedFree<3> release_counts(counter, cnt, off);
     RQ_TRY(dalloc(h, counter, 1));
     RQ_TRY(dalloc(h, cnt, N + 1));
     RQ_TRY(dalloc(h, off, N + 1));
@@ -601,10 +594,10 @@ int find_new_impl(risqgpu* h, const double* coeffs, double eps, bool singles, co
         size_t tb = 0;
         cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, off, (int)(N + 1), h->stream);
         char* tmp = nullptr;
+        ScopedFree<1> release_tmp(tmp);
         RQ_TRY(dalloc(h, tmp, tb));
         cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, off, (int)(N + 1), h->stream);
         RQ_TRY(sync(h, "expand scan"));
-        dfree(tmp);
     }
     int64_t M = 0;
     RQ_CUDA(h, cudaMemcpy(&M, off + N, sizeof(int64_t), cudaMemcpyDeviceToHost));
@@ -613,6 +606,12 @@ int find_new_impl(risqgpu* h, const double* coeffs, double eps, bool singles, co
         uint64_t* cfg = nullptr;
         int32_t* parent = nullptr;
         uint32_t* code = nullptr;
+        int64_t* idx = nullptr;
+        uint64_t *pcfg = nullptr, *outd = nullptr;
+        double *pdg = nullptr, *outg = nullptr;
+        int32_t* keep = nullptr;
+        int64_t *lidx = nullptr, *lkeep = nullptr;
+        ScopedFree<11> release_cand(cfg, parent, code, idx, pcfg, pdg, keep, lidx, lkeep, outd, outg);
         RQ_TRY(dalloc(h, cfg, (size_t)2 * W * M));
         RQ_TRY(dalloc(h, parent, M));
         RQ_TRY(dalloc(h, code, M));
@@ -621,23 +620,18 @@ int find_new_impl(risqgpu* h, const double* coeffs, double eps, bool singles, co
                                                          nullptr, off, cfg, parent, code, M, cache);
         RQ_TRY(check_launch(h, "expand fill"));
         // first occurrence of each configuration
-        int64_t* idx = nullptr;
         RQ_TRY(dalloc(h, idx, M));
         k_iota64<<<grid_of(h, M), 256, 0, h->stream>>>(idx, M);
         int64_t K = 0;
         RQ_TRY(unique_first<W>(h, cfg, M, idx, M, K));
         // diagonals and [flip(d), d] pairs
         const int64_t L = 2 * K;
-        uint64_t* pcfg = nullptr;
-        double* pdg = nullptr;
         RQ_TRY(dalloc(h, pcfg, (size_t)2 * W * L));
         RQ_TRY(dalloc(h, pdg, L));
         k_finish<W><<<grid_of(h, K), 256, 0, h->stream>>>(idx, K, cfg, M, parent, code, aos, dgc, I, pcfg, pdg);
         RQ_TRY(check_launch(h, "finish"));
         dfree(cfg); dfree(parent); dfree(code); dfree(idx);
         // drop flips already in the space, then first occurrence again
-        int32_t* keep = nullptr;
-        int64_t *lidx = nullptr, *lkeep = nullptr;
         RQ_TRY(dalloc(h, keep, L));
         RQ_TRY(dalloc(h, lidx, L));
         RQ_TRY(dalloc(h, lkeep, L));
@@ -647,8 +641,6 @@ int find_new_impl(risqgpu* h, const double* coeffs, double eps, bool singles, co
         RQ_TRY(compact_i64(h, lidx, keep, L, lkeep, L2));
         int64_t F = 0;
         RQ_TRY(unique_first<W>(h, pcfg, L, lkeep, L2, F));
-        uint64_t* outd = nullptr;
-        double* outg = nullptr;
         RQ_TRY(dalloc(h, outd, 4 * std::max<int64_t>(F, 1)));
         RQ_TRY(dalloc(h, outg, std::max<int64_t>(F, 1)));
         k_gather_out<<<grid_of(h, std::max<int64_t>(F, 1)), 256, 0, h->stream>>>(lkeep, F, pcfg, L, pdg, W, outd, outg);
@@ -659,12 +651,9 @@ int find_new_impl(risqgpu* h, const double* coeffs, double eps, bool singles, co
         RQ_CUDA(h, cudaMemcpyAsync(new_diag.data(), outg, sizeof(double) * F, cudaMemcpyDeviceToHost, h->stream));
         RQ_TRY(sync(h, "select out"));
         if (st) { st->unique = (uint64_t)K; st->added = (uint64_t)F; }
-        dfree(pcfg); dfree(pdg); dfree(keep); dfree(lidx); dfree(lkeep); dfree(outd); dfree(outg);
     } else if (st) {
         st->unique = st->added = 0;
     }
-    dfree(aos); dfree(cf); dfree(dgc);
-    dfree(counter); dfree(cnt); dfree(off);
     return RISQGPU_OK;
 }
 
@@ -793,8 +782,16 @@ int sort_double_lists(risqgpu* h, SelectTables& t) {
 int find_new_dets_impl(risqgpu* h, const double* coeffs, double eps, bool singles, const SelectTables& tab,
                        std::vector<uint64_t>& new_dets, std::vector<double>& new_diag, SelectStats* st) {
     if (h->N == 0 || !h->d_diag) { h->err = "no determinants set"; return RISQGPU_ERR_INVALID; }
-    return h->W == 1 ? find_new_impl<1>(h, coeffs, eps, singles, tab, new_dets, new_diag, st)
-                     : find_new_impl<2>(h, coeffs, eps, singles, tab, new_dets, new_diag, st);
+    if (h->W != 1) return find_new_impl<2>(h, coeffs, eps, singles, tab, new_dets, new_diag, st, false);
+    // a refused set has no groups, and its determinants may hold more electrons than n_up
+    int rc = RISQGPU_ERR_OOM;
+    if (h->grouped) rc = find_new_impl<1>(h, coeffs, eps, singles, tab, new_dets, new_diag, st, true);
+    // without room for the group strings: the general search
+    if (rc == RISQGPU_ERR_OOM) {
+        h->err.clear();
+        rc = find_new_impl<1>(h, coeffs, eps, singles, tab, new_dets, new_diag, st, false);
+    }
+    return rc;
 }
 
 }  // namespace risq
