@@ -1282,7 +1282,7 @@ template <int W>
 int build_upper(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int precision, int* counter, int threads,
                 cudaEvent_t* ev, std::chrono::steady_clock::time_point& t1, int64_t& cap, int64_t& nnz) {
     ScopedFree<1> release(h->d_agree);
-    if (h->part_n > 1) RQ_TRY(dalloc(h, h->d_agree, 1));
+    if (h->part_n > 1) RQ_TRY(dalloc_reduced(h, h->d_agree, 1));
     auto counted = [&]() -> int {
         RQ_TRY((count_candidates<W, OUT_UPPER>(h, v, I, thr, counter, threads, ev, cap)));
         t1 = std::chrono::steady_clock::now();

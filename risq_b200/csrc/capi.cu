@@ -18,7 +18,7 @@ namespace {
 // their power of two, so that one set's matrix fits the blocks another one left; a pool that
 // cuts small buffers, or the first of two large ones, from a freed matrix's hole has to map
 // new memory for the rest (131,611 determinants, three handles in turn: 13 ms a build,
-// against 8 here).  Those of handles with a memory bound: the device.
+// against 8 here).  Those of handles with a memory bound, and what ranks reduce: the device.
 enum Source { FROM_DEVICE, FROM_POOL, FROM_BLOCKS };
 constexpr size_t POOL_LARGE = (size_t)64 << 20;
 
@@ -152,7 +152,7 @@ void drop_parked(risqgpu* h, bool reuse) {
     h->parked.clear();
 }
 
-int mem_alloc(risqgpu* h, void** p, size_t bytes) {
+int mem_alloc(risqgpu* h, void** p, size_t bytes, bool device) {
     *p = nullptr;
     if (h->mem_limit && h->mem_used + bytes > h->mem_limit) {
         h->err = "allocation of " + std::to_string(bytes) + " bytes exceeds the handle's device memory limit (" +
@@ -161,7 +161,7 @@ int mem_alloc(risqgpu* h, void** p, size_t bytes) {
     }
     Buffer b{h, bytes, FROM_DEVICE, bytes};
     cudaMemPool_t small = nullptr;
-    if (!h->mem_limit) {
+    if (!h->mem_limit && !device) {
         b.source = bytes < POOL_LARGE ? FROM_POOL : FROM_BLOCKS;
         if (b.source == FROM_BLOCKS) {
             // the smallest block that fits: of the handle's previous matrix, then of the idle ones

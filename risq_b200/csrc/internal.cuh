@@ -232,7 +232,7 @@ struct DeviceGuard {
 // handle (`parked`) until that build returns: unmapping and mapping them again took from 0.1
 // to 2.5 s for 120 GB on a host whose GPUs are shared.
 constexpr size_t POOL_KEEP = (size_t)6 << 30, SMALL_KEEP = (size_t)2 << 30;
-int mem_alloc(risqgpu* h, void** p, size_t bytes);  // RISQGPU status; sets h->err
+int mem_alloc(risqgpu* h, void** p, size_t bytes, bool device = false);  // RISQGPU status; sets h->err
 void mem_free(void* p);
 void drop_parked(risqgpu* h, bool reuse);  // to the idle blocks, or to the device
 int pool_acquire(int device);  // one call per handle made on the device
@@ -260,6 +260,15 @@ inline int dalloc(risqgpu* h, T*& p, size_t count) {
     dfree(p);
     if (count == 0) count = 1;
     return mem_alloc(h, (void**)&p, count * sizeof(T));
+}
+
+// A buffer that the ranks' reduce function is given: with a partition from cudaMalloc, since a
+// caller's own all-reduce may open it in another process or reach it from another GPU, which
+// memory of a private pool does not allow.
+template <typename T>
+inline int dalloc_reduced(risqgpu* h, T*& p, size_t count) {
+    dfree(p);
+    return mem_alloc(h, (void**)&p, (count ? count : 1) * sizeof(T), h->part_n > 1);
 }
 
 // Device bytes that new allocations may take: free device memory and what is kept idle or

@@ -1487,11 +1487,11 @@ int TileBuilder::begin(int64_t p_lo, int64_t p_hi, int precision, const uint32_t
     RQ_TRY(dalloc(h, h->d_left_row, (size_t)left));
     RQ_TRY(dalloc(h, h->d_left32, (size_t)left));
     if (lo) RQ_TRY(dalloc(h, h->d_left_lo, (size_t)left));
-    RQ_TRY(dalloc(h, h->d_acc, (size_t)(N + (N + 1) / 2)));
+    RQ_TRY(dalloc_reduced(h, h->d_acc, (size_t)(N + (N + 1) / 2)));
     RQ_TRY(dalloc(h, h->d_sig_scalars, 5));
     RQ_TRY(dalloc(h, h->d_wmax, (size_t)((N - 1) >> std::min(h->tile_rb, h->tile_cb)) + 1));
     RQ_TRY(dalloc(h, left_cur, (size_t)np));
-    RQ_TRY(dalloc(h, sums, (size_t)(np + ((N - 1) >> h->tile_cb) + 1)));
+    RQ_TRY(dalloc_reduced(h, sums, (size_t)(np + ((N - 1) >> h->tile_cb) + 1)));
     RQ_TRY(dalloc(h, counters, 5));
     RQ_CUDA(h, cudaMemsetAsync(h->d_sig_scalars, 0, sizeof(double) * 5, h->stream));
     RQ_CUDA(h, cudaMemsetAsync(h->d_left_len, 0, sizeof(int32_t) * np, h->stream));
@@ -1673,7 +1673,7 @@ int Tiles64Builder::begin(risqgpu* h_) {
     panel_tile.assign((size_t)h->n_panels + 1, 0);
     RQ_TRY(dalloc(h, h->d_row_left, (size_t)N));
     RQ_TRY(dalloc(h, h->d_row_nleft, (size_t)N));
-    RQ_TRY(dalloc(h, row_abs, (size_t)N));
+    RQ_TRY(dalloc_reduced(h, row_abs, (size_t)N));
     RQ_TRY(dalloc(h, absmax, 1));
     RQ_TRY(dalloc(h, counters, 4));
     RQ_CUDA(h, cudaMemsetAsync(h->d_row_nleft, 0, sizeof(int32_t) * N, h->stream));
@@ -1795,7 +1795,7 @@ int Tiles64Builder::finish() {
     if (tiles > 0)
         RQ_CUDA(h, cudaMemcpyAsync(tb.data(), h->d_tile_blocks, sizeof(TileBlock) * tiles, cudaMemcpyDeviceToHost, h->stream));
     RQ_CUDA(h, cudaMemcpyAsync(nl.data(), h->d_row_nleft, sizeof(int32_t) * N, cudaMemcpyDeviceToHost, h->stream));
-    RQ_TRY(dalloc(h, h->d_acc, (size_t)N));
+    RQ_TRY(dalloc_reduced(h, h->d_acc, (size_t)N));
     RQ_TRY(dalloc(h, h->d_sig_scalars, 5));
     RQ_TRY(dalloc(h, h->d_wmax, (size_t)((N - 1) >> std::min(h->tile_rb, h->tile_cb)) + 1));
     RQ_CUDA(h, cudaMemsetAsync(h->d_sig_scalars, 0, sizeof(double) * 5, h->stream));
@@ -1841,7 +1841,7 @@ int TileListBuilder::begin(risqgpu* h_, int precision_, int64_t cap_) {
     panel_tile.assign((size_t)h->n_panels + 1, 0);
     RQ_TRY(dalloc(h, h->d_row_left, (size_t)N));
     RQ_TRY(dalloc(h, h->d_row_nleft, (size_t)N));
-    RQ_TRY(dalloc(h, row_abs, (size_t)N));
+    RQ_TRY(dalloc_reduced(h, row_abs, (size_t)N));
     RQ_TRY(dalloc(h, absmax, 1));
     RQ_TRY(dalloc(h, h->d_el_idx, (size_t)cap));
     if (precision == RISQGPU_FP64) RQ_TRY(dalloc(h, h->d_val64, (size_t)cap));
@@ -1940,7 +1940,7 @@ int TileListBuilder::gather() {
     RQ_TRY(gather(h->d_tile_bound, &Part::bound));
     RQ_TRY(dalloc(h, h->d_panel_tile, (size_t)np + 1));
     const bool f64 = precision == RISQGPU_FP64;
-    RQ_TRY(dalloc(h, h->d_acc, (size_t)(f64 ? N : N + (N + 1) / 2)));
+    RQ_TRY(dalloc_reduced(h, h->d_acc, (size_t)(f64 ? N : N + (N + 1) / 2)));
     RQ_TRY(dalloc(h, h->d_sig_scalars, 5));
     return dalloc(h, h->d_wmax, (size_t)((N - 1) >> std::min(h->tile_rb, h->tile_cb)) + 1);
 }
