@@ -305,6 +305,26 @@ struct ScopedFree {
     ScopedFree& operator=(const ScopedFree&) = delete;
 };
 
+// Lets a kernel take `bytes` of dynamic shared memory.  The permission belongs to the kernel, in
+// the whole process: it is always the device's most, so that a thread with a smaller set does
+// not take it from another between that one's call and its launch.
+template <typename K>
+inline int allow_smem(risqgpu* h, K kern, size_t bytes) {
+    if (bytes <= ((size_t)40 << 10)) return RISQGPU_OK;  // needs none (48 KB with the static part)
+    cudaFuncAttributes a;
+    int most = 0;
+    cudaError_t e = cudaFuncGetAttributes(&a, kern);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&most, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, most - (int)a.sharedSizeBytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        h->err = std::string("shared memory of a kernel: ") + cudaGetErrorString(e);
+        return RISQGPU_ERR_CUDA;
+    }
+    return RISQGPU_OK;
+}
+
 inline int check_launch(risqgpu* h, const char* what) {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {

@@ -574,8 +574,8 @@ int find_new_impl(risqgpu* h, const double* coeffs, double eps, bool singles, co
     int cache = groups ? h->n_up * h->norb : 0;
     if ((size_t)cache * 8 * sizeof(int32_t) > ((size_t)64 << 10)) cache = 0;
     const size_t smem = (size_t)cache * 8 * sizeof(int32_t);
-    RQ_CUDA(h, cudaFuncSetAttribute(k_expand<W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    RQ_CUDA(h, cudaFuncSetAttribute(k_expand<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    RQ_TRY((allow_smem(h, k_expand<W, false>, smem)));
+    RQ_TRY((allow_smem(h, k_expand<W, true>, smem)));
     int* counter = nullptr;
     int64_t *cnt = nullptr, *off = nullptr;
     ScopedFree<3> release_counts(counter, cnt, off);

@@ -164,7 +164,7 @@ int launch_otf(risqgpu* h, const double* x, double* y) {
     int max_smem = 0;
     cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, h->device);
     if (smem <= (size_t)max_smem) {
-        RQ_CUDA(h, cudaFuncSetAttribute(k_spmv_otf<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        RQ_TRY((allow_smem(h, k_spmv_otf<W, true>, smem)));
         k_spmv_otf<W, true><<<num_sms(h), 1024, smem, h->stream>>>(n, h->d_up, h->d_dn, h->d_row_start, h->d_row_len,
                                                                    h->d_cols, h->d_diag, I, (uint32_t)h->n1,
                                                                    (uint32_t)h->n2, x, y, h->stop_flag);

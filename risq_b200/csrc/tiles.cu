@@ -1287,7 +1287,7 @@ template <typename X, typename V, bool EXACT, typename K, typename T_>
 int launch_sigma(risqgpu* h, const X* x, X* y, K kern, size_t smem, const T_& T) {
     using Y = typename std::conditional<EXACT, long long, X>::type;
     const int64_t N = (int64_t)h->N;
-    RQ_CUDA(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    RQ_TRY(allow_smem(h, kern, smem));
     int occ = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, ST, smem);
     // FP32 sums: N columns, then the rows' in fixed point
@@ -1530,12 +1530,12 @@ int arrange_bins(risqgpu* h, TileBlock* blocks, int64_t k_lo, int64_t k_hi, int6
     RQ_TRY(dalloc(h, row_cnt, (size_t)nb * B));
     auto grid_of = [&](auto kern, size_t smem) {
         int occ = 0;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, AT, smem);
         return (int)std::min<int64_t>(nb, (int64_t)num_sms(h) * std::max(occ, 1));
     };
     RQ_CUDA(h, cudaMemsetAsync(counters, 0, sizeof(unsigned long long) * 3, h->stream));
     const size_t smem1 = sizeof(int) * (size_t)(3 * B + B / 32 + 4);
+    RQ_TRY(allow_smem(h, k_tile_size, smem1));
     k_tile_size<<<grid_of(k_tile_size, smem1), AT, smem1, h->stream>>>(k_lo, k_hi, h->tile_rb, h->tile_cb, h->tile_kb, el0,
                                                                        blocks, cur, code, row_cnt, counters);
     RQ_TRY(check_launch(h, "tile sizes"));
@@ -1557,6 +1557,7 @@ int arrange_bins(risqgpu* h, TileBlock* blocks, int64_t k_lo, int64_t k_hi, int6
     const int cap = (int)((((size_t)110 << 10) - std::min(fixed, (size_t)100 << 10)) / per) & ~63;
     const size_t smem = fixed + (size_t)cap * per;
     auto go = [&](auto kern) -> int {
+        RQ_TRY(allow_smem(h, kern, smem));
         kern<<<grid_of(kern, smem), AT, smem, h->stream>>>(k_lo, k_hi, h->tile_rb, h->tile_cb, h->tile_kb, el0, blocks,
                                                            code, vin, lin, row_cnt, cap, counters, ch.slots, ch.grp_off,
                                                            ch.col, val, ch.lo);
@@ -1583,7 +1584,7 @@ int TileBuilder::chunk(int64_t p_lo, int64_t p_hi, int64_t chunk_el0, const unsi
         const int64_t nt = z.tile - a.tile;
         const size_t smem = sizeof(uint32_t) << h->tile_cb;
         auto go = [&](auto kern) -> int {
-            RQ_CUDA(h, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            RQ_TRY(allow_smem(h, kern, smem));
             kern<<<(int)std::min<int64_t>(nt, (int64_t)num_sms(h) * 64), TT, smem, h->stream>>>(
                 a.tile, z.tile, z.block, h->tile_rb, h->tile_cb, h->n_panels, id, chunk_el0, h->d_tile_blocks, h->d_tile_blk,
                 h->d_tile_win, code, vin, h->d_tile_bound, sums, counters + 3);
@@ -1695,9 +1696,8 @@ int Tiles64Builder::chunk(int64_t p_lo, int64_t p_hi, const int64_t* row_start, 
     const int rb = h->tile_rb, cb = h->tile_cb;
     const size_t smem_count = sizeof(int32_t) * MAX_BINS;
     const size_t smem_scatter = sizeof(int32_t) * (MAX_BINS + ((size_t)1 << rb));
-    RQ_CUDA(h, cudaFuncSetAttribute(k_tile_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_count));
-    RQ_CUDA(h, cudaFuncSetAttribute(k_tile_scatter<double, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)smem_scatter));
+    RQ_TRY(allow_smem(h, k_tile_count, smem_count));
+    RQ_TRY((allow_smem(h, k_tile_scatter<double, false>, smem_scatter)));
     const int grid = (int)std::min<int64_t>(np, (int64_t)num_sms(h) * 2);
     k_tile_count<<<grid, CT, smem_count, h->stream>>>(N, p_lo, p_hi, rb, cb, row_start, base, row_len, cols, dc,
                                                       h->d_row_nleft);
@@ -1865,7 +1865,7 @@ int TileListBuilder::chunk(int64_t p_lo, int64_t p_hi, const int64_t* row_start,
     const int rb = h->tile_rb, cb = h->tile_cb;
     const size_t smem_count = sizeof(int32_t) * MAX_BINS;
     const size_t smem_scatter = sizeof(int32_t) * (MAX_BINS + ((size_t)1 << rb));
-    RQ_CUDA(h, cudaFuncSetAttribute(k_tile_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_count));
+    RQ_TRY(allow_smem(h, k_tile_count, smem_count));
     const int grid = (int)std::min<int64_t>(np, (int64_t)num_sms(h) * 2);
     k_tile_count<<<grid, CT, smem_count, h->stream>>>(N, p_lo, p_hi, rb, cb, row_start, base, row_len, cols, dc,
                                                       h->d_row_nleft);
@@ -1896,14 +1896,14 @@ int TileListBuilder::chunk(int64_t p_lo, int64_t p_hi, const int64_t* row_start,
     RQ_TRY(dalloc(h, c.len, (size_t)nt));
     RQ_TRY(dalloc(h, c.bound, (size_t)nt));
     auto go = [&](auto scatter, auto bounds, auto* vin, auto* val) -> int {
-        RQ_CUDA(h, cudaFuncSetAttribute(scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_scatter));
+        RQ_TRY(allow_smem(h, scatter, smem_scatter));
         scatter<<<grid, CT, smem_scatter, h->stream>>>(N, p_lo, p_hi, rb, cb, row_start, base, row_len, cols, vin, vlo, db, 0,
                                                        h->d_row_nleft, c.win, nullptr, c.off, c.len, h->d_row_left,
                                                        h->d_el_idx, val, h->d_val_lo, h->d_el_idx, val, h->d_val_lo, row_abs);
         RQ_TRY(check_launch(h, "tile scatter"));
         if (nt == 0) return RISQGPU_OK;
         const size_t smem = (sizeof(uint32_t) << rb) + (sizeof(uint32_t) << cb);
-        RQ_CUDA(h, cudaFuncSetAttribute(bounds, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        RQ_TRY(allow_smem(h, bounds, smem));
         bounds<<<(int)std::min<int64_t>(nt, (int64_t)num_sms(h) * 64), TT, smem, h->stream>>>(nt, rb, cb, c.off, c.len,
                                                                                           h->d_el_idx, val, c.bound);
         return check_launch(h, "tile bounds");
