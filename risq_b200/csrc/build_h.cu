@@ -375,17 +375,22 @@ __global__ void __launch_bounds__(256) k_build_rows(SetView<W> v, Ints I, double
                 pos = __shfl_sync(FULL, pos, leader) + __popc(grp & lt);
                 if (ok) {
                     const float hi = (float)val;
+                    // (within the arrays always: the search has counted every element)
                     if (pos & LEFT_BIN) {
                         const int64_t at = (int64_t)(pos & ~LEFT_BIN);
-                        T.lcol[at] = (uint32_t)q;
-                        T.lrow[at] = (uint16_t)(code0 >> T.cb);
-                        T.l32[at] = hi;
-                        if (MODE == 3) T.llo[at] = (float)(val - (double)hi);
+                        if (at < T.left_cap) {
+                            T.lcol[at] = (uint32_t)q;
+                            T.lrow[at] = (uint16_t)(code0 >> T.cb);
+                            T.l32[at] = hi;
+                            if (MODE == 3) T.llo[at] = (float)(val - (double)hi);
+                        }
                     } else {
                         const int64_t at = (int64_t)pos - T.el0;
-                        T.code[at] = code0 | ((uint32_t)q & ((1u << T.cb) - 1u));
-                        v32[at] = hi;
-                        if (MODE == 3) vlo[at] = (float)(val - (double)hi);
+                        if (at < T.cap) {
+                            T.code[at] = code0 | ((uint32_t)q & ((1u << T.cb) - 1u));
+                            v32[at] = hi;
+                            if (MODE == 3) vlo[at] = (float)(val - (double)hi);
+                        }
                     }
                 }
             } else {
@@ -1258,6 +1263,8 @@ int build_tiled(risqgpu* h, const SetView<W>& v, const Ints& I, double thr, int 
     if (precision == RISQGPU_MIXED) RQ_TRY(dalloc(h, clo, (size_t)max_chunk));
     T.cur = cur;
     T.left_cur = tb.left_cur;
+    T.cap = max_chunk;
+    T.left_cap = tb.left;
     T.code = code;
     T.lcol = h->d_left_col;
     T.lrow = h->d_left_row;

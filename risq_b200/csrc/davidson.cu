@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(DBLK) k_ritz(const T* __restrict__ V, const T*
 // blocks to finish, which puts what the host needs into page-locked memory.  The first
 // kernel also decides whether the solve ends there; the ones after it then do nothing.
 // Every sum is formed in the order of the kernels above (same grid, same tree).
-// Measured: 6,943 determinants 100 -> 38 us an iteration besides sigma.
+// Measured: 6,943 determinants 100 -> 50 us an iteration besides sigma.
 
 // Slots of the results, in device and in page-locked memory.
 enum Slot : int { S_RES2 = 0, S_T2 = 1, S_NORM2 = 2, S_STOP = 3, S_COL = 4 };

@@ -397,6 +397,7 @@ struct TileBuilder {
     unsigned long long* sums = nullptr;             // row bounds per panel, column bounds per window
     unsigned long long* counters = nullptr;
     std::vector<int32_t> panel_chunk;
+    int64_t left = 0;                               // leftovers there is room for
     int64_t stored = 0;                             // pairs, after finish
     int plan(risqgpu* h, const uint32_t* hist, const int64_t* bin_off, int64_t n_blocks);
     int begin(int64_t p_lo, int64_t p_hi, int precision, const uint32_t* hist, const int64_t* bin_off,

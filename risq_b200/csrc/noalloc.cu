@@ -1,12 +1,12 @@
 // sigma without any device allocation in the call.
 //
-// risqgpu_sigma stages the caller's vector through cudaMalloc'd buffers: the
+// risqgpu_sigma stages the caller's vector through device buffers that it allocates: the
 // caller-order x is permuted into the library's internal (sorted) order, H is
 // applied, and the result is permuted back.  Some callers cannot have a library
 // allocate device memory on their behalf: a host code whose own pool allocator
 // owns the device memory budget, or a solver loop that overlaps work on several
-// streams and cannot afford the device-wide synchronisation that cudaFree
-// implies on every Davidson iteration.  risqgpu_sigma_noalloc does the same work
+// streams and cannot afford the device-wide synchronisation of the allocation calls
+// that the library makes when no kept memory fits.  risqgpu_sigma_noalloc does the same work
 // with both permuted vectors held in one file-scope device array of fixed size,
 // so the call itself allocates nothing: the caller passes device pointers for x
 // and y, and the matrix was allocated earlier, by risqgpu_build_h.

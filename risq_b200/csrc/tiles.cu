@@ -1459,7 +1459,7 @@ int TileBuilder::begin(int64_t p_lo, int64_t p_hi, int precision, const uint32_t
     base.assign((size_t)np + 1, PanelBase{0, 0, 0});
     panel_chunk.assign((size_t)np, 0);
     std::vector<int64_t> loff((size_t)np, 0), pt((size_t)np + 1, 0);
-    int64_t left = 0;
+    left = 0;
     PanelBase b{0, 0, 0};
     for (int64_t P = 0; P <= np; P++) {
         base[(size_t)P] = b;

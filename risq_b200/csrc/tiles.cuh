@@ -55,6 +55,7 @@ struct TileOut {
     unsigned long long* cur = nullptr;       // fill: next element of every bin
     unsigned long long* left_cur = nullptr;  // fill: next leftover of every panel
     long long el0 = 0;                       // first element of the chunk being filled
+    long long cap = 0, left_cap = 0;         // elements its arrays and the leftovers' hold
     uint32_t* code = nullptr;                // fill: row in panel << cb | column in window
     uint32_t* lcol = nullptr;                // leftovers: column, row in panel, values
     uint16_t* lrow = nullptr;
