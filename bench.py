@@ -61,7 +61,7 @@ DAV_MAX_ITER = 2000  # the reference's cap of 50 does not converge on these inte
 # kernel on the n20 eps 1e-3 set (profiles/k_sigma_fx_fp32_n20_eps1e-3.md); the
 # element stream is the traffic and grows with the stored pairs, so a launch over
 # another set is scaled by its pairs
-SIGMA32_CAPTURE = {"pairs": 334_413_323, "dram_bytes": 2_696_127_488 + 11_001_088,
+SIGMA32_CAPTURE = {"pairs": 334_413_323, "dram_bytes": 2_469_325_568 + 5_799_424,
                    "set": "n20 8a8b eps_var 1e-3 seed 0 (551,147 dets)"}
 # The CPU legs time the variational space of the last HCI iteration whose set holds at
 # most this many determinants (the whole set when it is smaller).
@@ -77,7 +77,7 @@ THICK_SPACE = (32, 8)
 THICK_MIN_DETS = 1_000_000
 # From this size both paths store the upper triangle in tiles even where both
 # triangles would fit: the tiled sigma is the faster one there (n20 eps 1e-3, 551,147
-# dets: FP32 0.88 ms against 1.43 ms for both triangles; n24 HCI iteration 4,
+# dets: FP32 0.64 ms against 1.43 ms for both triangles; n24 HCI iteration 4,
 # 5,042,871 dets: FP64 27.4 ms against 38.2 ms) and holds half the bytes.
 UPPER_MIN_DETS = 500_000
 
@@ -486,21 +486,19 @@ def main():
         return ms_s / R
 
     t_sig = time_sigma(x, y, 0)
-    tiles64 = int(hs64.get("n_tiles", 0))
 
-    # algorithmic bytes of one sigma: values + int32 column / element index of every stored
-    # element, per row its start and length (12 B), x and the diagonal read once, y written
-    # once; tiled upper storage also reads 16 B per tile header (20 B for the FP32 sigma,
-    # which reads each tile's bound); the recomputing kernel reads both strings of every
-    # determinant once (N * 16 B)
-    def sigma_bytes(prec, s_v, s_x, n_tiles):
+    # algorithmic bytes of one sigma: value + int32 column of every stored element, per row its
+    # start and length (12 B), x and the diagonal read once, y written once; tiles hold columns
+    # in 2 bytes (their padding, about an eighth, and group headers are not counted); the
+    # recomputing kernel reads both strings of every determinant once (N * 16 B)
+    def sigma_bytes(prec, s_v, s_x):
         if prec in (_capi.FP64, _capi.MIXED, _capi.FP32):
             return nnz_f * (s_v + 4) + N * 12 + N * (2 * s_x + 8)
         if prec in (_capi.FP64_UPPER, _capi.MIXED_UPPER, _capi.FP32_UPPER):
-            return nnz_u * (s_v + 4) + N * 12 + N * (2 * s_x + 8) + (20 if s_x == 4 else 16) * n_tiles
+            return nnz_u * (s_v + 2) + N * (2 * s_x + 8)
         return nnz_f * 4 + N * 12 + N * (2 * s_x + 8) + N * 16
 
-    b_sig = sigma_bytes(prec64, 8, 8, tiles64)
+    b_sig = sigma_bytes(prec64, 8, 8)
     peak, peak_kind = peaks()
     sig_gbs = b_sig / (t_sig * 1e-3) / 1e9
 
@@ -510,7 +508,7 @@ def main():
     y32 = torch.empty_like(x32)
     t_sig32 = time_sigma(x32, y32, 1)
     full_m = precm == _capi.MIXED
-    b_sig32 = sigma_bytes(precm, 4, 4, int(hs_p.get("n_tiles", 0)))
+    b_sig32 = sigma_bytes(precm, 4, 4)
     sig32_gbs = b_sig32 / (t_sig32 * 1e-3) / 1e9
 
     # ---- end to end through the public API: host dets in, energy + coefficients out ----

@@ -68,10 +68,12 @@ enum risqgpu_precision {
                            (bitwise the stored FP64 values) for sets whose values do not fit */
     /* Upper triangle only (each pair once, as the reference's SparseMatUpperTri): half the
      * storage.  The pairs are regrouped into row-panel x column-window tiles whose x and
-     * y windows sigma stages in shared memory.  The FP64 sigma sums in 64-bit fixed
-     * point, so it and the solves built on it are bitwise reproducible; the FP32 sigma
-     * sums in FP32 (order-dependent in the last bits) unless risqgpu_set_reproducible
-     * asks for fixed point too.  Built from scratch every time (no n_stored_h reuse). */
+     * y windows sigma stages in shared memory; where their padding does not fit the device
+     * or the handle's bound, the tiles are plain lists of pairs.  The FP64 sigma sums in
+     * 64-bit fixed point, so it and the solves built on it are bitwise reproducible (for
+     * the same of the two forms); the FP32 sigma sums columns in FP32 (order-dependent in
+     * the last bits) unless risqgpu_set_reproducible asks for fixed point too.  Built from
+     * scratch every time (no n_stored_h reuse). */
     RISQGPU_FP64_UPPER = 4,
     RISQGPU_FP32_UPPER = 5,
     RISQGPU_MIXED_UPPER = 6,
@@ -227,9 +229,9 @@ RISQGPU_API int risqgpu_sparse_optimize(risqgpu_t* h, const double* init_coeffs,
 RISQGPU_API int risqgpu_set_subspace(risqgpu_t* h, int max_space, int keep);
 
 /* Reproducible sums for the FP32 sigma of upper-triangle storage.  By default it sums
- * in FP32 with atomic adds, whose order (and so the last bits of the result) varies
+ * columns in FP32 with atomic adds, whose order (and so the last bits of the result) varies
  * from run to run; on = 1 makes it sum in 64-bit fixed point like the FP64 sigma,
- * bitwise reproducible, about 10 % slower.  FP64 sigma and partitioned handles always
+ * bitwise reproducible, up to 5 % slower.  FP64 sigma and partitioned handles always
  * sum in fixed point.  The reference's serial sums are reproducible by construction
  * (tests/integration_test_suite.rs:413-440). */
 RISQGPU_API int risqgpu_set_reproducible(risqgpu_t* h, int on);
@@ -307,8 +309,8 @@ RISQGPU_API int risqgpu_var_log(risqgpu_t* h, risqgpu_var_iter* out, int cap, in
  * point has no counterpart in the reference.  It is for callers that cannot let a
  * library allocate device memory during a solve: a host code whose pool allocator
  * owns the device memory budget, or a Davidson loop that overlaps work on several
- * streams, where the cudaMalloc/cudaFree pair inside risqgpu_sigma would add a
- * device-wide synchronisation to every iteration.  x_dev and y_dev are device
+ * streams, where an allocation inside risqgpu_sigma (with a memory bound, or when no
+ * kept memory fits) would add a device-wide synchronisation.  x_dev and y_dev are device
  * pointers to N doubles in the caller's determinant order (allocated by the
  * caller; x_dev may equal y_dev); the two internal-order copies live in one static
  * device array of 2 x 2^20 doubles (16 MiB), held by every GPU that loads the
