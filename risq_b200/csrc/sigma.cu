@@ -30,13 +30,16 @@ __device__ __forceinline__ T warp_sum(T v) {
 //
 // One warp per row, consecutive warps on consecutive rows.  What bounds it is the latency
 // of the column stream (HBM) followed by the gather of x (L1 / L2), so the loop is
-// software pipelined: the next 256 elements' columns and values (of this row, or the
-// first ones of the warp's next row) are in flight while this chunk's x are gathered.
+// software pipelined: the next 256 elements' (192 with remainders) columns and values (of
+// this row, or the first ones of the warp's next row) are in flight while this chunk's x
+// are gathered.
 // Measured, CUDA events: 200,003 rows, 2.0e8 elements, FP32: 420 us with four loads per
 // lane and no pipelining, 365 us here (4.4 TB/s of stream); 131,611 rows, 1.2e8
-// elements, FP64: 264 -> 253 us (5.6 TB/s); 6,943 rows: 13.9 -> 11.5 us.  Larger blocks,
-// and contiguous runs of rows per block, were slower (1.1x and 1.3-2x).
-constexpr int SPMV_U = 8;  // elements per lane in one chunk
+// elements, FP64: 264 -> 253 us (5.6 TB/s); 6,943 rows: 13.9 -> 11.5 us; FP32 + remainder
+// 327 -> 286 us, with six elements a lane (eight need more than the 64 registers of four
+// CTAs: 311), kept as they are stored until x is there (added on load, the chunk waited for
+// its own loads: 387).  Larger blocks, and contiguous runs of rows per block, were slower
+// (1.1x and 1.3-2x).
 
 template <int VK, typename X>
 __global__ void __launch_bounds__(256, 4) k_spmv(int64_t N, const int64_t* __restrict__ row_start,
@@ -47,24 +50,30 @@ __global__ void __launch_bounds__(256, 4) k_spmv(int64_t N, const int64_t* __res
                                                  const int* __restrict__ stop) {
     if (stop && *stop) return;
     using A = typename std::conditional<VK == 1, float, double>::type;
+    using R = typename std::conditional<VK == 2, float2, A>::type;  // a value as it is stored
+    constexpr int SPMV_U = VK == 2 ? 6 : 8;  // elements per lane in one chunk
     const int lane = threadIdx.x & 31;
     const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
     int64_t p = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
     if (p >= N) return;
     // a chunk's columns (-1: past the row's end) and values
-    auto load = [&](int64_t s, int k0, int len, int (&c)[SPMV_U], A (&a)[SPMV_U]) {
+    auto load = [&](int64_t s, int k0, int len, int (&c)[SPMV_U], R (&a)[SPMV_U]) {
 #pragma unroll
         for (int j = 0; j < SPMV_U; j++) {
             const int k = k0 + lane + 32 * j;
             c[j] = -1;
-            a[j] = 0;
+            a[j] = R{};
             if (k < len) {
                 c[j] = __ldcs(cols + s + k);
                 if constexpr (VK == 0) a[j] = __ldcs(v64 + s + k);
-                else if constexpr (VK == 2) a[j] = (double)__ldcs(v32 + s + k) + (double)__ldcs(vlo + s + k);
+                else if constexpr (VK == 2) a[j] = make_float2(__ldcs(v32 + s + k), __ldcs(vlo + s + k));
                 else a[j] = __ldcs(v32 + s + k);
             }
         }
+    };
+    auto value = [](R r) -> A {
+        if constexpr (VK == 2) return (double)r.x + (double)r.y;
+        else return r;
     };
     int64_t s = row_start[p], s_next = 0;
     int len = row_len[p], len_next = 0;
@@ -73,7 +82,7 @@ __global__ void __launch_bounds__(256, 4) k_spmv(int64_t N, const int64_t* __res
         len_next = row_len[p + nwarps];
     }
     int c[SPMV_U], cn[SPMV_U];
-    A a[SPMV_U], an[SPMV_U];
+    R a[SPMV_U], an[SPMV_U];
     load(s, 0, len, c, a);
     int k0 = 0;
     A acc = 0;
@@ -86,7 +95,7 @@ __global__ void __launch_bounds__(256, 4) k_spmv(int64_t N, const int64_t* __res
         for (int j = 0; j < SPMV_U; j++) xv[j] = c[j] >= 0 ? (A)__ldg(x + c[j]) : (A)0;
 #pragma unroll
         for (int j = 0; j < SPMV_U; j++)
-            if (c[j] >= 0) acc += a[j] * xv[j];
+            if (c[j] >= 0) acc += value(a[j]) * xv[j];
         if (!more) {
             acc = warp_sum(acc);
             if (lane == 0) y[p] = (X)(diag[p] * (double)x[p] + (double)acc);
