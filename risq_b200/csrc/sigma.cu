@@ -119,6 +119,75 @@ __global__ void __launch_bounds__(256, 4) k_spmv(int64_t N, const int64_t* __res
     }
 }
 
+// The same for sets of more rows than the chip holds warps whose rows hold few elements: a row
+// is then a chain of three latencies (its start, its columns, x) and k_spmv's chunks mostly
+// empty.  A warp takes NR rows at once, U elements a lane of each; every row's sums are formed
+// in the order of k_spmv.  Measured, 100,000 rows, FP64, us: 2 elements a row 24.0 (k_spmv
+// 41.8), 60: 30.4 (44.1), 84: 34.5 (44.5) with two rows and one element; 113: 38.5 (47.4) with
+// one row and four (54 with two and one).  Rows of 300 and more: k_spmv is the faster one.
+constexpr int64_t ROWS_TWO = 96, ROWS_ONE = 192;  // elements a row, on average, up to which
+
+template <int VK, typename X, int NR, int U>
+__global__ void __launch_bounds__(256) k_spmv_short(int64_t N, const int64_t* __restrict__ row_start,
+                                                    const int32_t* __restrict__ row_len, const int32_t* __restrict__ cols,
+                                                    const double* __restrict__ v64, const float* __restrict__ v32,
+                                                    const float* __restrict__ vlo, const double* __restrict__ diag,
+                                                    const X* __restrict__ x, X* __restrict__ y,
+                                                    const int* __restrict__ stop) {
+    if (stop && *stop) return;
+    using A = typename std::conditional<VK == 1, float, double>::type;
+    const int lane = threadIdx.x & 31;
+    const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    for (int64_t p0 = ((blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5) * NR; p0 < N; p0 += nwarps * NR) {
+        int64_t s[NR];
+        int len[NR], most = 0;
+        A acc[NR];
+#pragma unroll
+        for (int r = 0; r < NR; r++) {
+            s[r] = 0;
+            len[r] = 0;
+            acc[r] = 0;
+            if (p0 + r < N) {
+                s[r] = row_start[p0 + r];
+                len[r] = row_len[p0 + r];
+            }
+            most = max(most, len[r]);
+        }
+        for (int k0 = lane; k0 < most; k0 += 32 * U) {
+            int c[NR][U];
+            A a[NR][U], xv[NR][U];
+#pragma unroll
+            for (int r = 0; r < NR; r++)
+#pragma unroll
+                for (int j = 0; j < U; j++) {
+                    const int k = k0 + 32 * j;
+                    c[r][j] = -1;
+                    a[r][j] = 0;
+                    if (k < len[r]) {
+                        c[r][j] = __ldcs(cols + s[r] + k);
+                        if constexpr (VK == 0) a[r][j] = __ldcs(v64 + s[r] + k);
+                        else if constexpr (VK == 2) a[r][j] = (double)__ldcs(v32 + s[r] + k) + (double)__ldcs(vlo + s[r] + k);
+                        else a[r][j] = __ldcs(v32 + s[r] + k);
+                    }
+                }
+#pragma unroll
+            for (int r = 0; r < NR; r++)
+#pragma unroll
+                for (int j = 0; j < U; j++) xv[r][j] = c[r][j] >= 0 ? (A)__ldg(x + c[r][j]) : (A)0;
+#pragma unroll
+            for (int r = 0; r < NR; r++)
+#pragma unroll
+                for (int j = 0; j < U; j++)
+                    if (c[r][j] >= 0) acc[r] += a[r][j] * xv[r][j];
+        }
+#pragma unroll
+        for (int r = 0; r < NR; r++) acc[r] = warp_sum(acc[r]);
+#pragma unroll
+        for (int r = 0; r < NR; r++)
+            if (lane == r && p0 + r < N) y[p0 + r] = (X)(diag[p0 + r] * (double)x[p0 + r] + (double)acc[r]);
+    }
+}
+
 // FP64 sigma that recomputes every stored element from the two determinants and
 // the integrals (Slater-Condon in FP64, bitwise the values a FP64 build stores),
 // reading only the int32 column stream from HBM.  SMEM: the packed integral tables
@@ -242,16 +311,23 @@ int sigma_device(risqgpu* h, const void* x, void* y, int kind) {
         return sigma_matrix_free(h, (const double*)x, (double*)y);
     }
     // every warp of the chip resident, no more of them than rows
-    const int grid = (int)std::min<int64_t>((n + 7) / 8, (int64_t)num_sms(h) * 4);
+    const int64_t chip = (int64_t)num_sms(h) * 32, nnz = (int64_t)h->nnz_full;
+    const bool two = n > chip && nnz <= ROWS_TWO * n, one = !two && n > chip && nnz <= ROWS_ONE * n;
+    const int64_t ctas = two ? (n + 15) / 16 : (n + 7) / 8;
+    const int grid = (int)std::min<int64_t>(ctas, (int64_t)num_sms(h) * (two || one ? 8 : 4));
+    auto go = [&](auto kern, const double* v64, const float* v32, const float* vlo, auto* xv, auto* yv) {
+        kern<<<grid, 256, 0, h->stream>>>(n, h->d_row_start, h->d_row_len, h->d_cols, v64, v32, vlo, h->d_diag, xv, yv,
+                                          h->stop_flag);
+    };
     if (kind == 0) {
         const double* xd = (const double*)x;
         double* yd = (double*)y;
         if (h->precision == RISQGPU_FP64)
-            k_spmv<0, double><<<grid, 256, 0, h->stream>>>(n, h->d_row_start, h->d_row_len, h->d_cols, h->d_val64,
-                                                           nullptr, nullptr, h->d_diag, xd, yd, h->stop_flag);
+            go(two ? k_spmv_short<0, double, 2, 1> : one ? k_spmv_short<0, double, 1, 4> : k_spmv<0, double>, h->d_val64, nullptr,
+               nullptr, xd, yd);
         else if (h->precision == RISQGPU_MIXED)
-            k_spmv<2, double><<<grid, 256, 0, h->stream>>>(n, h->d_row_start, h->d_row_len, h->d_cols, nullptr,
-                                                           h->d_val32, h->d_val_lo, h->d_diag, xd, yd, h->stop_flag);
+            go(two ? k_spmv_short<2, double, 2, 1> : one ? k_spmv_short<2, double, 1, 4> : k_spmv<2, double>, nullptr, h->d_val32,
+               h->d_val_lo, xd, yd);
         else  // FP32 or columns-only storage: exact FP64 elements recomputed on the fly
             return h->W == 1 ? launch_otf<1>(h, xd, yd) : launch_otf<2>(h, xd, yd);
     } else {
@@ -259,8 +335,8 @@ int sigma_device(risqgpu* h, const void* x, void* y, int kind) {
             h->err = "FP32 sigma needs an FP32 or MIXED build";
             return RISQGPU_ERR_INVALID;
         }
-        k_spmv<1, float><<<grid, 256, 0, h->stream>>>(n, h->d_row_start, h->d_row_len, h->d_cols, nullptr, h->d_val32,
-                                                      nullptr, h->d_diag, (const float*)x, (float*)y, h->stop_flag);
+        go(two ? k_spmv_short<1, float, 2, 1> : one ? k_spmv_short<1, float, 1, 4> : k_spmv<1, float>, nullptr, h->d_val32, nullptr,
+           (const float*)x, (float*)y);
     }
     return check_launch(h, "sigma");
 }
