@@ -53,8 +53,11 @@ size_t block_size(size_t bytes) {
     return (bytes + unit - 1) / unit * unit;
 }
 
-// Whether a block may serve a request: at most an eighth of it unused.
-bool fits(size_t block, size_t bytes) { return block >= bytes && block - bytes <= bytes / 8; }
+// Whether a block may serve a request: at most an eighth more, or hardly any where the build
+// counts on every byte.
+bool fits(size_t block, size_t bytes, bool exact) {
+    return block >= bytes && block - bytes <= bytes / (exact ? 64 : 8);
+}
 
 void drop_oldest(Pool& P) {  // cudaFree waits for the work that uses the block
     const Block b = P.blocks.front();
@@ -168,7 +171,7 @@ int mem_alloc(risqgpu* h, void** p, size_t bytes, bool device) {
             b.held = h->exact ? bytes : block_size(bytes);
             auto best = h->parked.end();
             for (auto k = h->parked.begin(); k != h->parked.end(); ++k)
-                if (fits(k->second, bytes) && (best == h->parked.end() || k->second < best->second)) best = k;
+                if (fits(k->second, bytes, h->exact) && (best == h->parked.end() || k->second < best->second)) best = k;
             if (best != h->parked.end()) {
                 *p = best->first;
                 b.held = best->second;
@@ -182,7 +185,7 @@ int mem_alloc(risqgpu* h, void** p, size_t bytes, bool device) {
             auto best = P.blocks.end();
             if (b.source == FROM_BLOCKS)
                 for (auto k = P.blocks.begin(); k != P.blocks.end(); ++k)
-                    if (fits(k->bytes, bytes) && (best == P.blocks.end() || k->bytes < best->bytes)) best = k;
+                    if (fits(k->bytes, bytes, h->exact) && (best == P.blocks.end() || k->bytes < best->bytes)) best = k;
             if (best != P.blocks.end()) {
                 cudaStreamWaitEvent(h->stream, best->done, 0);
                 cudaEventDestroy(best->done);
